@@ -84,9 +84,11 @@ dftd3_b200_get_dispersion_batched(dftd3_error /* error */,
  * from host memory (NULL keeps the current ones).  param_grad[nsys][5], if
  * non-NULL, receives
  * dE/d(s6, s8, a1, a2, s9) (rational) or dE/d(s6, s8, rs6, rs8, s9) (zero).
- * Two-body evaluations are asynchronous with respect to the host.  With the
- * three-body term the call waits for the device once: for the neighbour
- * list sizes (ordinary sequence) or for the list capacity check at the end
+ * Evaluations are asynchronous with respect to the host, except with the
+ * three-body term when its pair blocks of all tile pairs and translations
+ * exceed 1 GiB (3 KiB each, 1.5 KiB in the mixed form): then only those in
+ * reach of the cutoff are kept and the call waits for the device once, for
+ * their number (ordinary sequence) or for the capacity check at the end
  * (captured sequence, dftd3_b200_set_batch_graph). */
 SDFTD3_API_ENTRY void SDFTD3_API_CALL
 dftd3_b200_get_dispersion_device(dftd3_error /* error */,
@@ -141,7 +143,7 @@ dftd3_b200_get_batch_graph_kernels(dftd3_error /* error */,
  * and launch shape runs the ordinary launch sequence and then captures it;
  * later evaluations launch the graph on the caller's stream.  Inputs and
  * outputs are staged through buffers the batch owns.  Per-stage times are
- * not recorded for graph replays.  A replay whose three-body lists outgrow
+ * not recorded for graph replays.  A replay whose three-body blocks outgrow
  * the captured buffers is detected and evaluated again without the graph. */
 SDFTD3_API_ENTRY void SDFTD3_API_CALL
 dftd3_b200_set_batch_graph(dftd3_error /* error */,
@@ -155,10 +157,9 @@ dftd3_b200_set_batch_graph(dftd3_error /* error */,
  * tuning[1] work items per tile pair of the pair sweeps (1, 2
  * or 4; 0 chooses 1 for batches of molecules, else 2, and 1 for the CN
  * sweeps of the mixed form when the tile pairs give every SM eight warps),
- * tuning[2] resident blocks per SM of the neighbour-list three-body
- * kernel (0 = occupancy limit), tuning[3] the block-per-molecule three-body
- * kernel for non-periodic systems of at most 256 atoms (0: when the batch has
- * at least one such molecule per SM, 1: always, 2: never). */
+ * tuning[2] resident blocks per SM of the three-body kernel (0 = occupancy
+ * limit), tuning[3] 0, 1 or 2, accepted for callers that set it: one
+ * three-body kernel serves molecules and periodic systems. */
 SDFTD3_API_ENTRY void SDFTD3_API_CALL
 dftd3_b200_set_batch_tuning(dftd3_error /* error */,
                             dftd3_b200_batch /* batch */,

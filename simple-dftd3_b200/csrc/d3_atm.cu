@@ -1,267 +1,87 @@
 // Axilrod-Teller-Muto three-body dispersion (get_atm_dispersion, atm.f90:433-825)
-// with energy, gradient, virial and dE/dCN.
+// with energy, gradient, virial and dE/dCN, for molecules and periodic systems.
 //
-// Enumeration: every atom i (the root) owns the triples whose other two
-// members are neighbours (j, T_j), (k, T_k) within the three-body cutoff with
-// k <= j <= i in the batch atom order -- the reference's i >= j >= k loop
-// (atm.f90:705-733) over any fixed atom order, so every triple is counted once
-// and triple_scale (atm.f90:954-980) handles repeated atoms.
+// Pair form.  With x = r^2 of the three pairs of a triple, u = 1/x,
+// m = sqrt(C6) r^-3 (times the smooth switch of the pair) and P = (r0/r)^(alp/3)
+// every factor of the triple is a product of pair factors:
+//   E = s9 M (1 + A) f,  M = m m m,  A = 3/8 S u u u,  f = 1 / (1 + 6 P P P),
+//   S = (x1 + x3 - x2)(x1 + x2 - x3)(x2 + x3 - x1)          (atm.f90:744-776)
+// and with K = (1 + A)(alp/2 6P f - 3/2) - A (P the product; alp = (alp + 2)/3)
+//   dE/dx1 = M f (u1 K + 3/8 u u u dS/dx1).
+// So the triple loop reads one 4-value record per pair and adds to two sums per
+// pair, D = sum dE/dx and W = sum E: gradient (2 D v), virial, dE/dCN
+// (W/2 dlnC6/dCN) and the derivative of the switch (W dln(sw)/dx) follow from D
+// and W once per pair instead of once per triple, and a pair outside the cutoff,
+// a ghost or a padding slot is a record with m = 0: the loop has no tests.
 //
-// Pipeline:
-//   k_c6_matrix     dense per-system table {sqrt(C6), dC6_rc/dCN_r / C6,
-//                   dC6_rc/dCN_c / C6} for the (j, k) lookups of the triples
-//   k_nbr_count     neighbour entries (j <= i, T) of every root
-//   (device scan)   entry offsets
-//   k_nbr_fill      entries image by image (for each translation T the atoms
-//                   j <= i in spatial order): vector x_j + T - x_i and r^2
-//   k_triples       persistent blocks take roots from a queue (largest lists
-//                   first); the warps sweep 32 x 32 tiles of (entry, entry)
-//                   pairs in the rounds of a round-robin schedule (disjoint
-//                   tiles per round), walking each tile along its diagonals
-//                   with the column sums travelling between the lanes, and
-//                   skip the steps in which no candidate is inside the cutoff
-//                   (the image-by-image order keeps tiles compact).  Per-entry
-//                   sums (scalar pair factor S, jk-gradient G, dE/dCN share D)
-//                   are updated in a fixed order; at the end of the root the
-//                   force and dE/dCN share of every entry's atom, and the
-//                   root's own, are added to per-atom fixed-point accumulators
-//                   (integer additions, so their order does not matter).
-//   k_atm_fixed     the accumulators into the FP64 gradient and dE/dCN: the
-//                   result is bit-reproducible in both forms.
-
+// Tiles and blocks.  Every 32-atom tile of the spatial order is cut into compact
+// tiles of 8 atoms (k_atm_order).  A block holds the 64 records of a tile pair
+// (A, B <= A) for one lattice translation (k_atm_pairs; batches whose blocks
+// exceed kAtmDenseCap keep only those whose spheres are in reach, k_atm_mark).
+// Tiles of 8 fill 0.6 of their triple slots with accepted triples on periodic
+// frames (cutoff 40 Bohr), tiles of 16 0.44 and of 32 0.30 (CPU replay).
+//
+// Triples (k_atm_triples).  Every unordered triple of tile images (modulo a
+// common translation) is visited once.  A unit is a pair block (J, K, T) whose
+// third atoms, the roots, run over the tiles I > J and their images; for J = K
+// (T in one half space, T = 0 as half of the walk) over all tiles, and then the
+// triples inside one tile index are met three times and weighted by 1/3.  One
+// (k_atm_lists: the tile images in reach of J.)  One warp takes a unit: four quarters of eight lanes hold four roots, the lane one
+// atom j, its eight (j, k) records and their sums D, W in registers, and the
+// quarter walks k = (j + t) mod 8; the sums of (i, k) move one lane down per step
+// with k.  Roots without a partner in J or K inside the cutoff are dropped
+// before (8-bit masks of the blocks).  Per four roots D and W of (i, j) and
+// (i, k) become forces; every 128 roots the (j, k) sums do.
+//
+// All sums over units go to fixed-point accumulators (integer additions), so the
+// results do not depend on the order of the warps and repeat bit for bit.
 #include <cub/cub.cuh>
 
 #include <algorithm>
-
 #include <cfloat>
 #include <cstdint>
 
-#include "d3_device.cuh"
 #include "d3_atm_common.cuh"
+#include "d3_device.cuh"
 
 namespace d3 {
 
 namespace {
 
-constexpr int kThreadsAtm = 256; // 8 warps
-// resident blocks per SM the triple kernel is compiled for (FP32 and FP64 forms)
-#ifndef TRI_MINB_F
-#define TRI_MINB_F 3
-#endif
-#ifndef TRI_MINB_D
-#define TRI_MINB_D 2
-#endif
-constexpr int kAcc = 5;          // per-entry accumulators: S, Gx, Gy, Gz, dE/dCN of the partner
+constexpr int kT8 = 8;                  // atoms per three-body tile
+constexpr int kRecs = kT8 * kT8;        // records per block
+constexpr int kAtmWarps = 4;            // warps per block of the triple kernel
+constexpr int kRing = 512;              // root queue of a warp: up to 127 left over + 32 tiles of 8
+constexpr int kRootChunk = 128;         // roots between two flushes: FP32 sums run over at most 32 terms
 
-// ------------------------------------------------------------ C6 matrix ----
-
-// {sqrt(C6_rc), dC6_rc/dCN_r / C6_rc, dC6_rc/dCN_c / C6_rc} for every ordered
-// pair (r, c) of each system (get_atomic_c6, model.f90:432-461); ghosts give 0.
-// The double sum over the references is taken as a dot product of r's
-// weights with c's species vector for r's species, U_c[s_r][ir] =
-// sum_jr C6ref(ir, jr) gw_c[jr] (and dU with dgw), accumulated in FP64.
-// One warp per row r; the lanes take the columns.  The damping-radius terms
-// alp3 log(r0) of the row's species pairs are computed once per row (for up
-// to 32 species), the species vectors are read with vector loads.
-template <class R>
-__global__ void k_c6_matrix(Batch b, Species s, Work w, const R* UV, double alp3, const long long* mat_off,
-                            C6Entry<R>* mat)
-{
-    __shared__ R slr0[8][32];
-    const int lane = threadIdx.x & 31, wid = (threadIdx.x >> 5) & 7;
-    const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (r >= b.natoms) return;
-    const int sys = b.sys_of_atom[r];
-    const int a0 = b.atom_off[sys];
-    const int n = b.atom_off[sys + 1] - a0;
-    C6Entry<R>* row = mat + mat_off[sys] + (long long)(r - a0) * n;
-    const int sr = b.sp[r];
-    const int nr = s.nref[sr];
-    const bool gr = b.ghost && b.ghost[r];
-    const bool table = b.nid <= 32;
-    auto lr0_of = [&](int sc) {
-        const double r0 = __ldg(s.atm_r0 + sr * b.nid + sc);
-        return R(alp3 * (sizeof(R) == 8 ? log(r0) : log2(r0)));
-    };
-    if (table && lane < b.nid) slr0[wid][lane] = lr0_of(lane);
-    __syncwarp();
-    const R* gw = (const R*)(sizeof(R) == 8 ? (const void*)w.gw : (const void*)w.gwf) + (size_t)r * kMaxRef;
-    const R* dgw = (const R*)(sizeof(R) == 8 ? (const void*)w.dgw : (const void*)w.dgwf) + (size_t)r * kMaxRef;
-    double g[kRefPad], dg[kRefPad];
-#pragma unroll
-    for (int ir = 0; ir < kRefPad; ir++) {
-        g[ir] = ir < nr ? double(gw[ir]) : 0.0;
-        dg[ir] = ir < nr ? double(dgw[ir]) : 0.0;
-    }
-    // the lower triangle (c <= r) and its mirror: C6 is symmetric and the entry
-    // (c, r) swaps the two CN-derivative ratios (the damping radius table is
-    // symmetric), so every product is formed once
-    const int rl = r - a0;
-    C6Entry<R>* mat_sys = mat + mat_off[sys];
-    for (int cl = lane; cl <= rl; cl += 32) {
-        const int c = a0 + cl;
-        const int sc = b.sp[c];
-        const R lr0 = table ? slr0[wid][sc] : lr0_of(sc);
-        C6Entry<R> out{R(0), R(0), R(0), lr0};
-        if (!(gr || (b.ghost && b.ghost[c]))) {
-            // U[0..7] and dU[0..7] of atom c for species sr (padding entries are zero)
-            R u[2 * kRefPad];
-            const R* up = UV + ((size_t)c * b.nid + sr) * (2 * kRefPad);
-            if constexpr (sizeof(R) == 4) {
-#pragma unroll
-                for (int q = 0; q < kRefPad / 2; q++) {
-                    const float4 v = __ldg(reinterpret_cast<const float4*>(up) + q);
-                    u[4 * q] = v.x; u[4 * q + 1] = v.y; u[4 * q + 2] = v.z; u[4 * q + 3] = v.w;
-                }
-            } else {
-#pragma unroll
-                for (int q = 0; q < kRefPad; q++) {
-                    const double2 v = __ldg(reinterpret_cast<const double2*>(up) + q);
-                    u[2 * q] = v.x; u[2 * q + 1] = v.y;
-                }
-            }
-            if constexpr (sizeof(R) == 4) {
-                // the FP32 entries of the mixed form from FP32 operands: FP32 arithmetic
-                float c6 = 0.f, dr = 0.f, dc = 0.f;
-#pragma unroll
-                for (int ir = 0; ir < kMaxRef; ir++) {
-                    c6 += float(g[ir]) * u[ir];
-                    dr += float(dg[ir]) * u[ir];
-                    dc += float(g[ir]) * u[kRefPad + ir];
-                }
-                if (c6 != 0.f) {
-                    const float inv = 1.0f / c6;
-                    out = C6Entry<R>{sqrtf(c6), dr * inv, dc * inv, lr0};
-                }
-            } else {
-                double c6 = 0.0, dr = 0.0, dc = 0.0;
-#pragma unroll
-                for (int ir = 0; ir < kMaxRef; ir++) {
-                    const double uv = double(u[ir]), du = double(u[kRefPad + ir]);
-                    c6 += g[ir] * uv;
-                    dr += dg[ir] * uv;
-                    dc += g[ir] * du;
-                }
-                if (c6 != 0.0) {
-                    const double inv = 1.0 / c6;
-                    out = C6Entry<R>{R(sqrt(c6)), R(dr * inv), R(dc * inv), lr0};
-                }
-            }
-        }
-        row[cl] = out;
-        if (cl < rl) mat_sys[(long long)cl * n + rl] = C6Entry<R>{out.sc6, out.qcr, out.qrc, out.lr0};
-    }
-}
-
-// --------------------------------------------------------- neighbour lists --
+template <class R> struct RecT;
+template <> struct RecT<double> { using rec = double4; using aux = double2; };
+template <> struct RecT<float> { using rec = float4; using aux = float2; };
 
 __device__ __forceinline__ bool in_shell(double r2, double cut2) { return !(r2 > cut2 || r2 < DBL_EPSILON); }
 
-// |v|^2 with a fixed rounding sequence, so that the counting and the filling
-// of the lists take exactly the same decisions
 __device__ __forceinline__ double norm2(double x, double y, double z)
 {
     return __fma_rn(z, z, __fma_rn(y, y, __dmul_rn(x, x)));
 }
 
-// Number of entries (j <= i, T) with eps <= |x_j + T - x_i|^2 <= cutoff^2.
-__global__ void k_nbr_count(Batch b, Config c, const uint8_t* sys_skip, int* cnt, int* max_cnt)
-{
-    const int lane = threadIdx.x & 31;
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (i >= b.natoms) return;
-    const int sys = b.sys_of_atom[i];
-    if (sys_skip && sys_skip[sys]) {
-        if (lane == 0) cnt[i] = 0;
-        return;
-    }
-    const int j0 = b.atom_off[sys];
-    const int t0 = b.img_off[kImgDisp3 * (b.nsys + 1) + sys], t1 = b.img_off[kImgDisp3 * (b.nsys + 1) + sys + 1];
-    const double xi = b.x[i], yi = b.y[i], zi = b.z[i];
-    const double cut2 = c.cut3 * c.cut3;
-    int n = 0;
-    for (int j = j0 + lane; j <= i; j += 32) {
-        const double dx = b.x[j] - xi, dy = b.y[j] - yi, dz = b.z[j] - zi;
-        for (int t = t0; t < t1; t++) {
-            const double vx = dx + __ldg(b.img + 3 * t), vy = dy + __ldg(b.img + 3 * t + 1),
-                         vz = dz + __ldg(b.img + 3 * t + 2);
-            n += in_shell(norm2(vx, vy, vz), cut2);
-        }
-    }
-    for (int off = 16; off > 0; off >>= 1) n += __shfl_xor_sync(0xffffffffu, n, off);
-    if (lane == 0) {
-        cnt[i] = n;
-        atomicMax(max_cnt, n);
-    }
-}
-
-__global__ void k_atm_guard(const long long* total, const int* max_cnt, long long cap, int stride, int* guard)
-{
-    *guard = (*total > cap || *max_cnt > stride) ? 1 : 0;
-}
-
-// Entries of root i, image by image: for each lattice translation T the
-// atoms j <= i (in the batch's spatial order) with eps <= |x_j + T - x_i|^2
-// <= cutoff^2, so that runs of consecutive entries are compact in space.
-// vec = (x_j + T) - x_i as in atm.f90:718.
-__global__ void k_nbr_fill(Batch b, Config c, const uint8_t* sys_skip, const long long* off, const int* cnt,
-                           int* nbr_j, int* nbr_gend, double4* nbr_v, const int* guard)
-{
-    const int lane = threadIdx.x & 31;
-    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (i >= b.natoms || *guard) return;
-    const int sys = b.sys_of_atom[i];
-    if (sys_skip && sys_skip[sys]) return;   // no entries were counted for this root
-    const int j0 = b.atom_off[sys];
-    const int t0 = b.img_off[kImgDisp3 * (b.nsys + 1) + sys], t1 = b.img_off[kImgDisp3 * (b.nsys + 1) + sys + 1];
-    const double xi = b.x[i], yi = b.y[i], zi = b.z[i];
-    const double cut2 = c.cut3 * c.cut3;
-    long long pos = off[i];
-    const long long end = off[i] + cnt[i];
-    for (int t = t0; t < t1; t++) {
-        const double tx = __ldg(b.img + 3 * t), ty = __ldg(b.img + 3 * t + 1), tz = __ldg(b.img + 3 * t + 2);
-        for (int jb = j0; jb <= i; jb += 32) {
-            const int j = jb + lane;
-            const bool valid = j <= i;
-            // the arithmetic of k_nbr_count, so that both accept the same entries
-            // (a self image at exactly the cutoff must not be counted and then missed)
-            const double dx = valid ? b.x[j] - xi : 0.0, dy = valid ? b.y[j] - yi : 0.0,
-                         dz = valid ? b.z[j] - zi : 0.0;
-            const double vx = dx + tx, vy = dy + ty, vz = dz + tz;
-            const double r2 = norm2(vx, vy, vz);
-            const bool ok = valid && in_shell(r2, cut2);
-            const unsigned msk = __ballot_sync(0xffffffffu, ok);
-            if (ok) {
-                const long long p = pos + __popc(msk & ((1u << lane) - 1u));
-                if (p < end) {
-                    nbr_j[p] = j;
-                    nbr_gend[p] = 0;
-                    nbr_v[p] = make_double4(vx, vy, vz, r2);
-                }
-            }
-            pos += __popc(msk);
-        }
-    }
-    // the list holds exactly the counted entries: slots the fill did not reach
-    // (which identical arithmetic rules out) become empty entries (r^2 = -1)
-    for (long long q = pos + lane; q < end; q += 32) {
-        nbr_j[q] = i;
-        nbr_gend[q] = 0;
-        nbr_v[q] = make_double4(0.0, 0.0, 0.0, -1.0);
-    }
-}
-
-// Deterministic accumulation of per-atom sums from many blocks: a value is
-// added as two 64-bit integers, its multiple of 2^-32 (floor) and the rest
-// rounded to units of 2^-72, so that the total does not depend on the order
-// of the additions.  Range +-2^31 per addition; the rest word takes up to
-// 2^23 additions (each below 2^40 + 1) before it could overflow.
-__device__ __forceinline__ void fixed_add(unsigned long long* acc2, double v)
+// Deterministic accumulation of sums from many warps: a value is added as two
+// 64-bit integers, its multiple of 2^-32 (floor) and the rest rounded to units
+// of 2^-72, so that the total does not depend on the order of the additions.
+// Range +-2^31 per addition; the rest word takes up to 2^23 additions (each
+// below 2^40 + 1) before it could overflow.
+__device__ __forceinline__ void fixed_split(double v, long long& hi, long long& lo)
 {
     const double sv = v * 4294967296.0;                 // 2^32
     const double h = floor(sv);
-    const long long hi = (long long)h;
-    const long long lo = __double2ll_rn((sv - h) * 1099511627776.0);   // 2^40
+    hi = (long long)h;
+    lo = __double2ll_rn((sv - h) * 1099511627776.0);    // 2^40
+}
+
+__device__ __forceinline__ void fixed_add(unsigned long long* acc2, double v)
+{
+    long long hi, lo;
+    fixed_split(v, hi, lo);
     atomicAdd(acc2, (unsigned long long)hi);
     atomicAdd(acc2 + 1, (unsigned long long)lo);
 }
@@ -272,496 +92,894 @@ __device__ __forceinline__ double fixed_value(const unsigned long long* acc2)
            double((long long)acc2[1]) * 2.117582368135751e-22;        // 2^-72
 }
 
-// ------------------------------------------------------------ triple sum ----
-
-template <class R> struct Vec4;
-template <> struct Vec4<double> { using type = double4; };
-template <> struct Vec4<float> { using type = float4; };
-
-// One neighbour entry of the current root, precomputed once per root.
-template <class R>
-struct Slot {
-    typename Vec4<R>::type v;   // head of x_j + T - x_i, r^2
-    typename Vec4<R>::type l;   // tail of the vector (mixed form), 1/r^2
-    typename Vec4<R>::type c;   // sqrt(C6_ij), dC6_ij/dCN_i / C6, dC6_ij/dCN_j / C6, alp3 log(r0_ij / r_ij)
-    typename Vec4<R>::type s;   // 1/r, switch, dsw/dr / r, valid (1 or 0)
-    int4 meta;                  // atom, group end, species, input index
-};
-
-// Column entries of one warp's tile pair, one array per field (rotated reads
-// of the lanes hit consecutive slots).
-template <class R>
-struct EntryTile {
-    typename Vec4<R>::type v[32], l[32], c[32], s[32];
-    int4 meta[32];
-};
-
-// Entry tiles a and b of the round-robin schedule of T' (even) tiles: round r
-// < T' - 1 pairs tile T' - 1 with r and (r + k) with (r - k) (mod T' - 1),
-// k = 1 .. T'/2 - 1; every tile is in exactly one pair of a round.
-__device__ __forceinline__ void rr_pair(int r, int k, int tp, int& a, int& b)
+// 1/x: the hardware approximation (FP32, 1 ulp), or its FP64 form (relative
+// error e0 below 2^-20) with one cubic correction y (1 + e + e^2), e = 1 - x y.
+__device__ __forceinline__ float rcp_fast(float x)
 {
-    const int q = tp - 1;
-    if (k == 0) { a = q; b = r; }
-    else { a = (r + k) % q; b = (r - k + q) % q; }
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ double rcp_fast(double x)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y, 1.0);
+    return fma(y, fma(e, e, e), y);
 }
 
-// Triple sum of the roots.  Persistent blocks take roots from a queue
-// (largest lists first).  A root's entries (j <= i, T) are cut into tiles of
-// 32, and every unordered pair of entries {a, b} is one candidate triple
-// (i, j, k): the atom pair (j, k) is the pair of entry atoms, larger first,
-// and two images of one atom stand for both orders of the reference's loop
-// (atm.f90:705-733), so they count twice (triple_scale, atm.f90:954-980, of
-// the atoms times 2).  The tile pairs (A, B) run in rounds of a round-robin
-// schedule, in which every tile occurs in one pair, and the block waits at
-// the end of each round; within a round the warps own their tiles alone, so
-// the per-entry sums are updated without atomics and in a fixed order, and
-// the result is bit-reproducible.  A warp walks its 32 x 32 tile pair along
-// the diagonals: at step t lane l pairs row entry 32 A + l with column entry
-// 32 B + (l + t) mod 32; the column's five sums move one lane down per step
-// with the column, the row's stay in the lane.  The diagonal pairs (A, A)
-// take steps 1..16.  Candidates are evaluated without branches (weight zero
-// outside the cutoff).
-template <class R, bool GRAD, bool PER, bool SMOOTH>
-__global__ void __launch_bounds__(kThreadsAtm, sizeof(R) == 4 ? TRI_MINB_F : TRI_MINB_D)
-k_triples(Batch b, Species sp, Damp d, Config c, Partition part, Work w, const C6Entry<R>* mat,
-          const long long* mat_off, const long long* off, const int* cnt, const int* nbr_j, const int* nbr_gend,
-          const double4* nbr_v, unsigned int* queue, double* slot_acc, Slot<R>* slot_scr, int slot_stride,
-          double* e3, double* sig3, unsigned long long* fxacc)
-{
-    extern __shared__ __align__(16) unsigned char smem[];
-    EntryTile<R>* tiles = reinterpret_cast<EntryTile<R>*>(smem);
-    __shared__ int s_root;
-    __shared__ double wsum[kThreadsAtm / 32][13];
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    constexpr int kWarps = kThreadsAtm / 32;
-    double* acc = slot_acc + (size_t)blockIdx.x * slot_stride * kAcc;
-    Slot<R>* scr = slot_scr + (size_t)blockIdx.x * slot_stride;
-    EntryTile<R>& tl = tiles[wid];
-    const R s9 = R(d.s9);
-    const R alp = R(d.alp + 2.0);        // ATM exponent alp + 2 (rational.f90:563)
-    const R alp3 = alp / R(3);
-    const R cut2 = R(c.cut3 * c.cut3);
-    const R cutoff = R(c.cut3), width = R(c.width3);
-    if (w.atm_guard && *w.atm_guard) return;   // lists did not fit the reserved buffers
-    __syncthreads();
+// Candidate block c of the processing order: system, tile pair (A >= B, local
+// tile indices) and translation index.
+struct BlockId { int sys, t8, A, B, t; };
 
-    for (;;) {
-        if (tid == 0) {
-            const unsigned q = atomicAdd(queue, 1u);
-            s_root = q < (unsigned)b.natoms ? b.natoms - 1 - (int)q : -1;
+__device__ __forceinline__ BlockId block_id(const AtmView& v, long long c, int lane)
+{
+    // 32-way search of the system (whole warp)
+    int lo = 0, hi = v.nord;
+    while (hi - lo > 1) {
+        const int step = (hi - lo + 31) >> 5;
+        const int p = lo + lane * step;
+        const unsigned ok = __ballot_sync(0xffffffffu, p < hi && v.cand_off[p] <= c);
+        lo += (__popc(ok) - 1) * step;
+        hi = min(hi, lo + step);
+    }
+    BlockId id;
+    id.sys = v.ord[lo];
+    id.t8 = v.t8_off[id.sys];
+    const long long e = c - v.cand_off[lo];
+    const int nT = v.rep[4 * id.sys + 3];
+    const unsigned p = (unsigned)(e / nT);
+    id.t = (int)(e - (long long)p * nT);
+    int a = (int)((sqrtf(8.0f * (float)p + 1.0f) - 1.0f) * 0.5f);
+    while ((unsigned)(a + 1) * (unsigned)(a + 2) / 2 <= p) a++;
+    while ((unsigned)a * (unsigned)(a + 1) / 2 > p) a--;
+    id.A = a;
+    id.B = (int)(p - (unsigned)a * (unsigned)(a + 1) / 2);
+    return id;
+}
+
+// ------------------------------------------------------------- tile order --
+
+// Axis of the longest extent of the atoms in group g of the warp.
+__device__ __forceinline__ int longest_axis(double x, double y, double z, bool mine)
+{
+    double lo[3] = {mine ? x : DBL_MAX, mine ? y : DBL_MAX, mine ? z : DBL_MAX};
+    double hi[3] = {mine ? x : -DBL_MAX, mine ? y : -DBL_MAX, mine ? z : -DBL_MAX};
+    for (int o = 16; o > 0; o >>= 1)
+        for (int k = 0; k < 3; k++) {
+            lo[k] = fmin(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], o));
+            hi[k] = fmax(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o));
         }
-        __syncthreads();
-        const int i = s_root;
-        __syncthreads();
-        if (i < 0) break;
-        const int m = cnt[i];
-        const long long base = off[i];
-        const int sys = b.sys_of_atom[i];
-        const int a0 = b.atom_off[sys];
-        const int nsys_n = b.atom_off[sys + 1] - a0;
-        const C6Entry<R>* msys = mat + mat_off[sys];
-        const long long mrow_i = (long long)(i - a0) * nsys_n;
-        const int orig_i = b.local[i];
-        const int si = b.sp[i];
-        // per-lane sums of this root: energy, dE/dCN, jk virial, accepted triples
-        double e_root = 0.0, dei = 0.0;
-        double sxx = 0, syy = 0, szz = 0, sxy = 0, sxz = 0, syz = 0;
-        int ntrip = 0;
-        if (m > 1) {
-            // entry records of this root (all threads)
-            for (int k = tid; k < m; k += kThreadsAtm) {
-                const int j = nbr_j[base + k];
-                double4 v = nbr_v[base + k];
-                const bool ventry = v.w > 0.0;   // not an empty entry
-                if (!ventry) v.w = 1.0;
-                Slot<R> r;
-                const int sj = b.sp[j];
-                const C6Entry<R> e = msys[mrow_i + (j - a0)];
-                const double r0 = __ldg(sp.atm_r0 + si * b.nid + sj);
-                if constexpr (sizeof(R) == 8) {
-                    r.v = make_double4(v.x, v.y, v.z, v.w);
-                    r.l = make_double4(0.0, 0.0, 0.0, 1.0 / v.w);
-                    r.c = make_double4(e.sc6, e.qrc, e.qcr, alp3 * (log(r0) - 0.5 * log(v.w)));
-                    r.s = make_double4(rsqrt(v.w), 1.0, 0.0, 1.0);
-                } else {
-                    const float hx = __double2float_rn(v.x), hy = __double2float_rn(v.y), hz = __double2float_rn(v.z);
-                    r.v = make_float4(hx, hy, hz, __double2float_rn(v.w));
-                    r.l = make_float4(__double2float_rn(v.x - (double)hx), __double2float_rn(v.y - (double)hy),
-                                      __double2float_rn(v.z - (double)hz), __double2float_rn(1.0 / v.w));
-                    r.c = make_float4(e.sc6, e.qrc, e.qcr,
-                                      __double2float_rn(double(alp3) * (log2(r0) - 0.5 * log2(v.w))));
-                    r.s = make_float4(__double2float_rn(rsqrt(v.w)), 1.f, 0.f, 1.f);
-                }
-                if (SMOOTH) {
-                    R sw, dsw;
-                    const R rr = R(sqrt(v.w));
-                    smooth<R>(rr, cutoff, width, sw, dsw);
-                    r.s.y = sw;
-                    r.s.z = dsw / rr;
-                }
-                r.meta = make_int4(j, 0, sj, b.local[j]);
-                if (!ventry) { r.c.x = R(0); r.s.w = R(0); }
-                scr[k] = r;
-                if (GRAD)
-                    for (int v2 = 0; v2 < kAcc; v2++) acc[k * kAcc + v2] = 0.0;
+    const double ex = hi[0] - lo[0], ey = hi[1] - lo[1], ez = hi[2] - lo[2];
+    return ex >= ey && ex >= ez ? 0 : ey >= ez ? 1 : 2;
+}
+
+// Compact tiles of 8 atoms inside each 32-atom tile (one warp each): the atoms
+// are ordered along the longest axis of their box and cut into tiles of 8, above
+// 16 atoms into two halves that are ordered along their own longest axis (fill
+// of the triple slots on periodic frames 0.56, against 0.49 with fixed x and y).
+// Also writes the tiles' positions and clears the accumulators of the evaluation.
+__global__ void k_atm_order(Batch b, const int* tile_off, const int* tile_sys, int ntiles, AtmView v, double4* spheres,
+                            unsigned long long* fxf, unsigned long long* fxe, unsigned long long* queue)
+{
+    pdl_wait();
+    const int lane = threadIdx.x & 31;
+    const int tile = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (blockIdx.x == 0 && threadIdx.x < 2) queue[threadIdx.x] = 0;
+    if (tile >= ntiles) return;
+    const int sys = tile_sys[tile];
+    const int lt = tile - tile_off[sys];
+    const int a0 = b.atom_off[sys] + lt * kTile;
+    const int n = min(kTile, b.atom_off[sys + 1] - a0);
+    const bool in = lane < n;
+    const int a = a0 + (in ? lane : 0);
+    const double x = b.x[a], y = b.y[a], z = b.z[a];
+    auto rank_in = [&](int axis, int group) {
+        const double c = axis == 0 ? x : axis == 1 ? y : z;
+        int r = 0;
+        for (int k = 0; k < n; k++) {
+            const double ck = __shfl_sync(0xffffffffu, c, k);
+            const int gk = __shfl_sync(0xffffffffu, group, k);
+            r += gk == group && (ck < c || (ck == c && k < lane));
+        }
+        return r;
+    };
+    int slot = rank_in(longest_axis(x, y, z, in), 0);
+    if (n > 16) {
+        const int half = slot >> 4;
+        const int ax0 = longest_axis(x, y, z, in && half == 0), ax1 = longest_axis(x, y, z, in && half == 1);
+        slot = 16 * half + rank_in(half ? ax1 : ax0, half);
+    }
+    const int base8 = v.t8_off[sys] + 4 * lt;
+    const int n8 = (n + kT8 - 1) / kT8;
+    if (in) {
+        v.sub[kT8 * base8 + slot] = a;
+        v.pos[kT8 * base8 + slot] = make_double4(x, y, z, (double)a);
+    } else if (lane < kT8 * n8) {
+        v.sub[kT8 * base8 + lane] = -1;
+        v.pos[kT8 * base8 + lane] = make_double4(0.0, 0.0, 0.0, 0.0);
+    }
+    if (fxf && in) {
+        unsigned long long* f = fxf + (size_t)8 * a;
+#pragma unroll
+        for (int k = 0; k < 8; k++) f[k] = 0;
+    }
+    if (lane < n8) {
+        unsigned long long* f = fxe + (size_t)20 * (base8 + lane);
+#pragma unroll
+        for (int k = 0; k < 20; k++) f[k] = 0;
+    }
+    if (!spheres) return;
+    // bounding spheres (box centre, largest distance)
+    for (int q = 0; q < n8; q++) {
+        const bool mine = in && (slot >> 3) == q;
+        double lo[3] = {mine ? x : DBL_MAX, mine ? y : DBL_MAX, mine ? z : DBL_MAX};
+        double hi[3] = {mine ? x : -DBL_MAX, mine ? y : -DBL_MAX, mine ? z : -DBL_MAX};
+        for (int o = 16; o > 0; o >>= 1)
+            for (int k = 0; k < 3; k++) {
+                lo[k] = fmin(lo[k], __shfl_xor_sync(0xffffffffu, lo[k], o));
+                hi[k] = fmax(hi[k], __shfl_xor_sync(0xffffffffu, hi[k], o));
             }
-            __syncthreads();
-            const int T = (m + 31) >> 5;
-            const int tp = T + (T & 1);
-            // rounds 0 .. tp - 2: disjoint pairs of different tiles; round tp - 1: the tiles with themselves
-            for (int round = 0; round < tp; round++) {
-                const bool diag = round == tp - 1;
-                const int npairs = diag ? T : tp / 2;
-                for (int pk = wid; pk < npairs; pk += kWarps) {
-                    int ta, tb;
-                    if (diag) { ta = pk; tb = pk; }
-                    else {
-                        int x, y;
-                        rr_pair(round, pk, tp, x, y);
-                        if (x >= T || y >= T) continue;   // the pad tile of an odd tile count
-                        ta = x > y ? x : y; tb = x > y ? y : x;
+        double c[3], d2 = 0.0;
+        for (int k = 0; k < 3; k++) c[k] = 0.5 * (lo[k] + hi[k]);
+        if (mine) d2 = norm2(x - c[0], y - c[1], z - c[2]);
+        for (int o = 16; o > 0; o >>= 1) d2 = fmax(d2, __shfl_xor_sync(0xffffffffu, d2, o));
+        if (lane == 0) spheres[base8 + q] = make_double4(c[0], c[1], c[2], sqrt(d2));
+    }
+}
+
+// ------------------------------------------------------------ pair blocks --
+
+// flag[c] = 1 for the candidate blocks whose spheres are within the cutoff
+// (with a margin far above the rounding of the sphere test).
+__global__ void k_atm_mark(Batch b, Config c, AtmView v, const double4* spheres, int* flag)
+{
+    const int lane = threadIdx.x & 31;
+    const long long w0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) & ~31LL;
+    if (w0 >= v.ncand) return;
+    // the 32 candidates of a warp may span systems: the search takes them one
+    // system at a time only where they do
+    const long long cand = w0 + lane;
+    const BlockId first = block_id(v, w0, lane);
+    const long long last_c = min(w0 + 31, v.ncand - 1);
+    const BlockId last = block_id(v, last_c, lane);
+    BlockId id = first;
+    if (first.sys == last.sys) {
+        const int nT = v.rep[4 * first.sys + 3];
+        const long long t = (long long)first.t + lane;
+        long long p = (long long)first.A * (first.A + 1) / 2 + first.B + t / nT;
+        id.t = (int)(t % nT);
+        int a = first.A;
+        while ((long long)(a + 1) * (a + 2) / 2 <= p) a++;
+        id.A = a;
+        id.B = (int)(p - (long long)a * (a + 1) / 2);
+    } else {
+        for (int k = 0; k < 32; k++) {
+            const BlockId q = block_id(v, min(w0 + k, v.ncand - 1), lane);
+            if (k == lane) id = q;
+        }
+    }
+    if (cand >= v.ncand) return;
+    const double4 sa = spheres[id.t8 + id.A], sb = spheres[id.t8 + id.B];
+    const double* T = b.img + 3 * (size_t)(b.img_off[kImgDisp3 * (b.nsys + 1) + id.sys] + id.t);
+    const double reach = (c.cut3 + sa.w + sb.w) * (1.0 + 1e-9) + 1e-9;
+    flag[cand] = norm2(sb.x + T[0] - sa.x, sb.y + T[1] - sa.y, sb.z + T[2] - sa.z) <= reach * reach ? 1 : 0;
+}
+
+__global__ void k_atm_guard(const int* total, long long cap, int* guard) { *guard = *total > cap ? 1 : 0; }
+
+// The 64 records {x, u, m, P} of a block and, with gradients, {dlnC6/dCN_a / 2,
+// dlnC6/dCN_b / 2} of (row atom a of A, column atom b of B + T): one warp per
+// candidate.  C6 is the dot product of a's reference weights with b's species
+// vector for a's species, U_b[s_a][r] = sum_q C6ref(r, q) gw_b[q]
+// (get_atomic_c6, model.f90:432-461).  mask: bits 0-7 the rows, bits 8-15 the
+// columns with a pair inside the cutoff.
+template <class R>
+__global__ void __launch_bounds__(256)
+k_atm_pairs(Batch b, Species s, Config c, Work w, AtmView v, const R* UV, double alp3, const int* guard)
+{
+    pdl_wait();
+    const int lane = threadIdx.x & 31;
+    const long long cand = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (cand >= v.ncand || (guard && *guard)) return;
+    long long blk = cand;
+    if (v.map) {
+        const int m0 = v.map[cand], m1 = v.map[cand + 1];
+        if (m0 == m1) {
+            if (lane == 0) v.mask[cand] = 0;
+            return;
+        }
+        blk = m0;
+    }
+    const BlockId id = block_id(v, cand, lane);
+    const double* T = b.img + 3 * (size_t)(b.img_off[kImgDisp3 * (b.nsys + 1) + id.sys] + id.t);
+    const double tx = T[0], ty = T[1], tz = T[2];
+    const double cut2 = c.cut3 * c.cut3;
+    const int bc = v.sub[kT8 * (id.t8 + id.B) + (lane & 7)];
+    double x2[2];
+    int ar[2];
+    bool ok[2];
+    unsigned vote[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        ar[h] = v.sub[kT8 * (id.t8 + id.A) + 4 * h + (lane >> 3)];
+        x2[h] = 1.0;
+        ok[h] = ar[h] >= 0 && bc >= 0;
+        if (ok[h]) {
+            const double r2 = norm2(b.x[bc] + tx - b.x[ar[h]], b.y[bc] + ty - b.y[ar[h]], b.z[bc] + tz - b.z[ar[h]]);
+            ok[h] = in_shell(r2, cut2);
+            if (ok[h]) x2[h] = r2;
+        }
+        vote[h] = __ballot_sync(0xffffffffu, ok[h]);
+    }
+    if (lane == 0) {
+        unsigned rows = 0, cols = vote[0] | vote[1];
+        cols |= cols >> 16;
+        cols |= cols >> 8;
+        for (int q = 0; q < 4; q++) {
+            rows |= ((vote[0] >> (8 * q)) & 0xffu) ? 1u << q : 0u;
+            rows |= ((vote[1] >> (8 * q)) & 0xffu) ? 1u << (q + 4) : 0u;
+        }
+        v.mask[cand] = (unsigned short)(rows | (cols & 0xffu) << 8);
+    }
+    if (!(vote[0] | vote[1])) return;
+    using Rec = typename RecT<R>::rec;
+    using Aux = typename RecT<R>::aux;
+    Rec* rec = static_cast<Rec*>(v.rec) + blk * kRecs;
+    Aux* aux = static_cast<Aux*>(v.aux) + blk * kRecs;
+    const R* gw_all = (const R*)(sizeof(R) == 8 ? (const void*)w.gw : (const void*)w.gwf);
+    const R* dgw_all = (const R*)(sizeof(R) == 8 ? (const void*)w.dgw : (const void*)w.dgwf);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        Rec o;
+        o.x = R(1); o.y = R(0); o.z = R(0); o.w = R(0);
+        Aux q;
+        q.x = R(0); q.y = R(0);
+        if (ok[h]) {
+            const int a = ar[h];
+            const int sa = b.sp[a], sb = b.sp[bc];
+            o.x = R(x2[h]);
+            o.y = R(1) / o.x;
+            const R* gw = gw_all + (size_t)a * kMaxRef;
+            const R* dgw = dgw_all + (size_t)a * kMaxRef;
+            const R* up = UV + ((size_t)bc * b.nid + sa) * (2 * kRefPad);
+            const int nr = s.nref[sa];
+            R c6 = R(0), dr = R(0), dc = R(0);
+            for (int r = 0; r < nr; r++) {
+                const R u0 = __ldg(up + r);
+                c6 += gw[r] * u0;
+                dr += dgw[r] * u0;
+                dc += gw[r] * __ldg(up + kRefPad + r);
+            }
+            if (b.ghost && b.ghost[a]) c6 = R(0);
+            const R r0 = R(__ldg(s.atm_r0 + sa * b.nid + sb));
+            // the pair's share of (r0/r)^alp3, bounded so that the product of
+            // three stays finite (the damping has vanished long before)
+            if constexpr (sizeof(R) == 8) o.w = fmin(exp(0.5 * alp3 * log(r0 * r0 * o.y)), 1e100);
+            else o.w = fminf(exp2f(0.5f * float(alp3) * log2f(r0 * r0 * o.y)), 1e12f);
+            if (c6 != R(0)) {
+                R m = sqrt(c6) * o.y * sqrt(o.y);
+                if (c.width3 > 0.0) {
+                    R sw, dsw;
+                    smooth<R>(R(sqrt(x2[h])), R(c.cut3), R(c.width3), sw, dsw);
+                    m *= sw;
+                }
+                o.z = m;
+                const R ic6 = R(0.5) / c6;
+                q.x = dr * ic6;
+                q.y = dc * ic6;
+            }
+        }
+        rec[32 * h + lane] = o;
+        if (c.grad) aux[32 * h + lane] = q;
+    }
+}
+
+// Root tiles of every tile J, ascending: the tile images (I, T_I) whose block
+// with J has a pair inside the cutoff, {block, mask of the roots << 24 | I, T_I,
+// candidate}.  One warp per tile; gt[J] is the first entry with I > J.
+__global__ void k_atm_lists(AtmView v, int ntiles8, const int* tile8_sys, const long long* list_off, int4* list,
+                            int2* range, const int* guard)
+{
+    pdl_wait();
+    const int lane = threadIdx.x & 31;
+    const int tile = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (tile >= ntiles8 || (guard && *guard)) return;
+    const int sys = tile8_sys[tile];
+    const int t8 = v.t8_off[sys], nt8 = v.t8_off[sys + 1] - t8, J = tile - t8;
+    const int nT = v.rep[4 * sys + 3];
+    const long long cbase = v.cand_off_sys[sys];
+    int4* out = list + list_off[sys] + (long long)J * nt8 * nT;
+    int n = 0, gt = 0;
+    for (int e0 = 0; e0 < nt8 * nT; e0 += 32) {
+        const int e = e0 + lane;
+        int4 o = make_int4(0, 0, 0, 0);
+        unsigned m = 0;
+        int I = 0;
+        if (e < nt8 * nT) {
+            I = nT == 1 ? e : e / nT;
+            const int tI = e - I * nT;
+            // stored as (I, J) with J at -T_I, or for I < J as (J, I) with I at T_I
+            const long long c = I < J ? cbase + ((long long)J * (J + 1) / 2 + I) * nT + tI
+                                      : cbase + ((long long)I * (I + 1) / 2 + J) * nT + (nT - 1 - tI);
+            m = v.mask[c];
+            m = I < J ? m >> 8 : m & 0xffu;
+            if (m) o = make_int4((int)(v.map ? v.map[c] : c), (int)(m << 24) | I, tI, 0);
+        }
+        const unsigned keep = __ballot_sync(0xffffffffu, m != 0);
+        gt += __popc(__ballot_sync(0xffffffffu, m != 0 && I <= J));
+        if (m) out[n + __popc(keep & ((1u << lane) - 1u))] = o;
+        n += __popc(keep);
+    }
+    if (lane == 0) range[tile] = make_int2(gt, n);
+}
+
+// ---------------------------------------------------------------- triples --
+
+template <class R>
+__device__ __forceinline__ R sel(bool p, R a, R b) { return p ? a : b; }
+
+// dln(sw)/dx of a pair's switch at r = sqrt(x) (zero where the switch is 1 or 0)
+template <class R>
+__device__ __forceinline__ R dln_switch(R x, R cutoff, R width)
+{
+    R sw, dsw;
+    const R r = sqrt(x);
+    smooth<R>(r, cutoff, width, sw, dsw);
+    return sw > R(0) ? R(0.5) * dsw / (sw * r) : R(0);
+}
+
+// Per-warp shared memory of the triple kernel: the records of four roots (two
+// buffers, filled one step of four ahead by asynchronous copies) and the queue.
+template <class R>
+struct AtmStage {
+    typename RecT<R>::rec ik[32], ij[32];
+    typename RecT<R>::aux qij[32], qik[32];
+    double4 pos[4];                  // root position, atom
+    double T[4][4];                  // root translation
+};
+template <class R>
+struct AtmShared {
+    AtmStage<R> st[2];
+    int4 ring[kRing];                // roots: block (i, j), block (i, k), tile slot, flags and translation
+};
+
+template <int BYTES>
+__device__ __forceinline__ void async_copy(void* dst, const void* src)
+{
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(BYTES) : "memory");
+}
+template <class V>
+__device__ __forceinline__ void async_copy_value(V* dst, const V* src)
+{
+    if constexpr (sizeof(V) == 32) {
+        async_copy<16>(dst, src);
+        async_copy<16>(reinterpret_cast<char*>(dst) + 16, reinterpret_cast<const char*>(src) + 16);
+    } else {
+        async_copy<(int)sizeof(V)>(dst, src);
+    }
+}
+
+// What bounds it: issue slots and dependent latencies (FP32: 2.5 instructions per
+// cycle and SM; FP64: 1.5, the FP64 pipe at 46%).  Per lane slot 42 arithmetic
+// instructions, one reciprocal, two (FP32) or four shuffles and one or two 16-byte
+// shared loads, 62 in all with the work per four roots; the (j, k) records and sums
+// stay in registers.  Whole evaluations, the neighbour-list and block-per-molecule
+// kernels that this one replaced against it (185 instructions per slot, exp, log
+// and divisions per triple in FP64): cluster of 5000 atoms (FP64) 54.0 -> 16.8 ms,
+// 512 molecules (FP64) 21.4 -> 2.1 ms, 4096 molecules (mixed) 13.9 -> 7.5 ms, eight
+// periodic frames (mixed) 149 -> 64 ms, one molecule of 100 atoms 216 -> 85 us.
+// GEN: work partition and term counting (the owner test of every triple).
+template <class R, bool GRAD, bool PER, bool GEN>
+__global__ void __launch_bounds__(32 * kAtmWarps, sizeof(R) == 4 ? (GRAD ? 4 : 6) : (GRAD ? 2 : 4))
+k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int split, int grab,
+              unsigned long long* queue, unsigned long long* fxf, unsigned long long* fxe, int counting,
+              const int* guard)
+{
+    pdl_wait();
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    using Rec = typename RecT<R>::rec;
+    using Aux = typename RecT<R>::aux;
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    AtmShared<R>& sh = reinterpret_cast<AtmShared<R>*>(smem_raw)[wid];
+    if (guard && *guard) return;                 // blocks did not fit the reserved buffers
+    const Rec* rec = static_cast<const Rec*>(v.rec);
+    const Aux* aux = static_cast<const Aux*>(v.aux);
+    const int q = lane >> 3, j = lane & 7, qbase = lane & 24;
+    const R ahalf = R(0.5 * alp3d);
+    const bool smooth_on = c.width3 > 0.0 && c.width3 < c.cut3;
+    const R cutoff = R(c.cut3), width = R(c.width3);
+    const unsigned long long nunits = (unsigned long long)v.ncand * split;
+    unsigned long long u = 0, u_end = 0;
+    for (;;) {
+        if (u == u_end) {
+            if (lane == 0) u = atomicAdd(queue, (unsigned long long)grab);
+            u = __shfl_sync(kAll, u, 0);
+            if (u >= nunits) break;
+            u_end = min(u + grab, nunits);
+        }
+        const long long cand = (long long)(u / split);
+        const int piece = (int)(u % split);
+        u++;
+        if (v.mask[cand] == 0) continue;
+        const BlockId id = block_id(v, cand, lane);
+        const int nT = PER ? v.rep[4 * id.sys + 3] : 1;
+        const bool same = id.A == id.B;
+        if (PER && same && 2 * id.t < nT - 1) continue;      // the other half space
+        const bool diag = same && 2 * id.t == nT - 1;
+        const int nt8 = v.t8_off[id.sys + 1] - id.t8;
+        const int J = id.A, K = id.B;
+        int rx = 0, ry = 0, rz = 0, jx = 0, jy = 0, jz = 0;
+        if (PER) {
+            rx = v.rep[4 * id.sys]; ry = v.rep[4 * id.sys + 1]; rz = v.rep[4 * id.sys + 2];
+            jz = id.t % (2 * rz + 1) - rz;
+            jy = id.t / (2 * rz + 1) % (2 * ry + 1) - ry;
+            jx = id.t / ((2 * rz + 1) * (2 * ry + 1)) - rx;
+        }
+        const long long cbase = cand - ((long long)J * (J + 1) / 2 + K) * nT - id.t;    // first candidate of the system
+        const double* img = b.img + 3 * (size_t)b.img_off[kImgDisp3 * (b.nsys + 1) + id.sys];
+        const double kx = PER ? img[3 * id.t] : 0.0, ky = PER ? img[3 * id.t + 1] : 0.0,
+                     kz = PER ? img[3 * id.t + 2] : 0.0;
+        const long long bjk = v.map ? v.map[cand] : cand;
+        const int aj = v.sub[kT8 * (id.t8 + J) + j], ak = v.sub[kT8 * (id.t8 + K) + j];
+        double xj = 0, yj = 0, zj = 0, xk = 0, yk = 0, zk = 0;
+        if (GRAD) {
+            if (aj >= 0) { xj = b.x[aj]; yj = b.y[aj]; zj = b.z[aj]; }
+            if (ak >= 0) { xk = b.x[ak] + kx; yk = b.y[ak] + ky; zk = b.z[ak] + kz; }
+        }
+        int oj = 0, ok = 0;
+        if (GEN) {
+            oj = aj >= 0 ? b.local[aj] : 0;
+            ok = ak >= 0 ? b.local[ak] : 0;
+        }
+        // the (j, k) records of this lane, step t: k = (j + t) mod 8
+        Rec rjk[kT8];
+#pragma unroll
+        for (int t = 0; t < kT8; t++) {
+            rjk[t] = rec[bjk * kRecs + kT8 * j + ((j + t) & 7)];
+            if (diag && t == 4 && j >= 4) { rjk[t].z = R(0); if (GEN) rjk[t].y = R(0); }
+        }
+        const int2 range = v.range[id.t8 + J];
+        const int4* list = v.list + v.list_off[id.sys] + (long long)J * nt8 * nT;
+        const int nE = range.y;
+        int e0 = (same ? 0 : range.x) + piece;
+        int head = 0, cnt = 0;
+        while (true) {
+            // roots: tiles I (and images) with a pair in reach of both J and K
+            while (cnt < kRootChunk && e0 < nE) {
+                const int e = e0 + lane * split;
+                e0 += 32 * split;
+                unsigned m = 0;
+                int bij = 0, bik = 0, I = 0, fl = 0;
+                if (e < nE) {
+                    const int4 en = list[e];
+                    bij = en.x;
+                    I = en.y & 0xffffff;
+                    const int tI = en.z;
+                    int d = 0;
+                    bool in = true;
+                    const bool tr = I < J;                  // block stored as (J, I)
+                    if (PER) {
+                        const int iz = tI % (2 * rz + 1) - rz, iy = tI / (2 * rz + 1) % (2 * ry + 1) - ry,
+                                  ix = tI / ((2 * rz + 1) * (2 * ry + 1)) - rx;
+                        // translation of K seen from the root: T - T_I (of the root seen from K: T_I - T)
+                        const int sg = tr ? -1 : 1;
+                        const int dx = sg * (jx - ix), dy = sg * (jy - iy), dz = sg * (jz - iz);
+                        in = abs(dx) <= rx && abs(dy) <= ry && abs(dz) <= rz;
+                        d = ((dx + rx) * (2 * ry + 1) + (dy + ry)) * (2 * rz + 1) + dz + rz;
                     }
-                    // row entry of this lane (registers), column entries (warp tile)
-                    const int ea = 32 * ta + lane, eb = 32 * tb + lane;
-                    const bool arow = ea < m;
-                    Slot<R> A;
-                    if (arow) A = scr[ea];
-                    else {
-                        A = scr[0];
-                        A.c.x = R(0); A.s.w = R(0);
+                    if (in) {
+                        const long long cik = tr ? cbase + ((long long)J * (J + 1) / 2 + I) * nT + d
+                                                 : cbase + ((long long)I * (I + 1) / 2 + K) * nT + d;
+                        m = v.mask[cik];
+                        m = ((unsigned)en.y >> 24) & (tr ? m >> 8 : m & 0xffu);
+                        if (m) bik = (int)(v.map ? v.map[cik] : cik);
+                        fl = (tr ? 1 : 0) | (same && I == J ? 2 : 0) | tI << 2;
                     }
-                    __syncwarp();
-                    if (eb < m) {
-                        const Slot<R> Bown = diag ? A : scr[eb];
-                        tl.v[lane] = Bown.v; tl.l[lane] = Bown.l; tl.c[lane] = Bown.c; tl.s[lane] = Bown.s;
-                        tl.meta[lane] = Bown.meta;
-                    } else {
-                        tl.v[lane] = A.v; tl.l[lane] = A.l; tl.c[lane] = A.c; tl.s[lane] = A.s;
-                        tl.s[lane].w = R(0);
-                        tl.c[lane].x = R(0);
-                        tl.meta[lane] = A.meta;
+                }
+                int at = __popc(m);
+                int total = at;
+                {
+                    // exclusive prefix of the root counts
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const int x = __shfl_up_sync(kAll, total, o);
+                        if (lane >= o) total += x;
                     }
-                    __syncwarp();
-                    const C6Entry<R>* row_a = msys + (long long)(A.meta.x - a0) * nsys_n;
-                    const int t0 = diag ? 1 : 0, t1 = diag ? 16 : 31;
-                    R kS = R(0), kGx = R(0), kGy = R(0), kGz = R(0), kD = R(0);
-                    R rS = R(0), rGx = R(0), rGy = R(0), rGz = R(0), rD = R(0), rde = R(0);
-                    R te = R(0), txx = R(0), tyy = R(0), tzz = R(0), txy = R(0), txz = R(0), tyz = R(0);
-                    for (int st = t0; st <= t1; st++) {
-                        const int mm = (lane + st) & 31;
-                        const typename Vec4<R>::type Bv = tl.v[mm], Bl = tl.l[mm], Bc = tl.c[mm], Bs = tl.s[mm];
-                        const int4 Bm = tl.meta[mm];
-                        // C6 of the entry atoms (row a, column b): qrc = dC6/dCN_a / C6, qcr = dC6/dCN_b / C6
-                        const C6Entry<R> ejk = row_a[Bm.x - a0];
-                        // j-k vector: (x_k + T_k - x_i) - (x_j + T_j - x_i)
-                        R vx, vy, vz;
-                        if constexpr (sizeof(R) == 8) {
-                            vx = Bv.x - A.v.x; vy = Bv.y - A.v.y; vz = Bv.z - A.v.z;
-                        } else {
-                            vx = (Bv.x - A.v.x) + (Bl.x - A.l.x);
-                            vy = (Bv.y - A.v.y) + (Bl.y - A.l.y);
-                            vz = (Bv.z - A.v.z) + (Bl.z - A.l.z);
-                        }
-                        const R rc0 = vx * vx + vy * vy + vz * vz;   // r_jk^2
-                        bool valid = A.s.w != R(0) && Bs.w != R(0) && (!diag || st < 16 || lane < 16) &&
-                                     !(rc0 > cut2 || rc0 < R(DBL_EPSILON));
-                        // a step without any candidate inside the cutoff only moves the column sums
-                        // (not for non-periodic systems in the FP32 form, where the test costs more
-                        // than it saves)
-                        if ((sizeof(R) == 4 && !PER) || __any_sync(0xffffffffu, valid)) {
+                    at = total - at;
+                    total = __shfl_sync(kAll, total, 31);
+                }
+                if (m) {
+                    int p = head + cnt + at;
+                    while (m) {
+                        const int i = __ffs(m) - 1;
+                        m &= m - 1;
+                        sh.ring[p & (kRing - 1)] = make_int4(bij, bik, kT8 * (id.t8 + I) + i, fl);
+                        p++;
+                    }
+                }
+                cnt += total;
+            }
+            __syncwarp();
+            if (cnt == 0) break;
+            const int nroot = min(cnt, kRootChunk);
+            R Djk[kT8], Wjk[kT8];
+            R fj[4] = {R(0), R(0), R(0), R(0)}, fk[4] = {R(0), R(0), R(0), R(0)};   // force and dE/dCN of j, k
+            double vr[3] = {0, 0, 0};          // component (lane >> 1) & 3 of sum F_i (x) T_I
+            R esum = R(0);
+            int ntrip = 0;
+            if (GRAD)
+#pragma unroll
+                for (int t = 0; t < kT8; t++) { Djk[t] = R(0); Wjk[t] = R(0); }
+            auto fetch = [&](int r0) {
+                const int4 e = sh.ring[(head + min(r0 + q, nroot - 1)) & (kRing - 1)];
+                AtmStage<R>& s = sh.st[(r0 >> 2) & 1];
+                const int i8 = e.z & 7;
+                const int off = (e.w & 1) ? kT8 * j + i8 : kT8 * i8 + j;
+                async_copy_value(&s.ij[lane], rec + (long long)e.x * kRecs + off);
+                async_copy_value(&s.ik[lane], rec + (long long)e.y * kRecs + off);
+                if (GRAD) {
+                    async_copy_value(&s.qij[lane], aux + (long long)e.x * kRecs + off);
+                    async_copy_value(&s.qik[lane], aux + (long long)e.y * kRecs + off);
+                    if (j < 2) async_copy<16>(reinterpret_cast<char*>(&s.pos[q]) + 16 * j,
+                                              reinterpret_cast<const char*>(v.pos + e.z) + 16 * j);
+                    else if (PER && j < 5) async_copy<8>(&s.T[q][j - 2], img + 3 * (e.w >> 2) + j - 2);
+                }
+            };
+            fetch(0);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            for (int r0 = 0; r0 < nroot; r0 += 4) {
+                const bool rin = r0 + q < nroot;
+                if (r0 + 4 < nroot) fetch(r0 + 4);
+                asm volatile("cp.async.commit_group;\ncp.async.wait_group 1;" ::: "memory");
+                __syncwarp();
+                const AtmStage<R>& st = sh.st[(r0 >> 2) & 1];
+                const int4 e = sh.ring[(head + min(r0 + q, nroot - 1)) & (kRing - 1)];
+                Rec rij = st.ij[lane];
+                int ai = 0;
+                if (GEN) ai = v.sub[e.z];
+                if (!rin) { rij.z = R(0); if (GEN) rij.y = R(0); }
+                if (same && (e.w & 2)) rij.z *= R(1.0 / 3.0);
+                const R P6 = R(6) * rij.w, u38 = R(0.375) * rij.y;
+                R rK = R(0), rV = R(0), rE = R(0), kS = R(0), kE = R(0);
+#pragma unroll
+                for (int t = 0; t < kT8; t++) {
+                    if (diag && (t == 0 || t > 4)) continue;
+                    const Rec B = st.ik[qbase | ((j + t) & 7)];
+                    R M = rij.z * B.z * rjk[t].z;
+                    if (GEN) {
+                        const int okt = __shfl_sync(kAll, ok, qbase | ((j + t) & 7));
+                        const int akt = __shfl_sync(kAll, ak, qbase | ((j + t) & 7));
+                        bool valid = rij.y * B.y * rjk[t].y != R(0);
                         if (part.nparts > 1) {
                             // owner of the triple: the pair of its two largest input indices
-                            int o1 = orig_i, o2 = A.meta.w, o3 = Bm.w, tq;
-                            if (o2 > o1) { tq = o1; o1 = o2; o2 = tq; }
-                            if (o3 > o2) { tq = o2; o2 = o3; o3 = tq; }
-                            if (o2 > o1) { tq = o1; o1 = o2; o2 = tq; }
+                            int o1 = b.local[ai], o2 = oj, o3 = okt, w_;
+                            if (o2 > o1) { w_ = o1; o1 = o2; o2 = w_; }
+                            if (o3 > o2) { w_ = o2; o2 = o3; o3 = w_; }
+                            if (o2 > o1) { w_ = o1; o1 = o2; o2 = w_; }
                             valid = valid && owns_pair_atm(part, o1, o2);
                         }
-                        const int jat = A.meta.x, kat = Bm.x;
-                        // the reference's loop visits two images of one atom in both orders
-                        ntrip += valid ? (jat == kat ? 2 : 1) : 0;
-                        // triple_scale (atm.f90:954-980) of the atoms, twice for two images of one atom
-                        R triple = R(1);
-                        if (PER) {
-                            if (jat == kat) triple = (i == jat) ? R(2.0 / 6.0) : R(1);
-                            else triple = (i == jat || i == kat) ? R(0.5) : R(1);
-                        }
-                        const R rc = valid ? rc0 : R(1);
-                        const R ra = A.v.w, rb = Bv.w;               // r_ij^2, r_ik^2
-                        const R rsc = rsqrt_r<R>(rc);
-                        const R irc = rsc * rsc;
-                        const R ir1 = A.s.x * Bs.x * rsc;            // 1 / (r_ij r_ik r_jk)
-                        const R ir2 = ir1 * ir1;
-                        const R ir3 = ir2 * ir1;
-                        const R ir5 = ir3 * ir2;
-                        // (r0/r1)^alp3, r0 = r0ij r0ik r0jk, r1 = r_ij r_ik r_jk (atm.f90:744-749)
-                        const R tq = rexp<R>(A.c.w + Bc.w + ejk.lr0 - R(0.5) * alp3 * rlog<R>(rc));
-                        const R fdmp = rcp_r<R>(R(1) + R(6) * tq);
-                        const R s1 = ra + rb + rc;
-                        const R ang = R(0.375) * (s1 - R(2) * rb) * (s1 - R(2) * rc) * (s1 - R(2) * ra) * ir5 + ir3;
-                        const R c9 = valid ? -s9 * A.c.x * Bc.x * ejk.sc6 : R(0);
-                        R sw = R(1), swjk = R(1), dswjkr = R(0);
-                        if (SMOOTH) {
-                            R dsw;
-                            const R rjk = rc * rsc;
-                            smooth<R>(rjk, cutoff, width, swjk, dsw);
-                            dswjkr = dsw * rsc;
-                            sw = A.s.y * Bs.y * swjk;
-                        }
-                        const R c9f = c9 * fdmp;
-                        const R dE0 = ang * c9f;
-                        const R dE = (SMOOTH ? dE0 * sw : dE0) * triple;
-                        te -= dE;
-                        if (GRAD) {
-                            const R common = dE0 * (R(-2) * alp * tq * fdmp);
-                            const R kfac = R(0.375) * c9f * ir5;
-                            R sij = (common + kfac * ang_deriv<R>(ra, rc, rb, s1)) * A.l.w;
-                            R sik = (common + kfac * ang_deriv<R>(rb, rc, ra, s1)) * Bl.w;
-                            R sjk = (common + kfac * ang_deriv<R>(rc, rb, ra, s1)) * irc;
-                            if (SMOOTH) {
-                                sij = sij * sw - dE0 * A.s.z * Bs.y * swjk;
-                                sik = sik * sw - dE0 * Bs.z * A.s.y * swjk;
-                                sjk = sjk * sw - dE0 * dswjkr * A.s.y * Bs.y;
-                            }
-                            if (PER) { sij *= triple; sik *= triple; sjk *= triple; }
-                            const R gx = sjk * vx, gy = sjk * vy, gz = sjk * vz;
-                            // dE/dCN: root share here, entry shares through the entry sums
-                            const R hdE = R(0.5) * dE;
-                            rde -= hdE * (A.c.y + Bc.y);
-                            rS += sij; rGx -= gx; rGy -= gy; rGz -= gz;
-                            rD -= hdE * (A.c.z + ejk.qrc);
-                            kS += sik; kGx += gx; kGy += gy; kGz += gz;
-                            kD -= hdE * (Bc.z + ejk.qcr);
-                            txx += gx * vx; tyy += gy * vy; tzz += gz * vz;
-                            txy += gx * vy; txz += gx * vz; tyz += gy * vz;
-                        }
-                        }
-                        if (GRAD) {
-                            // the column's sums move one lane down, with the column
-                            const int src = (lane + 1) & 31;
-                            kS = __shfl_sync(0xffffffffu, kS, src);
-                            kGx = __shfl_sync(0xffffffffu, kGx, src);
-                            kGy = __shfl_sync(0xffffffffu, kGy, src);
-                            kGz = __shfl_sync(0xffffffffu, kGz, src);
-                            kD = __shfl_sync(0xffffffffu, kD, src);
-                        }
+                        if (!valid) M = R(0);
+                        // visits of the reference's loop (atm.f90:705-733), times three
+                        const int eq = (ai == aj) + (ai == akt) + (aj == akt);
+                        const int mult = eq == 3 ? 6 : eq ? 2 : 1;
+                        if (valid) ntrip += (e.w & 2) ? mult : 3 * mult;
                     }
-                    e_root += double(te);
-                    if (GRAD) {
-                        dei += double(rde);
-                        sxx += double(txx); syy += double(tyy); szz += double(tzz);
-                        sxy += double(txy); sxz += double(txz); syz += double(tyz);
-                        // entry sums: the row's in this lane, the column (lane + t1 + 1) mod 32's too
-                        if (arow) {
-                            double* ar = acc + (size_t)ea * kAcc;
-                            ar[0] += double(rS); ar[1] += double(rGx); ar[2] += double(rGy); ar[3] += double(rGz);
-                            ar[4] += double(rD);
-                        }
-                        const int ef = 32 * tb + ((lane + t1 + 1) & 31);
-                        if (ef < m) {
-                            double* ak = acc + (size_t)ef * kAcc;
-                            ak[0] += double(kS); ak[1] += double(kGx); ak[2] += double(kGy); ak[3] += double(kGz);
-                            ak[4] += double(kD);
-                        }
+                    const R x = rij.x, y = B.x, z = rjk[t].x;
+                    const R U = u38 * B.y * rjk[t].y;
+                    const R p6 = P6 * B.w * rjk[t].w;
+                    const R s = x + y, d = x - y;
+                    const R a1 = z + d, a2 = s - z, a3 = z - d;
+                    const R q1 = a1 * a2;
+                    const R A = q1 * a3 * U;
+                    const R f = rcp_fast(p6 + R(1));
+                    const R B1 = A + R(1);
+                    const R Mf = M * f;
+                    if constexpr (!GRAD) {
+                        rE = fma(Mf, B1, rE);
+                    } else {
+                        const R E = Mf * B1;
+                        const R q2 = a2 * a3, q3 = a1 * a3;
+                        const R KM = fma(B1, fma(p6 * f, ahalf, R(-1.5)), -A) * Mf;
+                        const R V = U * Mf;
+                        const R dq = q2 - q1, sq = q2 + q1;
+                        rK += KM;
+                        rV = fma(V, q3 + dq, rV);
+                        kS = fma(B.y, KM, kS);
+                        kS = fma(V, q3 - dq, kS);
+                        Djk[t] = fma(rjk[t].y, KM, Djk[t]);
+                        Djk[t] = fma(V, sq - q3, Djk[t]);
+                        rE += E;
+                        kE += E;
+                        Wjk[t] += E;
+                        // the sums of (i, k) move one lane down, with k
+                        kS = __shfl_sync(kAll, kS, qbase | ((j + 1) & 7));
+                        kE = __shfl_sync(kAll, kE, qbase | ((j + 1) & 7));
                     }
-                    __syncwarp();
                 }
-                __syncthreads();
+                esum += rE;
+                if constexpr (GRAD) {
+                    if (diag) {     // steps 1..4: column k ended in lane k - 5
+                        kS = __shfl_sync(kAll, kS, qbase | ((j + 3) & 7));
+                        kE = __shfl_sync(kAll, kE, qbase | ((j + 3) & 7));
+                    }
+                    R Dij = fma(rij.y, rK, rV), Dik = kS;
+                    if (smooth_on) {
+                        if (rE != R(0)) Dij += rE * dln_switch<R>(rij.x, cutoff, width);
+                        if (kE != R(0)) Dik += kE * dln_switch<R>(st.ik[lane].x, cutoff, width);
+                    }
+                    const double4 pi = st.pos[q];
+                    double tix = 0, tiy = 0, tiz = 0;
+                    if (PER) { tix = st.T[q][0]; tiy = st.T[q][1]; tiz = st.T[q][2]; }
+                    const double xi = pi.x + tix, yi = pi.y + tiy, zi = pi.z + tiz;
+                    const Aux qij = st.qij[lane], qik = st.qik[lane];
+                    const bool tr = e.w & 1;
+                    R g0, g1, g2, g3;
+                    {
+                        const R gx = Dij * R(xj - xi), gy = Dij * R(yj - yi), gz = Dij * R(zj - zi);
+                        fj[0] += gx; fj[1] += gy; fj[2] += gz;
+                        fj[3] = fma(rE, tr ? qij.x : qij.y, fj[3]);
+                        const R hx = Dik * R(xk - xi), hy = Dik * R(yk - yi), hz = Dik * R(zk - zi);
+                        fk[0] += hx; fk[1] += hy; fk[2] += hz;
+                        fk[3] = fma(kE, tr ? qik.x : qik.y, fk[3]);
+                        g0 = -(gx + hx); g1 = -(gy + hy); g2 = -(gz + hz);
+                        g3 = fma(rE, tr ? qij.y : qij.x, kE * (tr ? qik.y : qik.x));
+                    }
+                    // force (and dE/dCN) of the root: component (lane >> 1) & 3 summed over the quarter
+                    {
+                        const bool b2 = lane & 4, b1 = lane & 2;
+                        R k0 = sel(b2, g2, g0) + __shfl_xor_sync(kAll, sel(b2, g0, g2), 4);
+                        R k1 = sel(b2, g3, g1) + __shfl_xor_sync(kAll, sel(b2, g1, g3), 4);
+                        R kk = sel(b1, k1, k0) + __shfl_xor_sync(kAll, sel(b1, k0, k1), 2);
+                        kk += __shfl_xor_sync(kAll, kk, 1);
+                        const int comp = (lane >> 1) & 3;
+                        const double g = double(kk);
+                        if (PER) { vr[0] = fma(g, tix, vr[0]); vr[1] = fma(g, tiy, vr[1]); vr[2] = fma(g, tiz, vr[2]); }
+                        if (rin) {
+                            long long hi, lo;
+                            fixed_split(g, hi, lo);
+                            atomicAdd(fxf + (size_t)8 * (int)pi.w + 2 * comp + (lane & 1),
+                                      (unsigned long long)((lane & 1) ? lo : hi));
+                        }
+                    }
+                }
+                __syncwarp();       // the buffer is filled again two steps on
             }
-        }
-        // per-entry results: the root share stays in registers, the force and
-        // dE/dCN share of the entry's atom go to its fixed-point accumulators
-        double gix = 0, giy = 0, giz = 0;
-        if (GRAD && m > 1) {
-            for (int k = tid; k < m; k += kThreadsAtm) {
-                const double S = acc[k * kAcc + 0];
-                const double Gx = acc[k * kAcc + 1], Gy = acc[k * kAcc + 2], Gz = acc[k * kAcc + 3];
-                const double Dx = acc[k * kAcc + 4];
-                const double4 v = nbr_v[base + k];
-                gix -= S * v.x; giy -= S * v.y; giz -= S * v.z;
-                sxx += S * v.x * v.x; syy += S * v.y * v.y; szz += S * v.z * v.z;
-                sxy += S * v.x * v.y; sxz += S * v.x * v.z; syz += S * v.y * v.z;
-                unsigned long long* fx = fxacc + (size_t)8 * nbr_j[base + k];
-                fixed_add(fx + 0, S * v.x + Gx);
-                fixed_add(fx + 2, S * v.y + Gy);
-                fixed_add(fx + 4, S * v.z + Gz);
-                fixed_add(fx + 6, Dx);
+            head = (head + nroot) & (kRing - 1);
+            cnt -= nroot;
+            // ---- flush: energy, then the (j, k) sums and the forces of j and k
+            unsigned long long* fe = fxe + (size_t)20 * (id.t8 + J);
+            {
+                double es = double(esum);
+                for (int o = 16; o > 0; o >>= 1) es += __shfl_xor_sync(kAll, es, o);
+                if (lane == 0) fixed_add(fe, es);
+                if (GEN && counting) {
+                    for (int o = 16; o > 0; o >>= 1) ntrip += __shfl_xor_sync(kAll, ntrip, o);
+                    if (lane == 0) atomicAdd(queue + 1, (unsigned long long)ntrip);
+                }
             }
-        }
-        // block reduction of the root's sums in a fixed order
-        double r[12] = {e_root, gix, giy, giz, dei, sxx, syy, szz, sxy, sxz, syz, double(ntrip)};
-        for (int v = 0; v < 12; v++)
-            for (int o = 16; o > 0; o >>= 1) r[v] += __shfl_xor_sync(0xffffffffu, r[v], o);
-        if (lane == 0)
-            for (int v = 0; v < 12; v++) wsum[wid][v] = r[v];
-        __syncthreads();
-        if (tid == 0) {
-            double t[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
-            for (int wq = 0; wq < kWarps; wq++)
-                for (int v = 0; v < 12; v++) t[v] += wsum[wq][v];
-            e3[i] = t[0];
-            if (w.counts) atomicAdd(w.counts + 1, (unsigned long long)t[11]);
-            if (GRAD) {
-                unsigned long long* fx = fxacc + (size_t)8 * i;
-                fixed_add(fx + 0, t[1]);
-                fixed_add(fx + 2, t[2]);
-                fixed_add(fx + 4, t[3]);
-                fixed_add(fx + 6, t[4]);
-                for (int v = 0; v < 6; v++) sig3[kSigma * i + v] = t[5 + v];
+            if constexpr (GRAD) {
+                // quarter q keeps the steps t = q and q + 4, summed over the quarters
+                R Dt[2], Wt[2];
+                {
+                    const bool h16 = lane & 16, h8 = lane & 8;
+                    R D4[4], W4[4];     // steps (q & 2) + {0, 1, 4, 5}
+#pragma unroll
+                    for (int p = 0; p < 4; p++) {
+                        const int lo_t = (p & 1) + 4 * (p >> 1), hi_t = lo_t + 2;
+                        D4[p] = sel(h16, Djk[hi_t], Djk[lo_t]) +
+                                __shfl_xor_sync(kAll, sel(h16, Djk[lo_t], Djk[hi_t]), 16);
+                        W4[p] = sel(h16, Wjk[hi_t], Wjk[lo_t]) +
+                                __shfl_xor_sync(kAll, sel(h16, Wjk[lo_t], Wjk[hi_t]), 16);
+                    }
+#pragma unroll
+                    for (int p = 0; p < 2; p++) {
+                        Dt[p] = sel(h8, D4[2 * p + 1], D4[2 * p]) +
+                                __shfl_xor_sync(kAll, sel(h8, D4[2 * p], D4[2 * p + 1]), 8);
+                        Wt[p] = sel(h8, W4[2 * p + 1], W4[2 * p]) +
+                                __shfl_xor_sync(kAll, sel(h8, W4[2 * p], W4[2 * p + 1]), 8);
+                    }
+                }
+#pragma unroll
+                for (int p = 0; p < 2; p++) {
+                    const int t = q + 4 * p;
+                    const int kl = qbase | ((j + t) & 7), back = qbase | ((j - t) & 7);
+                    if (smooth_on && Wt[p] != R(0))
+                        Dt[p] += Wt[p] * dln_switch<R>(rec[bjk * kRecs + kT8 * j + ((j + t) & 7)].x, cutoff, width);
+                    const R gx = Dt[p] * R(__shfl_sync(kAll, xk, kl) - xj), gy = Dt[p] * R(__shfl_sync(kAll, yk, kl) - yj),
+                            gz = Dt[p] * R(__shfl_sync(kAll, zk, kl) - zj);
+                    const Aux qa = aux[bjk * kRecs + kT8 * j + ((j + t) & 7)];
+                    fj[0] -= gx; fj[1] -= gy; fj[2] -= gz;
+                    fj[3] = fma(Wt[p], qa.x, fj[3]);
+                    fk[0] += __shfl_sync(kAll, gx, back);
+                    fk[1] += __shfl_sync(kAll, gy, back);
+                    fk[2] += __shfl_sync(kAll, gz, back);
+                    fk[3] += __shfl_sync(kAll, Wt[p] * qa.y, back);
+                }
+                // quarter q keeps component q of j and of k
+                const bool h16 = lane & 16, h8 = lane & 8;
+                double cj, ck;
+                {
+                    R p0 = sel(h16, fj[2], fj[0]) + __shfl_xor_sync(kAll, sel(h16, fj[0], fj[2]), 16);
+                    R p1 = sel(h16, fj[3], fj[1]) + __shfl_xor_sync(kAll, sel(h16, fj[1], fj[3]), 16);
+                    cj = double(sel(h8, p1, p0) + __shfl_xor_sync(kAll, sel(h8, p0, p1), 8));
+                    p0 = sel(h16, fk[2], fk[0]) + __shfl_xor_sync(kAll, sel(h16, fk[0], fk[2]), 16);
+                    p1 = sel(h16, fk[3], fk[1]) + __shfl_xor_sync(kAll, sel(h16, fk[1], fk[3]), 16);
+                    ck = double(sel(h8, p1, p0) + __shfl_xor_sync(kAll, sel(h8, p0, p1), 8));
+                }
+                if (aj >= 0) fixed_add(fxf + (size_t)8 * aj + 2 * q, cj);
+                if (ak >= 0) fixed_add(fxf + (size_t)8 * ak + 2 * q, ck);
+                if (PER) {
+                    // sum of F (x) T over the images: the roots' and k's
+                    double kc = ck;
+                    for (int o = 4; o > 0; o >>= 1) kc += __shfl_xor_sync(kAll, kc, o);
+                    for (int d = 0; d < 3; d++)
+                        for (int o = 8; o <= 16; o <<= 1) vr[d] += __shfl_xor_sync(kAll, vr[d], o);
+                    // lane 2c of quarter 0 holds the roots' component c; quarter c holds k's
+                    const int comp = lane >> 1;
+                    const double kcc = __shfl_sync(kAll, kc, (8 * comp) & 31);
+                    if (lane < 6 && !(lane & 1)) {
+                        fixed_add(fe + 2 * (1 + 3 * comp), fma(kcc, kx, vr[0]));
+                        fixed_add(fe + 2 * (2 + 3 * comp), fma(kcc, ky, vr[1]));
+                        fixed_add(fe + 2 * (3 + 3 * comp), fma(kcc, kz, vr[2]));
+                    }
+                }
             }
+            __syncwarp();
         }
     }
 }
 
-// Adds the fixed-point three-body sums of every atom (gradient, dE/dCN) to
-// the FP64 gradient and dE/dCN.
-__global__ void k_atm_fixed(int natoms, const unsigned long long* fxacc, const int* guard, Work w)
+// Accumulators into the FP64 arrays, one thread per tile slot: gradient and
+// dE/dCN, and per atom the three-body energy and virial (the tile's first slot
+// takes the tile's energy and image terms).  The virial of all triples is
+// sum F_a (x) x_a over the atoms, at their images, the origin being free.
+__global__ void k_atm_finish(Batch b, Config c, AtmView v, int ntiles8, double s9, const unsigned long long* fxf,
+                             const unsigned long long* fxe, const unsigned long long* queue, const int* guard, Work w,
+                             double* e3, double* sig3)
 {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= natoms || *guard) return;
-    const unsigned long long* f = fxacc + (size_t)8 * x;
-    w.grad[3 * x + 0] += fixed_value(f + 0);
-    w.grad[3 * x + 1] += fixed_value(f + 2);
-    w.grad[3 * x + 2] += fixed_value(f + 4);
-    w.dEdcn[x] += fixed_value(f + 6);
+    pdl_wait();
+    const int slot = blockIdx.x * blockDim.x + threadIdx.x;
+    if (slot >= kT8 * ntiles8 || (guard && *guard)) return;
+    if (slot == 0 && w.counts) w.counts[1] += queue[1] / 3;
+    const int a = v.sub[slot];
+    if (a < 0) return;
+    const bool first = (slot & 7) == 0;
+    const unsigned long long* fe = fxe + (size_t)20 * (slot >> 3);
+    e3[a] = first ? s9 * fixed_value(fe) : 0.0;
+    if (!c.grad) return;
+    const unsigned long long* f = fxf + (size_t)8 * a;
+    const double g[3] = {2.0 * s9 * fixed_value(f), 2.0 * s9 * fixed_value(f + 2), 2.0 * s9 * fixed_value(f + 4)};
+    for (int k = 0; k < 3; k++) w.grad[3 * a + k] += g[k];
+    w.dEdcn[a] += s9 * fixed_value(f + 6);
+    const int o = b.atom_off[b.sys_of_atom[a]];
+    const double x = b.x[a] - b.x[o], y = b.y[a] - b.y[o], z = b.z[a] - b.z[o];
+    double s[kSigma] = {g[0] * x, g[1] * y, g[2] * z, 0.5 * (g[0] * y + g[1] * x), 0.5 * (g[0] * z + g[2] * x),
+                        0.5 * (g[1] * z + g[2] * y)};
+    if (first) {
+        double t[9];
+        for (int k = 0; k < 9; k++) t[k] = 2.0 * s9 * fixed_value(fe + 2 * (1 + k));
+        s[0] += t[0]; s[1] += t[4]; s[2] += t[8];
+        s[3] += 0.5 * (t[1] + t[3]); s[4] += 0.5 * (t[2] + t[6]); s[5] += 0.5 * (t[5] + t[7]);
+    }
+    for (int k = 0; k < kSigma; k++) sig3[kSigma * a + k] = s[k];
+}
+
+template <class R, bool GRAD, bool PER, bool GEN>
+int atm_configure()
+{
+    static const int blocks = [] {
+        const int smem = (int)sizeof(AtmShared<R>) * kAtmWarps;
+        cudaFuncSetAttribute(k_atm_triples<R, GRAD, PER, GEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        int n = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_atm_triples<R, GRAD, PER, GEN>, 32 * kAtmWarps, smem);
+        return n > 0 ? n : 1;
+    }();
+    return blocks;
+}
+
+template <class R, bool GRAD, bool PER>
+int atm_occupancy_of(bool gen) { return gen ? atm_configure<R, GRAD, PER, true>() : atm_configure<R, GRAD, PER, false>(); }
+
+template <class R, bool GRAD, bool PER, bool GEN>
+void triples_t(const AtmLaunch& l)
+{
+    atm_configure<R, GRAD, PER, GEN>();
+    launch_pdl(k_atm_triples<R, GRAD, PER, GEN>, dim3(l.blocks), dim3(32 * kAtmWarps),
+               sizeof(AtmShared<R>) * kAtmWarps, l.stream, l.b, l.c, l.part, l.v, l.alp3, l.split, l.grab, l.queue,
+               l.fxf, l.fxe, l.counting ? 1 : 0, l.guard);
+}
+
+template <class R, bool GRAD>
+void triples_g(const AtmLaunch& l)
+{
+    const bool gen = l.part.nparts > 1 || l.counting;
+    if (l.periodic) { if (gen) triples_t<R, GRAD, true, true>(l); else triples_t<R, GRAD, true, false>(l); }
+    else { if (gen) triples_t<R, GRAD, false, true>(l); else triples_t<R, GRAD, false, false>(l); }
 }
 
 }  // namespace
 
-void launch_atm_fixed(int natoms, const unsigned long long* fxacc, const int* guard, const Work& w,
-                      cudaStream_t stream)
+size_t atm_block_bytes(bool mixed, bool grad)
 {
-    if (natoms <= 0) return;
-    k_atm_fixed<<<(natoms + 255) / 256, 256, 0, stream>>>(natoms, fxacc, guard, w);
+    return kRecs * ((mixed ? sizeof(float4) : sizeof(double4)) + (grad ? (mixed ? sizeof(float2) : sizeof(double2)) : 0));
 }
 
-size_t atm_c6_entry_bytes(bool mixed) { return mixed ? sizeof(C6Entry<float>) : sizeof(C6Entry<double>); }
+size_t atm_rec_bytes(bool mixed) { return kRecs * (mixed ? sizeof(float4) : sizeof(double4)); }
 
-void launch_c6_matrix(const Batch& b, const Species& s, const Work& w, const void* U, double alp3,
-                      const long long* d_mat_off, void* mat, long long total, bool mixed, cudaStream_t stream)
+int atm_warps_per_block() { return kAtmWarps; }
+
+int atm_blocks_per_sm(bool mixed, bool grad, bool periodic, bool gen)
 {
-    if (total <= 0 || b.natoms <= 0) return;
-    const unsigned blocks = (unsigned)((b.natoms + 7) / 8);
-    if (mixed)
-        k_c6_matrix<float><<<blocks, 256, 0, stream>>>(b, s, w, (const float*)U, alp3, d_mat_off, (C6Entry<float>*)mat);
-    else
-        k_c6_matrix<double><<<blocks, 256, 0, stream>>>(b, s, w, (const double*)U, alp3, d_mat_off,
-                                                        (C6Entry<double>*)mat);
+    if (mixed) {
+        if (grad) return periodic ? atm_occupancy_of<float, true, true>(gen) : atm_occupancy_of<float, true, false>(gen);
+        return periodic ? atm_occupancy_of<float, false, true>(gen) : atm_occupancy_of<float, false, false>(gen);
+    }
+    if (grad) return periodic ? atm_occupancy_of<double, true, true>(gen) : atm_occupancy_of<double, true, false>(gen);
+    return periodic ? atm_occupancy_of<double, false, true>(gen) : atm_occupancy_of<double, false, false>(gen);
 }
 
-void launch_nbr_count(const Batch& b, const Config& c, const uint8_t* sys_skip, int* cnt, int* max_cnt,
-                      cudaStream_t stream)
-{
-    if (b.natoms <= 0) return;
-    k_nbr_count<<<(b.natoms + 7) / 8, 256, 0, stream>>>(b, c, sys_skip, cnt, max_cnt);
-}
-
-size_t scan_temp_bytes(int n)
+size_t atm_scan_temp_bytes(long long n)
 {
     size_t bytes = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, bytes, (const int*)nullptr, (long long*)nullptr, n + 1);
+    cub::DeviceScan::ExclusiveSum(nullptr, bytes, (const int*)nullptr, (int*)nullptr, (int)(n + 1));
     return bytes;
 }
 
-void launch_scan(void* temp, size_t temp_bytes, const int* cnt_ext, long long* off, int n, cudaStream_t stream)
-{
-    // cnt_ext has n + 1 entries (last is 0): off[n] is the total
-    cub::DeviceScan::ExclusiveSum(temp, temp_bytes, cnt_ext, off, n + 1, stream);
-}
-
-void launch_atm_guard(const long long* total, const int* max_cnt, long long cap, int stride, int* guard,
+void launch_atm_order(const Batch& b, const int* tile_off, const int* tile_sys, int ntiles, const AtmView& v,
+                      double4* spheres, unsigned long long* fxf, unsigned long long* fxe, unsigned long long* queue,
                       cudaStream_t stream)
 {
-    k_atm_guard<<<1, 1, 0, stream>>>(total, max_cnt, cap, stride, guard);
+    if (ntiles <= 0) return;
+    launch_pdl(k_atm_order, dim3((ntiles + 3) / 4), dim3(128), 0, stream, b, tile_off, tile_sys, ntiles, v, spheres, fxf,
+               fxe, queue);
 }
 
-void launch_nbr_fill(const Batch& b, const Config& c, const uint8_t* sys_skip, const long long* off, const int* cnt,
-                     int* nbr_j, int* nbr_gend, double4* nbr_v, const int* guard, cudaStream_t stream)
+void launch_atm_mark(const Batch& b, const Config& c, const AtmView& v, const double4* spheres, int* flag, int* map,
+                     void* temp, size_t temp_bytes, cudaStream_t stream)
 {
-    if (b.natoms <= 0) return;
-    k_nbr_fill<<<(b.natoms + 7) / 8, 256, 0, stream>>>(b, c, sys_skip, off, cnt, nbr_j, nbr_gend, nbr_v, guard);
+    cudaMemsetAsync(flag + v.ncand, 0, sizeof(int), stream);
+    k_atm_mark<<<(unsigned)((v.ncand + 127) / 128), 128, 0, stream>>>(b, c, v, spheres, flag);
+    cub::DeviceScan::ExclusiveSum(temp, temp_bytes, flag, map, (int)(v.ncand + 1), stream);
 }
 
-template <class R>
-size_t triple_smem()
+void launch_atm_guard(const int* total, long long cap, int* guard, cudaStream_t stream)
 {
-    return sizeof(EntryTile<R>) * (kThreadsAtm / 32);
+    k_atm_guard<<<1, 1, 0, stream>>>(total, cap, guard);
 }
 
-template <class R, bool GRAD, bool PER, bool SMOOTH>
-int triple_occupancy_of()
+void launch_atm_pairs(const Batch& b, const Species& s, const Config& c, const Work& w, const AtmView& v, const void* U,
+                      double alp3, const int* guard, cudaStream_t stream)
 {
-    static bool configured = false;
-    if (!configured) {
-        cudaFuncSetAttribute(k_triples<R, GRAD, PER, SMOOTH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)triple_smem<R>());
-        configured = true;
-    }
-    int n = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_triples<R, GRAD, PER, SMOOTH>, kThreadsAtm, triple_smem<R>());
-    return n > 0 ? n : 1;
+    if (v.ncand <= 0) return;
+    const unsigned blocks = (unsigned)((v.ncand + 7) / 8);
+    if (c.mixed) launch_pdl(k_atm_pairs<float>, dim3(blocks), dim3(256), 0, stream, b, s, c, w, v, (const float*)U, alp3, guard);
+    else launch_pdl(k_atm_pairs<double>, dim3(blocks), dim3(256), 0, stream, b, s, c, w, v, (const double*)U, alp3, guard);
 }
 
-template <class R, bool GRAD>
-int triple_occupancy()
+void launch_atm_lists(const AtmView& v, int ntiles8, const int* tile8_sys, const long long* list_off, int4* list,
+                      int2* range, const int* guard, cudaStream_t stream)
 {
-    // every variant is configured; the occupancy is the smallest of them
-    return std::min(std::min(triple_occupancy_of<R, GRAD, false, false>(), triple_occupancy_of<R, GRAD, true, false>()),
-                    std::min(triple_occupancy_of<R, GRAD, false, true>(), triple_occupancy_of<R, GRAD, true, true>()));
+    if (ntiles8 <= 0) return;
+    launch_pdl(k_atm_lists, dim3((ntiles8 + 3) / 4), dim3(128), 0, stream, v, ntiles8, tile8_sys, list_off, list, range,
+               guard);
 }
 
-int atm_blocks_per_sm(bool mixed, bool grad)
+void launch_atm_triples(const AtmLaunch& l)
 {
-    if (mixed) return grad ? triple_occupancy<float, true>() : triple_occupancy<float, false>();
-    return grad ? triple_occupancy<double, true>() : triple_occupancy<double, false>();
+    if (l.v.ncand <= 0) return;
+    if (l.c.mixed) { if (l.c.grad) triples_g<float, true>(l); else triples_g<float, false>(l); }
+    else { if (l.c.grad) triples_g<double, true>(l); else triples_g<double, false>(l); }
 }
 
-size_t atm_slot_bytes(bool mixed) { return mixed ? sizeof(Slot<float>) : sizeof(Slot<double>); }
-
-template <class R, bool GRAD, bool PER, bool SMOOTH>
-void launch_triples_t(const Batch& b, const Species& s, const Damp& d, const Config& c, const Partition& p,
-                      const Work& w, const void* mat, const long long* mat_off, const long long* off, const int* cnt,
-                      const int* nbr_j, const int* nbr_gend, const double4* nbr_v, unsigned int* queue,
-                      double* slot_acc, void* slot_scr, int slot_stride, int blocks, double* e3, double* sig3,
-                      unsigned long long* fxacc, cudaStream_t stream)
+void launch_atm_finish(const Batch& b, const Config& c, const AtmView& v, int ntiles8, double s9,
+                       const unsigned long long* fxf, const unsigned long long* fxe, const unsigned long long* queue,
+                       const int* guard, const Work& w, double* e3, double* sig3, cudaStream_t stream)
 {
-    triple_occupancy_of<R, GRAD, PER, SMOOTH>();
-    k_triples<R, GRAD, PER, SMOOTH><<<blocks, kThreadsAtm, triple_smem<R>(), stream>>>(
-        b, s, d, c, p, w, (const C6Entry<R>*)mat, mat_off, off, cnt, nbr_j, nbr_gend, nbr_v, queue, slot_acc,
-        (Slot<R>*)slot_scr, slot_stride, e3, sig3, fxacc);
-}
-
-template <class R, bool GRAD>
-void launch_triples_g(const Batch& b, const Species& s, const Damp& d, const Config& c, const Partition& p,
-                      const Work& w, const void* mat, const long long* mat_off, const long long* off, const int* cnt,
-                      const int* nbr_j, const int* nbr_gend, const double4* nbr_v, unsigned int* queue,
-                      double* slot_acc, void* slot_scr, int slot_stride, int blocks, bool periodic, double* e3,
-                      double* sig3, unsigned long long* fxacc, cudaStream_t stream)
-{
-    const bool smooth_on = c.width3 > 0.0 && c.width3 < c.cut3;
-#define D3_TRIPLES(P, S)                                                                                     \
-    launch_triples_t<R, GRAD, P, S>(b, s, d, c, p, w, mat, mat_off, off, cnt, nbr_j, nbr_gend, nbr_v, queue,  \
-                                    slot_acc, slot_scr, slot_stride, blocks, e3, sig3, fxacc, stream)
-    if (periodic) { if (smooth_on) D3_TRIPLES(true, true); else D3_TRIPLES(true, false); }
-    else { if (smooth_on) D3_TRIPLES(false, true); else D3_TRIPLES(false, false); }
-#undef D3_TRIPLES
-}
-
-void launch_triples(const Batch& b, const Species& s, const Damp& d, const Config& c, const Partition& p,
-                    const Work& w, const void* mat, const long long* mat_off, const long long* off, const int* cnt,
-                    const int* nbr_j, const int* nbr_gend, const double4* nbr_v, unsigned int* queue,
-                    double* slot_acc, void* slot_scr, int slot_stride, int blocks, bool periodic, double* e3,
-                    double* sig3, unsigned long long* fxacc, cudaStream_t stream)
-{
-    if (b.natoms <= 0) return;
-    if (c.mixed) {
-        if (c.grad) launch_triples_g<float, true>(b, s, d, c, p, w, mat, mat_off, off, cnt, nbr_j, nbr_gend, nbr_v, queue, slot_acc, slot_scr, slot_stride, blocks, periodic, e3, sig3, fxacc, stream);
-        else launch_triples_g<float, false>(b, s, d, c, p, w, mat, mat_off, off, cnt, nbr_j, nbr_gend, nbr_v, queue, slot_acc, slot_scr, slot_stride, blocks, periodic, e3, sig3, fxacc, stream);
-    } else {
-        if (c.grad) launch_triples_g<double, true>(b, s, d, c, p, w, mat, mat_off, off, cnt, nbr_j, nbr_gend, nbr_v, queue, slot_acc, slot_scr, slot_stride, blocks, periodic, e3, sig3, fxacc, stream);
-        else launch_triples_g<double, false>(b, s, d, c, p, w, mat, mat_off, off, cnt, nbr_j, nbr_gend, nbr_v, queue, slot_acc, slot_scr, slot_stride, blocks, periodic, e3, sig3, fxacc, stream);
-    }
+    if (ntiles8 <= 0) return;
+    launch_pdl(k_atm_finish, dim3((kT8 * ntiles8 + 127) / 128), dim3(128), 0, stream, b, c, v, ntiles8, s9, fxf, fxe,
+               queue, guard, w, e3, sig3);
 }
 
 }  // namespace d3

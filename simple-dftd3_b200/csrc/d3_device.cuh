@@ -150,17 +150,13 @@ struct Work {
                                  // pairs (the stored-sum CN pass; virial = sum dE/dCN_i cn_sig_i)
     double* pg_atom = nullptr;   // [natoms][kParamGrad] or null
     unsigned long long* counts = nullptr;  // [3] pair, triple, cn terms or null
-    // three-body results per root atom (summed by the per-system reduction)
-    double* e3_atom = nullptr;   // [natoms] three-body energy of the root's triples
-    double* sig3_atom = nullptr; // [natoms][kSigma] three-body virial of the root's triples
+    // three-body results per atom (summed by the per-system reduction)
+    double* e3_atom = nullptr;   // [natoms] three-body energy
+    double* sig3_atom = nullptr; // [natoms][kSigma] three-body virial
     // dE/ds9 of the parameter derivatives: pg_s9_scale * sum of e3_pg (the
     // three-body energy at the current s9, or at s9 = 1 when s9 vanishes)
     const double* e3_pg = nullptr;
     double pg_s9_scale = 0.0;
-    // capacity guard of the three-body lists: set when the neighbour entries
-    // exceed the reserved buffers (captured launch sequences); the list fill
-    // and the triple sum then skip their work
-    int* atm_guard = nullptr;
 };
 
 struct Config {
@@ -179,9 +175,8 @@ struct Tuning {
                                    // with keys quantised to cells of this many Bohr
     int pair_split = 0;            // work items per tile pair of the pair sweeps: 1, 2 or 4; 0 = 1 for
                                    // molecules, else 2 (mixed form) or 4 (FP64 form)
-    int atm_blocks_per_sm = 0;     // resident blocks per SM of the neighbour-list triple kernel; 0 = occupancy
-    int atm_mol = 0;               // molecule triple kernel: 0 for batches of at least one molecule per SM,
-                                   // 1 for every eligible system, 2 never
+    int atm_blocks_per_sm = 0;     // resident blocks per SM of the triple kernel; 0 = occupancy
+    int atm_mol = 0;               // 0, 1 or 2: accepted for callers that set it, one kernel serves all systems
 };
 
 // Pairwise decomposition (d3_pairwise.cu), FP64: energy2 and energy3 of every
@@ -290,44 +285,68 @@ void launch_two_body_units(const Batch& b, const Species& s, const Damp& d, cons
                            const Work& w, const PairUnits& pu, cudaStream_t stream, cudaEvent_t ev_begin = nullptr,
                            cudaEvent_t ev_end = nullptr, bool species_ready = false);
 
-// Three-body term (d3_atm.cu): C6 table, neighbour lists, triple sum.
-size_t atm_c6_entry_bytes(bool mixed);
-// From the species vectors U (launch_species_vectors) and the weights.
-void launch_c6_matrix(const Batch& b, const Species& s, const Work& w, const void* U, double alp3,
-                      const long long* d_mat_off, void* mat, long long total, bool mixed, cudaStream_t stream);
-// sys_skip[nsys] (or null): systems whose roots get no entries (handled by
-// the molecule kernel)
-void launch_nbr_count(const Batch& b, const Config& c, const uint8_t* sys_skip, int* cnt, int* max_cnt,
+// Three-body term (d3_atm.cu).  Tiles of 8 atoms and candidate blocks: the
+// systems in processing order (largest first) have, for every tile pair
+// (A, B <= A) and every three-body lattice translation, one candidate block of
+// 64 pair records.
+struct AtmView {
+    int nord = 0;                          // systems
+    long long ncand = 0;                   // candidate blocks
+    const long long* cand_off = nullptr;   // [nord] first candidate of each system, in processing order
+    const int* ord = nullptr;              // [nord] system at each processing position
+    const int* rep = nullptr;              // [nsys][4] translations -r..r along each vector, their number
+    const int* t8_off = nullptr;           // [nsys + 1] first tile of each system
+    const long long* cand_off_sys = nullptr;   // [nsys] the same by system
+    int* sub = nullptr;                    // [ntiles8][8] atom of each tile slot, or -1
+    double4* pos = nullptr;                // [ntiles8][8] its position, and the atom
+    const long long* list_off = nullptr;   // [nsys] first root list entry
+    const int4* list = nullptr;            // root tiles of tile J of a system: from list_off + J nt8 nT
+    const int2* range = nullptr;           // [ntiles8] first entry with I > J, number of entries
+    const int* map = nullptr;              // [ncand + 1] block of each candidate (a kept one raises the next
+                                           // entry), or null: every candidate has its block
+    unsigned short* mask = nullptr;        // [ncand] rows (bits 0-7) and columns (8-15) with a pair in reach
+    void* rec = nullptr;                   // [blocks][64] pair records (4 values)
+    void* aux = nullptr;                   // [blocks][64] CN derivatives (2 values)
+};
+struct AtmLaunch {
+    Batch b;
+    Config c;
+    Partition part;
+    AtmView v;
+    double alp3 = 0.0;                     // (alp + 2) / 3
+    int split = 1;                         // warps that share the roots of a unit
+    int grab = 1;                          // units taken from the queue at a time
+    int blocks = 1;
+    bool periodic = false, counting = false;
+    unsigned long long *queue = nullptr;   // [2] next unit, counted triples x 3
+    unsigned long long *fxf = nullptr;     // [natoms][4][2] fixed-point force / (2 s9), dE/dCN / s9
+    unsigned long long *fxe = nullptr;     // [ntiles8][10][2] energy / s9, sum of F (x) T / (2 s9)
+    const int* guard = nullptr;            // set: the blocks did not fit, skip the work
+    cudaStream_t stream = nullptr;
+};
+size_t atm_block_bytes(bool mixed, bool grad);   // records and CN derivatives of one block
+size_t atm_rec_bytes(bool mixed);                // the records alone
+int atm_warps_per_block();
+int atm_blocks_per_sm(bool mixed, bool grad, bool periodic, bool gen);
+size_t atm_scan_temp_bytes(long long ncand);
+// Tile order; clears the accumulators and the queue.  spheres: [ntiles8] or null.
+void launch_atm_order(const Batch& b, const int* tile_off, const int* tile_sys, int ntiles, const AtmView& v,
+                      double4* spheres, unsigned long long* fxf, unsigned long long* fxe, unsigned long long* queue,
                       cudaStream_t stream);
-size_t scan_temp_bytes(int n);
-void launch_scan(void* temp, size_t temp_bytes, const int* cnt_ext, long long* off, int n,
-                 cudaStream_t stream);
-// Sets *guard when off[natoms] (the entry total) exceeds cap or the longest
-// list exceeds stride; the fill and triple kernels then return at once.
-void launch_atm_guard(const long long* total, const int* max_cnt, long long cap, int stride, int* guard,
-                      cudaStream_t stream);
-void launch_nbr_fill(const Batch& b, const Config& c, const uint8_t* sys_skip, const long long* off, const int* cnt,
-                     int* nbr_j, int* nbr_gend, double4* nbr_v, const int* guard, cudaStream_t stream);
-int atm_blocks_per_sm(bool mixed, bool grad);
-size_t atm_slot_bytes(bool mixed);
-// With gradients the force and dE/dCN share of every entry's atom and of the
-// root go to fxacc[natoms][4][2] (fixed point, zeroed before the launch);
-// launch_atm_fixed then adds them to the gradient and dE/dCN.
-void launch_triples(const Batch& b, const Species& s, const Damp& d, const Config& c, const Partition& p,
-                    const Work& w, const void* mat, const long long* mat_off, const long long* off,
-                    const int* cnt, const int* nbr_j, const int* nbr_gend, const double4* nbr_v,
-                    unsigned int* queue, double* slot_acc, void* slot_scr, int slot_stride, int blocks,
-                    bool periodic, double* e3, double* sig3, unsigned long long* fxacc, cudaStream_t stream);
-void launch_atm_fixed(int natoms, const unsigned long long* fxacc, const int* guard, const Work& w,
-                      cudaStream_t stream);
-// Three-body term of whole molecules, one block per system (d3_atm_mol.cu):
-// the non-periodic systems of at most atm_mol_max_atoms() atoms listed in
-// mol_order (largest first).  Writes e3/sig3 for every atom of those systems.
-int atm_mol_max_atoms();
-int atm_mol_blocks_per_sm(bool mixed, bool grad);
-void launch_triples_mol(const Batch& b, const Species& s, const Damp& d, const Config& c, const Partition& p,
-                        const Work& w, const void* mat, const long long* mat_off, const int* mol_order, int nmol,
-                        unsigned int* queue, int blocks, double* e3, double* sig3, cudaStream_t stream);
+// Candidates in reach of the cutoff and their block numbers: map[ncand] is the total.
+void launch_atm_mark(const Batch& b, const Config& c, const AtmView& v, const double4* spheres, int* flag, int* map,
+                     void* temp, size_t temp_bytes, cudaStream_t stream);
+// Sets *guard when the total exceeds cap; the kernels below then return at once.
+void launch_atm_guard(const int* total, long long cap, int* guard, cudaStream_t stream);
+void launch_atm_pairs(const Batch& b, const Species& s, const Config& c, const Work& w, const AtmView& v, const void* U,
+                      double alp3, const int* guard, cudaStream_t stream);
+void launch_atm_lists(const AtmView& v, int ntiles8, const int* tile8_sys, const long long* list_off, int4* list,
+                      int2* range, const int* guard, cudaStream_t stream);
+void launch_atm_triples(const AtmLaunch& l);
+// Adds the gradient and dE/dCN, writes e3 and sig3 (and the triple count).
+void launch_atm_finish(const Batch& b, const Config& c, const AtmView& v, int ntiles8, double s9,
+                       const unsigned long long* fxf, const unsigned long long* fxe, const unsigned long long* queue,
+                       const int* guard, const Work& w, double* e3, double* sig3, cudaStream_t stream);
 void launch_cn_chain_rule(const Batch& b, const Species& s, const Config& c, const Partition& p,
                           const Work& w, cudaStream_t stream,
                           bool direct = false);

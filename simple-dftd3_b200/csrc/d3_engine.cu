@@ -88,9 +88,10 @@ double ref_c6(int iref, int jref, int ati, int atj)
 
 }  // namespace
 
-std::vector<double> lattice_points(const double* lattice, const bool* periodic, double rthr)
+std::vector<double> lattice_points(const double* lattice, const bool* periodic, double rthr, int* rep_out)
 {
     const int np = (int)periodic[0] + (int)periodic[1] + (int)periodic[2];
+    if (rep_out) rep_out[0] = rep_out[1] = rep_out[2] = 0;
     if (np == 0) return {0.0, 0.0, 0.0};
     double lat[3][3];
     for (int k = 0; k < 3; k++)
@@ -115,6 +116,7 @@ std::vector<double> lattice_points(const double* lattice, const bool* periodic, 
         for (int k = 0; k < 3; k++)
             if (!periodic[k]) rep[k] = 0;
     }
+    if (rep_out) std::copy(rep, rep + 3, rep_out);
     std::vector<double> t;
     t.reserve(3 * (2 * rep[0] + 1) * (2 * rep[1] + 1) * (2 * rep[2] + 1));
     for (int ix = -rep[0]; ix <= rep[0]; ix++)
@@ -280,7 +282,7 @@ Engine::Engine(int nsys, const int* natoms, const int* numbers, const double* la
     d_tile_sys_ = dev_alloc<int>(std::max(ntiles_, 1));
     up(d_tile_off_, tile_off.data(), sizeof(int) * (nsys + 1));
     up(d_tile_sys_, tile_sys.data(), sizeof(int) * ntiles_);
-    // three-body dense blocks per system
+    // dense blocks per system (pairwise decomposition)
     c6mat_off_.assign(nsys, 0);
     long long off = 0;
     for (int s = 0; s < nsys; s++) {
@@ -293,9 +295,9 @@ Engine::Engine(int nsys, const int* natoms, const int* numbers, const double* la
     for (int sy = 0; sy < nsys; sy++)
         if (per_[3 * sy] || per_[3 * sy + 1] || per_[3 * sy + 2]) auto_split_ = 2;
     any_periodic_ = auto_split_ == 2;
-    d_mol_order_ = dev_alloc<int>(nsys);
-    d_sys_mol_ = dev_alloc<uint8_t>(nsys);
-    configure_molecules();
+    t8_off_.assign(nsys + 1, 0);
+    for (int sy = 0; sy < nsys; sy++) t8_off_[sy + 1] = t8_off_[sy] + (natoms[sy] + 7) / 8;
+    ntiles8_ = t8_off_[nsys];
     check(cudaStreamSynchronize(stream_), "upload sync");
 }
 
@@ -310,37 +312,9 @@ Engine::~Engine()
     if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
     for (void* p : allocations_) cudaFree(p);
     if (h_stage_) cudaFreeHost(h_stage_);
-    if (h_atm_counts_) cudaFreeHost(h_atm_counts_);
+    if (h_atm_total_) cudaFreeHost(h_atm_total_);
     if (h_guard_) cudaFreeHost(h_guard_);
     if (stream_) cudaStreamDestroy(stream_);
-}
-
-void Engine::configure_molecules()
-{
-    // molecules for the block-per-system three-body kernel: no periodic
-    // direction and at most atm_mol_max_atoms() atoms, largest first
-    std::vector<uint8_t> is_mol(nsys_, 0);
-    mol_order_.clear();
-    root_atoms_ = 0;
-    for (int s = 0; s < nsys_; s++) {
-        const bool per_any = per_[3 * s] || per_[3 * s + 1] || per_[3 * s + 2];
-        if (tune_.atm_mol != 2 && !per_any && sys_natoms_[s] <= atm_mol_max_atoms()) mol_order_.push_back(s);
-        else root_atoms_ += sys_natoms_[s];
-    }
-    // one block per molecule pays off for many molecules; a few are spread
-    // over all SMs by the neighbour-list kernel instead
-    if (tune_.atm_mol == 0 && (int)mol_order_.size() < sms_) {
-        for (int sy : mol_order_) root_atoms_ += sys_natoms_[sy];
-        mol_order_.clear();
-    }
-    std::stable_sort(mol_order_.begin(), mol_order_.end(),
-                     [&](int a, int b) { return sys_natoms_[a] > sys_natoms_[b]; });
-    for (int sy : mol_order_) is_mol[sy] = 1;
-    check(cudaStreamSynchronize(stream_), "molecules");
-    if (!mol_order_.empty())
-        check(cudaMemcpy(d_mol_order_, mol_order_.data(), sizeof(int) * mol_order_.size(), cudaMemcpyHostToDevice),
-              "molecule order");
-    check(cudaMemcpy(d_sys_mol_, is_mol.data(), nsys_, cudaMemcpyHostToDevice), "molecule flags");
 }
 
 void Engine::build_tables(const int* numbers)
@@ -449,10 +423,17 @@ void Engine::ensure_images(cudaStream_t stream)
     const double rthr[kImageKinds] = {cut_.cn, cut_.disp2, cut_.disp3};
     std::vector<int> off(kImageKinds * (nsys_ + 1), 0);
     std::vector<double> all;
+    img_rep_.assign(4 * (size_t)nsys_, 0);
+    atm_layout_valid_ = false;
     for (int k = 0; k < kImageKinds; k++) {
         for (int s = 0; s < nsys_; s++) {
             off[k * (nsys_ + 1) + s] = (int)(all.size() / 3);
-            std::vector<double> t = lattice_points(&lat_[9 * s], &per_[3 * s], rthr[k]);
+            int rep[3];
+            std::vector<double> t = lattice_points(&lat_[9 * s], &per_[3 * s], rthr[k], rep);
+            if (k == kImgDisp3) {
+                std::copy(rep, rep + 3, &img_rep_[4 * s]);
+                img_rep_[4 * s + 3] = (int)(t.size() / 3);
+            }
             all.insert(all.end(), t.begin(), t.end());
         }
         off[k * (nsys_ + 1) + nsys_] = (int)(all.size() / 3);
@@ -912,102 +893,178 @@ void Engine::free_block(void*& p)
     p = nullptr;
 }
 
+// Candidate blocks of the three-body sum: for every system, in the order of
+// their size, the tile pairs times the three-body translations.
+void Engine::ensure_atm_layout(cudaStream_t stream)
+{
+    if (!atm_ready_) {
+        const size_t n = std::max(natoms_, 1), n8 = std::max(ntiles8_, 1);
+        d_cand_off_ = dev_alloc<long long>(nsys_);
+        d_cand_off_sys_ = dev_alloc<long long>(nsys_);
+        d_list_off_ = dev_alloc<long long>(nsys_);
+        d_pos8_ = dev_alloc<double4>(8 * n8);
+        d_tile8_sys_ = dev_alloc<int>(n8);
+        d_atm_range_ = dev_alloc<int2>(n8);
+        d_atm_ord_ = dev_alloc<int>(nsys_);
+        d_atm_rep_ = dev_alloc<int>(4 * (size_t)nsys_);
+        d_t8_off_ = dev_alloc<int>(nsys_ + 1);
+        d_sub8_ = dev_alloc<int>(8 * n8);
+        d_spheres8_ = dev_alloc<double4>(n8);
+        d_e3_ = dev_alloc<double>(n);
+        d_sig3_ = dev_alloc<double>(kSigma * n);
+        d_fxf_ = dev_alloc<unsigned long long>(8 * n);
+        d_fxe_ = dev_alloc<unsigned long long>(20 * n8);
+        d_atm_queue_ = dev_alloc<unsigned long long>(2);
+        d_guard_ = dev_alloc<int>(1);
+        check(cudaMallocHost(&h_atm_total_, sizeof(int)), "cudaMallocHost");
+        check(cudaMemsetAsync(d_guard_, 0, sizeof(int), stream), "memset");
+        check(cudaMemcpyAsync(d_t8_off_, t8_off_.data(), sizeof(int) * (nsys_ + 1), cudaMemcpyHostToDevice, stream),
+              "three-body tiles");
+        std::vector<int> tile8_sys(ntiles8_);
+        for (int sy = 0; sy < nsys_; sy++)
+            std::fill(tile8_sys.begin() + t8_off_[sy], tile8_sys.begin() + t8_off_[sy + 1], sy);
+        check(cudaMemcpyAsync(d_tile8_sys_, tile8_sys.data(), sizeof(int) * ntiles8_, cudaMemcpyHostToDevice, stream),
+              "three-body tiles");
+        check(cudaStreamSynchronize(stream), "three-body tiles");
+        atm_ready_ = true;
+        atm_layout_valid_ = false;
+    }
+    if (atm_layout_valid_) return;
+    std::vector<int> ord(nsys_);
+    std::iota(ord.begin(), ord.end(), 0);
+    std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return sys_natoms_[a] > sys_natoms_[b]; });
+    std::vector<long long> off(nsys_), off_sys(nsys_), list_off(nsys_);
+    long long total = 0, entries = 0;
+    for (int k = 0; k < nsys_; k++) {
+        const long long nt = t8_off_[ord[k] + 1] - t8_off_[ord[k]], nT = img_rep_[4 * (size_t)ord[k] + 3];
+        off[k] = off_sys[ord[k]] = total;
+        list_off[ord[k]] = entries;
+        total += nt * (nt + 1) / 2 * nT;
+        entries += nt * nt * nT;
+    }
+    if (total > 0x7ffffff0LL) throw Error("The system is too large for the three-body term");
+    check(cudaMemcpyAsync(d_atm_ord_, ord.data(), sizeof(int) * nsys_, cudaMemcpyHostToDevice, stream), "order");
+    check(cudaMemcpyAsync(d_cand_off_, off.data(), sizeof(long long) * nsys_, cudaMemcpyHostToDevice, stream),
+          "candidates");
+    check(cudaMemcpyAsync(d_cand_off_sys_, off_sys.data(), sizeof(long long) * nsys_, cudaMemcpyHostToDevice, stream),
+          "candidates");
+    check(cudaMemcpyAsync(d_list_off_, list_off.data(), sizeof(long long) * nsys_, cudaMemcpyHostToDevice, stream),
+          "root lists");
+    check(cudaMemcpyAsync(d_atm_rep_, img_rep_.data(), sizeof(int) * 4 * nsys_, cudaMemcpyHostToDevice, stream),
+          "translations");
+    if (total > atm_cand_cap_) {
+        void* p = d_atm_mask_;
+        free_block(p);
+        atm_cand_cap_ = total + total / 4 + 16;
+        d_atm_mask_ = dev_alloc<unsigned short>(atm_cand_cap_);
+    }
+    if (entries > atm_list_cap_) {
+        void* p = d_atm_list_;
+        free_block(p);
+        atm_list_cap_ = entries + entries / 4 + 16;
+        d_atm_list_ = dev_alloc<int4>(atm_list_cap_);
+    }
+    // the host vectors go out of scope: make the copies complete first
+    check(cudaStreamSynchronize(stream), "three-body layout");
+    atm_.nord = nsys_;
+    // kernel arguments of a captured sequence: a new number of candidates needs a new capture
+    if (total != atm_.ncand) graph_valid_ = false;
+    atm_.ncand = total;
+    atm_.cand_off = d_cand_off_;
+    atm_.cand_off_sys = d_cand_off_sys_;
+    atm_.pos = d_pos8_;
+    atm_.list_off = d_list_off_;
+    atm_.list = d_atm_list_;
+    atm_.range = d_atm_range_;
+    atm_.ord = d_atm_ord_;
+    atm_.rep = d_atm_rep_;
+    atm_.t8_off = d_t8_off_;
+    atm_.sub = d_sub8_;
+    atm_.mask = d_atm_mask_;
+    atm_layout_valid_ = true;
+}
+
+bool Engine::atm_compact(bool mixed) const
+{
+    return (size_t)atm_.ncand * atm_block_bytes(mixed, true) > kAtmDenseCap;
+}
+
 void Engine::run_three_body(const Batch& b, const Species& s, const Damp& d, const Config& c, Work& w,
                             cudaStream_t stream)
 {
-    const int n = natoms_;
-    if (!atm_ready_) {
-        d_c6mat_off_ = dev_alloc<long long>(nsys_);
-        check(cudaMemcpy(d_c6mat_off_, c6mat_off_.data(), sizeof(long long) * nsys_, cudaMemcpyHostToDevice),
-              "c6 offsets");
-        // sized for the FP64 entries, which also hold the FP32 ones
-        d_c6mat_ = dev_alloc<unsigned char>(atm_c6_entry_bytes(false) * (size_t)std::max<long long>(c6mat_total_, 1));
-        d_cnt_ = dev_alloc<int>(n + 1);
-        d_off_ = dev_alloc<long long>(n + 1);
-        d_maxcnt_ = dev_alloc<int>(1);
-        d_queue_ = dev_alloc<unsigned int>(2);   // root queue, molecule queue
-        d_e3_ = dev_alloc<double>(n);
-        d_sig3_ = dev_alloc<double>((size_t)kSigma * n);
-        d_fxacc_ = dev_alloc<unsigned long long>((size_t)8 * n);
-        scan_bytes_ = scan_temp_bytes(n);
-        d_scan_temp_ = dev_alloc<unsigned char>(scan_bytes_);
-        check(cudaMallocHost(&h_atm_counts_, 2 * sizeof(long long)), "cudaMallocHost");
-        d_guard_ = dev_alloc<int>(1);
-        check(cudaMemsetAsync(d_guard_, 0, sizeof(int), stream), "memset");
-        atm_ready_ = true;
-    }
+    ensure_atm_layout(stream);
     // the two-body pass computed the species vectors; without it they are computed here
     if (!species_ready_) launch_species_vectors(b, s, c, w, pu_.U, stream);
-    launch_c6_matrix(b, s, w, pu_.U, (d.alp + 2.0) / 3.0, d_c6mat_off_, d_c6mat_, c6mat_total_, c.mixed, stream);
-    if (root_atoms_ > 0) {
-        check(cudaMemsetAsync(d_maxcnt_, 0, sizeof(int), stream), "memset");
-        check(cudaMemsetAsync(d_cnt_ + n, 0, sizeof(int), stream), "memset");
-        launch_nbr_count(b, c, d_sys_mol_, d_cnt_, d_maxcnt_, stream);
-        launch_scan(d_scan_temp_, scan_bytes_, d_cnt_, d_off_, n, stream);
-        const int blocks = std::max(1, std::min(n, sms_ * atm_blocks(c.mixed, c.grad)));
-        int stride = atm_stride_;
-        if (!capturing_) {
-            check(cudaMemcpyAsync(h_atm_counts_, d_off_ + n, sizeof(long long), cudaMemcpyDeviceToHost, stream), "total");
-            check(cudaMemcpyAsync(h_atm_counts_ + 1, d_maxcnt_, sizeof(int), cudaMemcpyDeviceToHost, stream), "max");
-            check(cudaStreamSynchronize(stream), "neighbour count");
-            const long long total = h_atm_counts_[0];
-            const int maxcnt = (int)(reinterpret_cast<int*>(h_atm_counts_ + 1)[0]);
-            last_triples_entries_ = total;
-            if (total > nbr_cap_) {
-                void* pj = d_nbr_j_; void* pgd = d_nbr_gend_; void* pv = d_nbr_v_;
-                free_block(pj); free_block(pgd); free_block(pv);
-                nbr_cap_ = total + total / 4 + 1024;
-                d_nbr_j_ = dev_alloc<int>(nbr_cap_);
-                d_nbr_gend_ = dev_alloc<int>(nbr_cap_);
-                d_nbr_v_ = dev_alloc<double4>(nbr_cap_);
-            }
-            // a captured sequence keeps the list length it was captured with: reserve headroom
-            stride = std::max(maxcnt, 1);
-            if (graph_on_) {
-                if (maxcnt > atm_stride_) atm_stride_ = maxcnt + maxcnt / 4 + 32;
-                stride = atm_stride_;
-            }
-            // the slot buffers are sized for the largest resident grid (one block per SM and unit of occupancy)
-            const long long grid = (long long)sms_ * std::max(atm_occupancy(c.mixed, true), atm_occupancy(c.mixed, false));
-            const long long need = grid * stride * 8;   // per-entry accumulators (up to 8 doubles)
-            if (need > slot_cap_) {
-                void* p = d_slot_acc_;
-                free_block(p);
-                slot_cap_ = need + need / 4;
-                d_slot_acc_ = dev_alloc<double>(slot_cap_);
-            }
-            const long long scr_need = grid * stride * (long long)atm_slot_bytes(false);
-            if (scr_need > slot_scr_cap_) {
-                void* p = d_slot_scr_;
-                free_block(p);
-                slot_scr_cap_ = scr_need + scr_need / 4;
-                d_slot_scr_ = dev_alloc<unsigned char>(slot_scr_cap_);
-            }
+    const bool compact = atm_compact(c.mixed);
+    const size_t rec = atm_rec_bytes(c.mixed), aux = atm_block_bytes(c.mixed, true) - rec;
+    AtmView v = atm_;
+    launch_atm_order(b, d_tile_off_, d_tile_sys_, ntiles_, v, compact ? d_spheres8_ : nullptr,
+                     c.grad ? d_fxf_ : nullptr, d_fxe_, d_atm_queue_, stream);
+    long long blocks = v.ncand;
+    if (compact) {
+        if (v.ncand > atm_flag_cap_) {
+            void *pf = d_atm_flag_, *pm = d_atm_map_;
+            free_block(pf); free_block(pm); free_block(d_scan_temp_);
+            atm_flag_cap_ = atm_cand_cap_;
+            d_atm_flag_ = dev_alloc<int>(atm_flag_cap_ + 1);
+            d_atm_map_ = dev_alloc<int>(atm_flag_cap_ + 1);
+            scan_bytes_ = atm_scan_temp_bytes(atm_flag_cap_);
+            d_scan_temp_ = dev_alloc<unsigned char>(scan_bytes_);
         }
-        launch_atm_guard(d_off_ + n, d_maxcnt_, nbr_cap_, stride, d_guard_, stream);
-        launch_nbr_fill(b, c, d_sys_mol_, d_off_, d_cnt_, d_nbr_j_, d_nbr_gend_, d_nbr_v_, d_guard_, stream);
-        check(cudaMemsetAsync(d_queue_, 0, sizeof(unsigned int), stream), "memset");
-        w.atm_guard = d_guard_;
-        if (profiling_ && !capturing_) check(cudaEventRecord(kev_[2], stream), "cudaEventRecord");
-        if (c.grad) check(cudaMemsetAsync(d_fxacc_, 0, sizeof(unsigned long long) * 8 * n, stream), "memset");
-        launch_triples(b, s, d, c, part_, w, d_c6mat_, d_c6mat_off_, d_off_, d_cnt_, d_nbr_j_, d_nbr_gend_, d_nbr_v_,
-                       d_queue_, d_slot_acc_, d_slot_scr_, stride, blocks, any_periodic_, d_e3_, d_sig3_, d_fxacc_,
-                       stream);
-        if (c.grad) launch_atm_fixed(n, d_fxacc_, d_guard_, w, stream);
+        launch_atm_mark(b, c, v, d_spheres8_, d_atm_flag_, d_atm_map_, d_scan_temp_, scan_bytes_, stream);
+        v.map = d_atm_map_;
+        if (!capturing_) {
+            check(cudaMemcpyAsync(h_atm_total_, d_atm_map_ + v.ncand, sizeof(int), cudaMemcpyDeviceToHost, stream), "total");
+            check(cudaStreamSynchronize(stream), "block count");
+            blocks = *h_atm_total_;
+        }
     }
-    if (!mol_order_.empty()) {
-        // after the root kernel, which writes zeros for the molecules' atoms
-        if (profiling_ && !capturing_ && root_atoms_ == 0) check(cudaEventRecord(kev_[2], stream), "cudaEventRecord");
-        const int nmol = (int)mol_order_.size();
-        const int mblocks = std::max(1, std::min(nmol, sms_ * atm_mol_occupancy(c.mixed, c.grad)));
-        check(cudaMemsetAsync(d_queue_ + 1, 0, sizeof(unsigned int), stream), "memset");
-        launch_triples_mol(b, s, d, c, part_, w, d_c6mat_, d_c6mat_off_, d_mol_order_, nmol, d_queue_ + 1, mblocks,
-                           d_e3_, d_sig3_, stream);
+    if (!capturing_) {
+        auto reserve = [&](void*& p, size_t& cap, size_t need) {
+            if (need <= cap) return;
+            free_block(p);
+            cap = compact ? need + need / 4 : need;
+            p = dev_alloc<unsigned char>(cap);
+        };
+        reserve(d_atm_rec_, atm_rec_cap_, (size_t)std::max<long long>(blocks, 1) * rec);
+        if (c.grad) reserve(d_atm_aux_, atm_aux_cap_, (size_t)std::max<long long>(blocks, 1) * aux);
     }
+    const int* guard = nullptr;
+    if (compact) {
+        size_t cap = atm_rec_cap_ / rec;
+        if (c.grad) cap = std::min(cap, atm_aux_cap_ / aux);
+        launch_atm_guard(d_atm_map_ + v.ncand, (long long)cap, d_guard_, stream);
+        guard = d_guard_;
+    }
+    v.rec = d_atm_rec_;
+    v.aux = d_atm_aux_;
+    AtmLaunch l;
+    l.b = b; l.c = c; l.part = part_; l.v = v;
+    l.alp3 = (d.alp + 2.0) / 3.0;     // ATM exponent alp + 2 (rational.f90:563)
+    l.periodic = any_periodic_;
+    l.counting = w.counts != nullptr;
+    l.queue = d_atm_queue_; l.fxf = d_fxf_; l.fxe = d_fxe_; l.guard = guard; l.stream = stream;
+    const bool gen = part_.nparts > 1 || l.counting;
+    int occ = atm_blocks_per_sm(c.mixed, c.grad, l.periodic, gen);
+    if (tune_.atm_blocks_per_sm > 0) occ = std::min(occ, tune_.atm_blocks_per_sm);
+    const long long warps = (long long)sms_ * occ * atm_warps_per_block();
+    // few units: several warps share the roots of one
+    long long most = 1;
+    for (int sy = 0; sy < nsys_; sy++)
+        most = std::max(most, (long long)(t8_off_[sy + 1] - t8_off_[sy]) * img_rep_[4 * (size_t)sy + 3]);
+    l.split = (int)std::max<long long>(1, std::min(most, (2 * warps + v.ncand) / std::max<long long>(v.ncand, 1)));
+    l.grab = v.ncand > 256 * warps ? 8 : 1;
+    const long long units = v.ncand * l.split;
+    l.blocks = (int)std::max<long long>(1, std::min<long long>((long long)sms_ * occ, (units + atm_warps_per_block() - 1) / atm_warps_per_block()));
+    launch_atm_pairs(b, s, c, w, v, pu_.U, l.alp3, guard, stream);
+    launch_atm_lists(v, ntiles8_, d_tile8_sys_, d_list_off_, d_atm_list_, d_atm_range_, guard, stream);
+    if (profiling_ && !capturing_) check(cudaEventRecord(kev_[2], stream), "cudaEventRecord");
+    launch_atm_triples(l);
     if (profiling_ && !capturing_) {
         check(cudaEventRecord(kev_[3], stream), "cudaEventRecord");
         kev3_recorded_ = true;
     }
+    launch_atm_finish(b, c, v, ntiles8_, d.s9, d_fxf_, d_fxe_, d_atm_queue_, guard, w, d_e3_, d_sig3_, stream);
     w.e3_atom = d_e3_;
     w.sig3_atom = c.grad ? d_sig3_ : nullptr;
 }
@@ -1027,26 +1084,6 @@ void Engine::stage_times(double out[kTimes])
     (void)cudaGetLastError();
     if (kev3_recorded_ && cudaEventElapsedTime(&ms, kev_[2], kev_[3]) == cudaSuccess) out[kStages + 1] = ms;
     (void)cudaGetLastError();
-}
-
-int Engine::atm_occupancy(bool mixed, bool grad)
-{
-    int& occ = atm_occ_[mixed ? 1 : 0][grad ? 1 : 0];
-    if (occ == 0) occ = atm_blocks_per_sm(mixed, grad);
-    return occ;
-}
-
-int Engine::atm_mol_occupancy(bool mixed, bool grad)
-{
-    int& occ = atm_mol_occ_[mixed ? 1 : 0][grad ? 1 : 0];
-    if (occ == 0) occ = atm_mol_blocks_per_sm(mixed, grad);
-    return occ;
-}
-
-int Engine::atm_blocks(bool mixed, bool grad)
-{
-    const int occ = atm_occupancy(mixed, grad);
-    return tune_.atm_blocks_per_sm > 0 ? std::min(tune_.atm_blocks_per_sm, occ) : occ;
 }
 
 // ------------------------------------------------------------------ graph --
@@ -1101,9 +1138,7 @@ void Engine::set_tuning(const Tuning& t)
     if (t.atm_blocks_per_sm < 0) throw Error("Three-body blocks per SM must not be negative");
     if (t.atm_mol < 0 || t.atm_mol > 2) throw Error("Molecule kernel mode must be 0, 1 or 2");
     check(cudaSetDevice(device_), "cudaSetDevice");
-    const bool remol = t.atm_mol != tune_.atm_mol;
     tune_ = t;
-    if (remol) configure_molecules();
     graph_valid_ = false;
 }
 
@@ -1179,10 +1214,11 @@ void Engine::run_graphed(const Damp& d, bool grad, bool pg, cudaStream_t stream)
     upload_pair_table(d, stream);
     const GraphKey key = make_key(d, grad, pg);
     const bool threebody = std::fabs(d.s9) >= DBL_EPSILON || pg;
+    if (threebody) ensure_atm_layout(stream);
     if (graph_valid_ && graph_epoch_ == alloc_epoch_ && std::memcmp(&key, &graph_key_, sizeof(key)) == 0) {
         check(cudaGraphLaunch(graph_exec_, stream), "cudaGraphLaunch");
-        if (!threebody) return;
-        // the three-body lists must have fitted the buffers the graph was captured with
+        if (!threebody || !atm_compact(mixed_)) return;
+        // the three-body blocks must have fitted the buffers the graph was captured with
         check(cudaMemcpyAsync(h_guard_, d_guard_, sizeof(int), cudaMemcpyDeviceToHost, stream), "guard");
         check(cudaStreamSynchronize(stream), "graph");
         if (*h_guard_ == 0) return;
@@ -1243,38 +1279,19 @@ double Engine::autotune(const Damp& d, const double* d_positions, bool grad, cud
         for (int sp : {1, 2, 4})
             if (sp != best.pair_split) { Tuning t = best; t.pair_split = sp; consider(t); }
         if (threebody) {
-            // molecules: one block each, or the neighbour-list kernel
-            bool any_mol = false;
-            for (int sy = 0; sy < nsys_; sy++)
-                any_mol = any_mol || (!(per_[3 * sy] || per_[3 * sy + 1] || per_[3 * sy + 2]) &&
-                                      sys_natoms_[sy] <= atm_mol_max_atoms());
-            if (any_mol)
-                for (int mode : {1, 2})
-                    if (mode != best.atm_mol) {
-                        Tuning t = best; t.atm_mol = mode;
-                        const bool remol = t.atm_mol != tune_.atm_mol;
-                        tune_ = t;
-                        if (remol) configure_molecules();
-                        const double ms = time_once();
-                        if (ms < best_ms) { best_ms = ms; best = t; }
-                        tune_ = best;
-                        configure_molecules();
-                    }
-            const int occ = atm_occupancy(mixed_, grad);
+            const int occ = atm_blocks_per_sm(mixed_, grad, any_periodic_, part_.nparts > 1);
             const int cur = best.atm_blocks_per_sm > 0 ? std::min(best.atm_blocks_per_sm, occ) : occ;
             for (int bps = 1; bps <= occ; bps++)
                 if (bps != cur) { Tuning t = best; t.atm_blocks_per_sm = bps; consider(t); }
         }
     } catch (...) {
         tune_ = best;
-        configure_molecules();
         profiling_ = prof;
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         throw;
     }
     tune_ = best;
-    configure_molecules();
     profiling_ = prof;
     graph_valid_ = false;
     cudaEventDestroy(e0);

@@ -32,7 +32,8 @@ struct Error : std::runtime_error {
 
 // Lattice translations within rthr (get_lattice_points, cutoff.f90:140-227).
 // lattice[3][3] holds one vector per row; periodic[3].
-std::vector<double> lattice_points(const double* lattice, const bool* periodic, double rthr);
+// rep (or null): the translations run over -rep[k]..rep[k] along vector k.
+std::vector<double> lattice_points(const double* lattice, const bool* periodic, double rthr, int* rep = nullptr);
 
 // Wrap positions into the central cell (wrap_to_central_cell, utils.f90:29-64).
 void wrap_to_central_cell(int nat, double* xyz, const double* lattice, const bool* periodic);
@@ -100,11 +101,11 @@ public:
 
     // Captured launch sequence.  With the graph on, an evaluation replays one
     // CUDA graph of the whole pipeline (sort, CN, weights, two-body, three-body
-    // lists and sum, chain rule, reductions) from engine-owned input/output
+    // blocks and sum, chain rule, reductions) from engine-owned input/output
     // buffers.  The first evaluation of a (parameters, derivatives, tuning)
-    // key runs the ordinary sequence, which sizes the three-body lists, and
+    // key runs the ordinary sequence, which sizes the three-body blocks, and
     // then captures the graph with 25% headroom on those buffers; a replay
-    // whose lists outgrow them is detected by a device flag and evaluated
+    // whose blocks outgrow them is detected by a device flag and evaluated
     // again without the graph, and the graph is captured anew.
     void set_graph(bool on);
     bool graph() const { return graph_on_; }
@@ -125,7 +126,7 @@ public:
     using Reducer = int (*)(double* buffer, int count, void* stream, void* user);
     void set_reducer(Reducer fn, void* user, int part, int nparts);
 
-    // Launch shapes (spatial sort cell, atoms per pair block, resident triple
+    // Launch shapes (spatial sort cell, items per tile pair, resident triple
     // blocks per SM).  autotune() times the candidates on the given device
     // positions and keeps the fastest; it returns that time in ms.
     void set_tuning(const Tuning& t);
@@ -182,28 +183,19 @@ private:
     void run_graphed(const Damp& d, bool grad, bool pg, cudaStream_t stream);
     void capture(const Damp& d, const GraphKey& key, bool grad, bool pg);
     void drop_graph();
-    int atm_blocks(bool mixed, bool grad);      // resident triple blocks per SM (tuned)
-    int atm_occupancy(bool mixed, bool grad);   // occupancy limit
-    int atm_mol_occupancy(bool mixed, bool grad);
-    int atm_mol_occ_[2][2] = {{0, 0}, {0, 0}};
     // two-body tile-pair units
     PairUnits pu_;
     int2* d_units_ = nullptr;
     int* d_unit_base_ = nullptr;
-    std::vector<int> mol_order_;         // systems of the molecule kernel, largest first
-    int* d_mol_order_ = nullptr;
     std::vector<int> sys_natoms_;
     int auto_split_ = 1;                 // pair split of tuning 0
     int pair_split() const;              // items per tile pair of the two-body sweep
     int cn_split() const;                // items per tile pair of the CN sweeps
     bool any_periodic_ = false;          // a system has a periodic direction
-    void configure_molecules();          // mol_order_ and root_atoms_ from tune_.atm_mol
     // systems small enough for the direct pair kernels (see direct_pairs)
     static constexpr int kDirectMaxAtoms = DIRECT_MAX_ATOMS;
     static constexpr int kDirectMaxTotal = DIRECT_MAX_TOTAL;
     bool direct_pairs(const Damp& d, bool pg) const;
-    uint8_t* d_sys_mol_ = nullptr;       // [nsys] 1 for those systems
-    long long root_atoms_ = 0;           // atoms of the other systems
     bool graph_on_ = false, capturing_ = false, graph_valid_ = false;
     cudaGraphExec_t graph_exec_ = nullptr;
     long long graph_kernels_ = 0;
@@ -211,11 +203,9 @@ private:
     unsigned long long alloc_epoch_ = 0, graph_epoch_ = 0;
     int* d_guard_ = nullptr;
     int* h_guard_ = nullptr;     // pinned
-    int atm_stride_ = 0;         // reserved per-root list length of captured three-body sums
     double* d_pg_out_ = nullptr;
     Tuning tune_;
     int sms_ = 0;
-    int atm_occ_[2][2] = {{0, 0}, {0, 0}};
 
     int device_ = 0;
     int nsys_ = 0, natoms_ = 0, max_sys_atoms_ = 0;
@@ -278,32 +268,40 @@ private:
     // three-body
     void run_three_body(const Batch& b, const Species& s, const Damp& d, const Config& c, Work& w,
                         cudaStream_t stream);
+    void ensure_atm_layout(cudaStream_t stream);
+    bool atm_compact(bool mixed) const;
     void free_block(void*& p);
-    std::vector<long long> c6mat_off_;
+    // blocks above this size are kept for the tile pairs in reach only
+    static constexpr size_t kAtmDenseCap = size_t(1) << 30;
+    std::vector<long long> c6mat_off_;   // dense [n_s][n_s] blocks of the pairwise decomposition
     long long c6mat_total_ = 0;
-    long long* d_c6mat_off_ = nullptr;
-    void* d_c6mat_ = nullptr;
-    int* d_cnt_ = nullptr;
-    long long* d_off_ = nullptr;
-    int* d_maxcnt_ = nullptr;
-    unsigned int* d_queue_ = nullptr;
+    int ntiles8_ = 0;
+    std::vector<int> t8_off_;
+    std::vector<int> img_rep_;           // [nsys][4] three-body translations of each system
+    bool atm_layout_valid_ = false;
+    AtmView atm_;
+    long long *d_cand_off_ = nullptr, *d_cand_off_sys_ = nullptr, *d_list_off_ = nullptr;
+    double4* d_pos8_ = nullptr;
+    int* d_tile8_sys_ = nullptr;
+    int4* d_atm_list_ = nullptr;
+    int2* d_atm_range_ = nullptr;
+    long long atm_list_cap_ = 0;
+    int *d_atm_ord_ = nullptr, *d_atm_rep_ = nullptr, *d_t8_off_ = nullptr, *d_sub8_ = nullptr;
+    double4* d_spheres8_ = nullptr;
+    unsigned short* d_atm_mask_ = nullptr;
+    long long atm_cand_cap_ = 0;
+    int *d_atm_flag_ = nullptr, *d_atm_map_ = nullptr;
     void* d_scan_temp_ = nullptr;
     size_t scan_bytes_ = 0;
-    int* d_nbr_j_ = nullptr;
-    int* d_nbr_gend_ = nullptr;
-    double4* d_nbr_v_ = nullptr;
-    long long nbr_cap_ = 0;
-    double* d_slot_acc_ = nullptr;
-    long long slot_cap_ = 0;
-    void* d_slot_scr_ = nullptr;
-    long long slot_scr_cap_ = 0;
+    long long atm_flag_cap_ = 0;
+    void *d_atm_rec_ = nullptr, *d_atm_aux_ = nullptr;
+    size_t atm_rec_cap_ = 0, atm_aux_cap_ = 0;        // bytes
     double* d_e3_ = nullptr;
     double* d_sig3_ = nullptr;
-    unsigned long long* d_fxacc_ = nullptr;   // [natoms][4][2] fixed-point three-body gradient, dE/dCN
-    long long* h_atm_counts_ = nullptr;   // pinned: total entries, largest list
+    unsigned long long *d_atm_queue_ = nullptr, *d_fxf_ = nullptr, *d_fxe_ = nullptr;
+    int* h_atm_total_ = nullptr;         // pinned: kept blocks
     bool atm_ready_ = false;
     bool species_ready_ = false;   // PairUnits::U holds this evaluation's species vectors
-    long long last_triples_entries_ = 0;
 };
 
 }  // namespace d3
