@@ -54,6 +54,14 @@ constexpr int kAtmWarps = 4;            // warps per block of the triple kernel
 constexpr int kRing = 512;              // root queue of a warp: up to 127 left over + 32 tiles of 8
 constexpr int kRootChunk = 128;         // roots between two flushes: FP32 sums run over at most 32 terms
 
+// Resident blocks per SM the triple kernel is compiled for.  FP32 with gradient:
+// 168 registers and 12 warps beat 128 registers (spills) and 16 warps, 54.8
+// against 59.1 ms on eight frames; FP64 with gradient: 254 registers and 8 warps
+// beat 168 and 12 (cluster of 5000 atoms 15.5 against 17.7 ms); energies: 16 and
+// 12 warps beat 20 and 16 (slab 0.63 against 0.74 ms).
+template <class R, bool GRAD>
+constexpr int kTripleBlocks = sizeof(R) == 4 ? (GRAD ? 3 : 4) : (GRAD ? 2 : 3);
+
 template <class R> struct RecT;
 template <> struct RecT<double> { using rec = double4; using aux = double2; };
 template <> struct RecT<float> { using rec = float4; using aux = float2; };
@@ -104,9 +112,57 @@ __device__ __forceinline__ double rcp_fast(double x)
 {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x, y, 1.0);
-    return fma(y, fma(e, e, e), y);
+    const double e = ::fma(-x, y, 1.0);
+    return ::fma(y, ::fma(e, e, e), y);
 }
+
+// Two values worked on together: the packed FP32 instructions of sm_100 (one
+// issue slot for two operations), or a plain pair in FP64.
+struct F2 { unsigned long long v; };
+struct D2 { double a, b; };
+template <class R> struct PairT;
+template <> struct PairT<float> { using type = F2; };
+template <> struct PairT<double> { using type = D2; };
+
+__device__ __forceinline__ F2 pk(float a, float b)
+{
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ D2 pk(double a, double b) { return D2{a, b}; }
+__device__ __forceinline__ float lo(F2 x) { return __uint_as_float((unsigned)x.v); }
+__device__ __forceinline__ float hi(F2 x) { return __uint_as_float((unsigned)(x.v >> 32)); }
+__device__ __forceinline__ double lo(D2 x) { return x.a; }
+__device__ __forceinline__ double hi(D2 x) { return x.b; }
+__device__ __forceinline__ F2 operator+(F2 x, F2 y)
+{
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(x.v), "l"(y.v));
+    return r;
+}
+__device__ __forceinline__ F2 operator-(F2 x, F2 y)
+{
+    F2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(x.v), "l"(y.v));
+    return r;
+}
+__device__ __forceinline__ F2 operator*(F2 x, F2 y)
+{
+    F2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(x.v), "l"(y.v));
+    return r;
+}
+__device__ __forceinline__ F2 fma(F2 x, F2 y, F2 z)
+{
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(x.v), "l"(y.v), "l"(z.v));
+    return r;
+}
+__device__ __forceinline__ D2 operator+(D2 x, D2 y) { return D2{x.a + y.a, x.b + y.b}; }
+__device__ __forceinline__ D2 operator-(D2 x, D2 y) { return D2{x.a - y.a, x.b - y.b}; }
+__device__ __forceinline__ D2 operator*(D2 x, D2 y) { return D2{x.a * y.a, x.b * y.b}; }
+__device__ __forceinline__ D2 fma(D2 x, D2 y, D2 z) { return D2{::fma(x.a, y.a, z.a), ::fma(x.b, y.b, z.b)}; }
 
 // Candidate block c of the processing order: system, tile pair (A >= B, local
 // tile indices) and translation index.
@@ -441,7 +497,9 @@ struct AtmStage {
 template <class R>
 struct AtmShared {
     AtmStage<R> st[2];
-    int4 ring[kRing];                // roots: block (i, j), block (i, k), tile slot, flags and translation
+    float4 xu[32], mp[32];           // FP32: (i, k) records of k and k ^ 4, {x, x', u, u'} and {m, m', P, P'}
+    int4 ring[kRing];                // roots: first record (i, j) and (i, k), tile slot, flags and translation
+    double4 pj[kT8], pk[kT8];        // positions of the atoms j and (at their image) k
 };
 
 template <int BYTES>
@@ -461,18 +519,21 @@ __device__ __forceinline__ void async_copy_value(V* dst, const V* src)
     }
 }
 
-// What bounds it: issue slots and dependent latencies (FP32: 2.5 instructions per
-// cycle and SM; FP64: 1.5, the FP64 pipe at 46%).  Per lane slot 42 arithmetic
-// instructions, one reciprocal, two (FP32) or four shuffles and one or two 16-byte
-// shared loads, 62 in all with the work per four roots; the (j, k) records and sums
-// stay in registers.  Whole evaluations, the neighbour-list and block-per-molecule
-// kernels that this one replaced against it (185 instructions per slot, exp, log
-// and divisions per triple in FP64): cluster of 5000 atoms (FP64) 54.0 -> 16.8 ms,
-// 512 molecules (FP64) 21.4 -> 2.1 ms, 4096 molecules (mixed) 13.9 -> 7.5 ms, eight
-// periodic frames (mixed) 149 -> 64 ms, one molecule of 100 atoms 216 -> 85 us.
+// What bounds it: dependent latencies and the issue of the work per four roots (22
+// of 47 instructions per step of 32 slots; FP32 2.2 instructions per cycle and SM;
+// FP64 1.6, the FP64 pipe at 46%).  A step of two partners (k and k ^ 4) is 39
+// packed FP32 instructions, two reciprocals, four shuffles and two 16-byte shared
+// loads; the (j, k) records and sums stay in registers.  One partner at a time and
+// plain FP32 instructions (62 per step) took 67.8 instead of 54.8 ms on eight
+// frames and, in FP64, 16.7 instead of 15.3 ms on the cluster.  Whole evaluations
+// with the neighbour-list and block-per-molecule kernels that this one replaced
+// (185 instructions per slot, exp, log and divisions per triple in FP64) against
+// now: cluster of 5000 atoms (FP64) 54.0 -> 15.3 ms, 512 molecules (FP64) 21.4 ->
+// 2.1 ms, 4096 molecules (mixed) 13.9 -> 7.6 ms, eight periodic frames (mixed) 149
+// -> 54.8 ms, one molecule of 100 atoms 216 -> 85 us, slab energy 2.6 -> 0.63 ms.
 // GEN: work partition and term counting (the owner test of every triple).
 template <class R, bool GRAD, bool PER, bool GEN>
-__global__ void __launch_bounds__(32 * kAtmWarps, sizeof(R) == 4 ? (GRAD ? 4 : 6) : (GRAD ? 2 : 4))
+__global__ void __launch_bounds__(32 * kAtmWarps, kTripleBlocks<R, GRAD>)
 k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int split, int grab,
               unsigned long long* queue, unsigned long long* fxf, unsigned long long* fxe, int counting,
               const int* guard)
@@ -481,6 +542,7 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
     extern __shared__ __align__(16) unsigned char smem_raw[];
     using Rec = typename RecT<R>::rec;
     using Aux = typename RecT<R>::aux;
+    using Pair = typename PairT<R>::type;
     constexpr unsigned kAll = 0xffffffffu;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     AtmShared<R>& sh = reinterpret_cast<AtmShared<R>*>(smem_raw)[wid];
@@ -488,7 +550,7 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
     const Rec* rec = static_cast<const Rec*>(v.rec);
     const Aux* aux = static_cast<const Aux*>(v.aux);
     const int q = lane >> 3, j = lane & 7, qbase = lane & 24;
-    const R ahalf = R(0.5 * alp3d);
+    const Pair ahalf = pk(R(0.5 * alp3d), R(0.5 * alp3d));
     const bool smooth_on = c.width3 > 0.0 && c.width3 < c.cut3;
     const R cutoff = R(c.cut3), width = R(c.width3);
     const unsigned long long nunits = (unsigned long long)v.ncand * split;
@@ -524,22 +586,28 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
                      kz = PER ? img[3 * id.t + 2] : 0.0;
         const long long bjk = v.map ? v.map[cand] : cand;
         const int aj = v.sub[kT8 * (id.t8 + J) + j], ak = v.sub[kT8 * (id.t8 + K) + j];
-        double xj = 0, yj = 0, zj = 0, xk = 0, yk = 0, zk = 0;
-        if (GRAD) {
-            if (aj >= 0) { xj = b.x[aj]; yj = b.y[aj]; zj = b.z[aj]; }
-            if (ak >= 0) { xk = b.x[ak] + kx; yk = b.y[ak] + ky; zk = b.z[ak] + kz; }
+        if (GRAD && q < 2) {
+            double4 o = v.pos[kT8 * (id.t8 + (q ? K : J)) + j];
+            if (q) { o.x += kx; o.y += ky; o.z += kz; }
+            (q ? sh.pk : sh.pj)[j] = o;
         }
+        __syncwarp();
         int oj = 0, ok = 0;
         if (GEN) {
             oj = aj >= 0 ? b.local[aj] : 0;
             ok = ak >= 0 ? b.local[ak] : 0;
         }
-        // the (j, k) records of this lane, step t: k = (j + t) mod 8
-        Rec rjk[kT8];
+        // the (j, k) records of this lane; pair p: k = (j + p) mod 8 and k ^ 4.
+        // Half of the walk (diag): steps 1..3, and 4 in the lower lanes.
+        Pair zx[4], zu[4], zm[4], zp[4];
 #pragma unroll
-        for (int t = 0; t < kT8; t++) {
-            rjk[t] = rec[bjk * kRecs + kT8 * j + ((j + t) & 7)];
-            if (diag && t == 4 && j >= 4) { rjk[t].z = R(0); if (GEN) rjk[t].y = R(0); }
+        for (int p = 0; p < 4; p++) {
+            Rec r0 = rec[bjk * kRecs + kT8 * j + ((j + p) & 7)], r1 = rec[bjk * kRecs + kT8 * j + ((j + p + 4) & 7)];
+            if (diag) {
+                if (p == 0) { r0.z = R(0); if (GEN) r0.y = R(0); }
+                if (p > 0 || j >= 4) { r1.z = R(0); if (GEN) r1.y = R(0); }
+            }
+            zx[p] = pk(r0.x, r1.x); zu[p] = pk(r0.y, r1.y); zm[p] = pk(r0.z, r1.z); zp[p] = pk(r0.w, r1.w);
         }
         const int2 range = v.range[id.t8 + J];
         const int4* list = v.list + v.list_off[id.sys] + (long long)J * nt8 * nT;
@@ -591,11 +659,13 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
                     total = __shfl_sync(kAll, total, 31);
                 }
                 if (m) {
+                    const unsigned rij0 = (unsigned)bij * kRecs, rik0 = (unsigned)bik * kRecs;
                     int p = head + cnt + at;
                     while (m) {
                         const int i = __ffs(m) - 1;
                         m &= m - 1;
-                        sh.ring[p & (kRing - 1)] = make_int4(bij, bik, kT8 * (id.t8 + I) + i, fl);
+                        const unsigned first = (fl & 1) ? i : kT8 * i;
+                        sh.ring[p & (kRing - 1)] = make_int4((int)(rij0 + first), (int)(rik0 + first), kT8 * (id.t8 + I) + i, fl);
                         p++;
                     }
                 }
@@ -604,24 +674,23 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
             __syncwarp();
             if (cnt == 0) break;
             const int nroot = min(cnt, kRootChunk);
-            R Djk[kT8], Wjk[kT8];
-            R fj[4] = {R(0), R(0), R(0), R(0)}, fk[4] = {R(0), R(0), R(0), R(0)};   // force and dE/dCN of j, k
+            Pair Djk[4], Wjk[4];
+            Pair fjk[4];                       // force and dE/dCN of j and of k
             double vr[3] = {0, 0, 0};          // component (lane >> 1) & 3 of sum F_i (x) T_I
             R esum = R(0);
             int ntrip = 0;
             if (GRAD)
 #pragma unroll
-                for (int t = 0; t < kT8; t++) { Djk[t] = R(0); Wjk[t] = R(0); }
+                for (int p = 0; p < 4; p++) { Djk[p] = pk(R(0), R(0)); Wjk[p] = pk(R(0), R(0)); fjk[p] = pk(R(0), R(0)); }
             auto fetch = [&](int r0) {
                 const int4 e = sh.ring[(head + min(r0 + q, nroot - 1)) & (kRing - 1)];
                 AtmStage<R>& s = sh.st[(r0 >> 2) & 1];
-                const int i8 = e.z & 7;
-                const int off = (e.w & 1) ? kT8 * j + i8 : kT8 * i8 + j;
-                async_copy_value(&s.ij[lane], rec + (long long)e.x * kRecs + off);
-                async_copy_value(&s.ik[lane], rec + (long long)e.y * kRecs + off);
+                const unsigned step = (e.w & 1) ? kT8 * j : j;
+                async_copy_value(&s.ij[lane], rec + ((unsigned)e.x + step));
+                async_copy_value(&s.ik[lane], rec + ((unsigned)e.y + step));
                 if (GRAD) {
-                    async_copy_value(&s.qij[lane], aux + (long long)e.x * kRecs + off);
-                    async_copy_value(&s.qik[lane], aux + (long long)e.y * kRecs + off);
+                    async_copy_value(&s.qij[lane], aux + ((unsigned)e.x + step));
+                    async_copy_value(&s.qik[lane], aux + ((unsigned)e.y + step));
                     if (j < 2) async_copy<16>(reinterpret_cast<char*>(&s.pos[q]) + 16 * j,
                                               reinterpret_cast<const char*>(v.pos + e.z) + 16 * j);
                     else if (PER && j < 5) async_copy<8>(&s.T[q][j - 2], img + 3 * (e.w >> 2) + j - 2);
@@ -641,73 +710,94 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
                 if (GEN) ai = v.sub[e.z];
                 if (!rin) { rij.z = R(0); if (GEN) rij.y = R(0); }
                 if (same && (e.w & 2)) rij.z *= R(1.0 / 3.0);
-                const R P6 = R(6) * rij.w, u38 = R(0.375) * rij.y;
-                R rK = R(0), rV = R(0), rE = R(0), kS = R(0), kE = R(0);
+                if constexpr (sizeof(R) == 4) {
+                    const float4 own = st.ik[lane];
+                    sh.xu[lane] = make_float4(own.x, __shfl_xor_sync(kAll, own.x, 4), own.y, __shfl_xor_sync(kAll, own.y, 4));
+                    sh.mp[lane] = make_float4(own.z, __shfl_xor_sync(kAll, own.z, 4), own.w, __shfl_xor_sync(kAll, own.w, 4));
+                    __syncwarp();
+                }
+                const Pair x = pk(rij.x, rij.x), xm = pk(rij.z, rij.z), one = pk(R(1), R(1));
+                const Pair xu = pk(R(0.375) * rij.y, R(0.375) * rij.y), xp = pk(R(6) * rij.w, R(6) * rij.w);
+                Pair rK = pk(R(0), R(0)), rV = rK, rE = rK, kS = rK, kE = rK;
 #pragma unroll
-                for (int t = 0; t < kT8; t++) {
-                    if (diag && (t == 0 || t > 4)) continue;
-                    const Rec B = st.ik[qbase | ((j + t) & 7)];
-                    R M = rij.z * B.z * rjk[t].z;
-                    if (GEN) {
-                        const int okt = __shfl_sync(kAll, ok, qbase | ((j + t) & 7));
-                        const int akt = __shfl_sync(kAll, ak, qbase | ((j + t) & 7));
-                        bool valid = rij.y * B.y * rjk[t].y != R(0);
-                        if (part.nparts > 1) {
-                            // owner of the triple: the pair of its two largest input indices
-                            int o1 = b.local[ai], o2 = oj, o3 = okt, w_;
-                            if (o2 > o1) { w_ = o1; o1 = o2; o2 = w_; }
-                            if (o3 > o2) { w_ = o2; o2 = o3; o3 = w_; }
-                            if (o2 > o1) { w_ = o1; o1 = o2; o2 = w_; }
-                            valid = valid && owns_pair_atm(part, o1, o2);
-                        }
-                        if (!valid) M = R(0);
-                        // visits of the reference's loop (atm.f90:705-733), times three
-                        const int eq = (ai == aj) + (ai == akt) + (aj == akt);
-                        const int mult = eq == 3 ? 6 : eq ? 2 : 1;
-                        if (valid) ntrip += (e.w & 2) ? mult : 3 * mult;
+                for (int p = 0; p < 4; p++) {
+                    const int kl = qbase | ((j + p) & 7);
+                    Pair y, yu, ym, yp;
+                    if constexpr (sizeof(R) == 4) {
+                        const float4 b0 = sh.xu[kl], b1 = sh.mp[kl];
+                        y = pk(b0.x, b0.y); yu = pk(b0.z, b0.w); ym = pk(b1.x, b1.y); yp = pk(b1.z, b1.w);
+                    } else {
+                        const Rec b0 = st.ik[kl], b1 = st.ik[kl ^ 4];
+                        y = pk(b0.x, b1.x); yu = pk(b0.y, b1.y); ym = pk(b0.z, b1.z); yp = pk(b0.w, b1.w);
                     }
-                    const R x = rij.x, y = B.x, z = rjk[t].x;
-                    const R U = u38 * B.y * rjk[t].y;
-                    const R p6 = P6 * B.w * rjk[t].w;
-                    const R s = x + y, d = x - y;
-                    const R a1 = z + d, a2 = s - z, a3 = z - d;
-                    const R q1 = a1 * a2;
-                    const R A = q1 * a3 * U;
-                    const R f = rcp_fast(p6 + R(1));
-                    const R B1 = A + R(1);
-                    const R Mf = M * f;
+                    Pair M = xm * ym * zm[p];
+                    if (GEN) {
+                        R mh[2] = {lo(M), hi(M)};
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            const int okt = __shfl_sync(kAll, ok, kl ^ (4 * h)), akt = __shfl_sync(kAll, ak, kl ^ (4 * h));
+                            bool valid = rij.y * (h ? hi(yu) * hi(zu[p]) : lo(yu) * lo(zu[p])) != R(0);
+                            if (part.nparts > 1) {
+                                // owner of the triple: the pair of its two largest input indices
+                                int o1 = b.local[ai], o2 = oj, o3 = okt, w_;
+                                if (o2 > o1) { w_ = o1; o1 = o2; o2 = w_; }
+                                if (o3 > o2) { w_ = o2; o2 = o3; o3 = w_; }
+                                if (o2 > o1) { w_ = o1; o1 = o2; o2 = w_; }
+                                valid = valid && owns_pair_atm(part, o1, o2);
+                            }
+                            if (!valid) mh[h] = R(0);
+                            // visits of the reference's loop (atm.f90:705-733), times three
+                            const int eq = (ai == aj) + (ai == akt) + (aj == akt);
+                            const int mult = eq == 3 ? 6 : eq ? 2 : 1;
+                            if (valid) ntrip += (e.w & 2) ? mult : 3 * mult;
+                        }
+                        M = pk(mh[0], mh[1]);
+                    }
+                    const Pair z = zx[p];
+                    const Pair U = xu * yu * zu[p];
+                    const Pair p6 = xp * yp * zp[p];
+                    const Pair s = x + y, d = x - y;
+                    const Pair a1 = z + d, a2 = s - z, a3 = z - d;
+                    const Pair q1 = a1 * a2;
+                    const Pair A = q1 * a3 * U;
+                    const Pair t = p6 + one;
+                    const Pair f = pk(rcp_fast(lo(t)), rcp_fast(hi(t)));
+                    const Pair B1 = A + one;
+                    const Pair Mf = M * f;
                     if constexpr (!GRAD) {
                         rE = fma(Mf, B1, rE);
                     } else {
-                        const R E = Mf * B1;
-                        const R q2 = a2 * a3, q3 = a1 * a3;
-                        const R KM = fma(B1, fma(p6 * f, ahalf, R(-1.5)), -A) * Mf;
-                        const R V = U * Mf;
-                        const R dq = q2 - q1, sq = q2 + q1;
-                        rK += KM;
+                        const Pair E = Mf * B1;
+                        const Pair q2 = a2 * a3, q3 = a1 * a3;
+                        // K = (1 + A) w - A with w = alp/2 6Pf - 3/2: (1 + A)(w - 1) + 1
+                        const Pair KM = fma(B1, fma(p6 * f, ahalf, pk(R(-2.5), R(-2.5))), one) * Mf;
+                        const Pair V = U * Mf;
+                        const Pair dq = q2 - q1, sq = q2 + q1;
+                        rK = rK + KM;
                         rV = fma(V, q3 + dq, rV);
-                        kS = fma(B.y, KM, kS);
+                        kS = fma(yu, KM, kS);
                         kS = fma(V, q3 - dq, kS);
-                        Djk[t] = fma(rjk[t].y, KM, Djk[t]);
-                        Djk[t] = fma(V, sq - q3, Djk[t]);
-                        rE += E;
-                        kE += E;
-                        Wjk[t] += E;
+                        Djk[p] = fma(zu[p], KM, Djk[p]);
+                        Djk[p] = fma(V, sq - q3, Djk[p]);
+                        rE = rE + E;
+                        kE = kE + E;
+                        Wjk[p] = Wjk[p] + E;
                         // the sums of (i, k) move one lane down, with k
-                        kS = __shfl_sync(kAll, kS, qbase | ((j + 1) & 7));
-                        kE = __shfl_sync(kAll, kE, qbase | ((j + 1) & 7));
+                        const int from = qbase | ((j + 1) & 7);
+                        kS = pk(__shfl_sync(kAll, lo(kS), from), __shfl_sync(kAll, hi(kS), from));
+                        kE = pk(__shfl_sync(kAll, lo(kE), from), __shfl_sync(kAll, hi(kE), from));
                     }
                 }
-                esum += rE;
+                const R sumE = lo(rE) + hi(rE);
+                esum += sumE;
                 if constexpr (GRAD) {
-                    if (diag) {     // steps 1..4: column k ended in lane k - 5
-                        kS = __shfl_sync(kAll, kS, qbase | ((j + 3) & 7));
-                        kE = __shfl_sync(kAll, kE, qbase | ((j + 3) & 7));
-                    }
-                    R Dij = fma(rij.y, rK, rV), Dik = kS;
+                    // after four moves the lane holds column j (upper value) and column j ^ 4 (lower)
+                    const R Wik = hi(kE) + __shfl_xor_sync(kAll, lo(kE), 4);
+                    R Dik = hi(kS) + __shfl_xor_sync(kAll, lo(kS), 4);
+                    R Dij = ::fma(rij.y, lo(rK) + hi(rK), lo(rV) + hi(rV));
                     if (smooth_on) {
-                        if (rE != R(0)) Dij += rE * dln_switch<R>(rij.x, cutoff, width);
-                        if (kE != R(0)) Dik += kE * dln_switch<R>(st.ik[lane].x, cutoff, width);
+                        if (sumE != R(0)) Dij += sumE * dln_switch<R>(rij.x, cutoff, width);
+                        if (Wik != R(0)) Dik += Wik * dln_switch<R>(st.ik[lane].x, cutoff, width);
                     }
                     const double4 pi = st.pos[q];
                     double tix = 0, tiy = 0, tiz = 0;
@@ -717,14 +807,14 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
                     const bool tr = e.w & 1;
                     R g0, g1, g2, g3;
                     {
-                        const R gx = Dij * R(xj - xi), gy = Dij * R(yj - yi), gz = Dij * R(zj - zi);
-                        fj[0] += gx; fj[1] += gy; fj[2] += gz;
-                        fj[3] = fma(rE, tr ? qij.x : qij.y, fj[3]);
-                        const R hx = Dik * R(xk - xi), hy = Dik * R(yk - yi), hz = Dik * R(zk - zi);
-                        fk[0] += hx; fk[1] += hy; fk[2] += hz;
-                        fk[3] = fma(kE, tr ? qik.x : qik.y, fk[3]);
-                        g0 = -(gx + hx); g1 = -(gy + hy); g2 = -(gz + hz);
-                        g3 = fma(rE, tr ? qij.y : qij.x, kE * (tr ? qik.y : qik.x));
+                        const double4 pj = sh.pj[j], pk_ = sh.pk[j];
+                        const Pair D = pk(Dij, Dik);
+                        const Pair gx = D * pk(R(pj.x - xi), R(pk_.x - xi)), gy = D * pk(R(pj.y - yi), R(pk_.y - yi)),
+                                   gz = D * pk(R(pj.z - zi), R(pk_.z - zi));
+                        fjk[0] = fjk[0] + gx; fjk[1] = fjk[1] + gy; fjk[2] = fjk[2] + gz;
+                        fjk[3] = fma(pk(sumE, Wik), tr ? pk(qij.x, qik.x) : pk(qij.y, qik.y), fjk[3]);
+                        g0 = -(lo(gx) + hi(gx)); g1 = -(lo(gy) + hi(gy)); g2 = -(lo(gz) + hi(gz));
+                        g3 = ::fma(sumE, tr ? qij.y : qij.x, Wik * (tr ? qik.y : qik.x));
                     }
                     // force (and dE/dCN) of the root: component (lane >> 1) & 3 summed over the quarter
                     {
@@ -735,7 +825,7 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
                         kk += __shfl_xor_sync(kAll, kk, 1);
                         const int comp = (lane >> 1) & 3;
                         const double g = double(kk);
-                        if (PER) { vr[0] = fma(g, tix, vr[0]); vr[1] = fma(g, tiy, vr[1]); vr[2] = fma(g, tiz, vr[2]); }
+                        if (PER) { vr[0] = ::fma(g, tix, vr[0]); vr[1] = ::fma(g, tiy, vr[1]); vr[2] = ::fma(g, tiz, vr[2]); }
                         if (rin) {
                             long long hi, lo;
                             fixed_split(g, hi, lo);
@@ -760,26 +850,26 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
                 }
             }
             if constexpr (GRAD) {
+                R fj[4], fk[4];
+#pragma unroll
+                for (int d = 0; d < 4; d++) { fj[d] = lo(fjk[d]); fk[d] = hi(fjk[d]); }
                 // quarter q keeps the steps t = q and q + 4, summed over the quarters
                 R Dt[2], Wt[2];
                 {
+                    // pair p holds the steps p and p + 4: halving over the quarters leaves pair q
                     const bool h16 = lane & 16, h8 = lane & 8;
-                    R D4[4], W4[4];     // steps (q & 2) + {0, 1, 4, 5}
+                    auto halve = [&](const Pair* X, R& first, R& second) {
+                        R a0[2], a1[2];
 #pragma unroll
-                    for (int p = 0; p < 4; p++) {
-                        const int lo_t = (p & 1) + 4 * (p >> 1), hi_t = lo_t + 2;
-                        D4[p] = sel(h16, Djk[hi_t], Djk[lo_t]) +
-                                __shfl_xor_sync(kAll, sel(h16, Djk[lo_t], Djk[hi_t]), 16);
-                        W4[p] = sel(h16, Wjk[hi_t], Wjk[lo_t]) +
-                                __shfl_xor_sync(kAll, sel(h16, Wjk[lo_t], Wjk[hi_t]), 16);
-                    }
-#pragma unroll
-                    for (int p = 0; p < 2; p++) {
-                        Dt[p] = sel(h8, D4[2 * p + 1], D4[2 * p]) +
-                                __shfl_xor_sync(kAll, sel(h8, D4[2 * p], D4[2 * p + 1]), 8);
-                        Wt[p] = sel(h8, W4[2 * p + 1], W4[2 * p]) +
-                                __shfl_xor_sync(kAll, sel(h8, W4[2 * p], W4[2 * p + 1]), 8);
-                    }
+                        for (int p = 0; p < 2; p++) {
+                            a0[p] = sel(h16, lo(X[p + 2]), lo(X[p])) + __shfl_xor_sync(kAll, sel(h16, lo(X[p]), lo(X[p + 2])), 16);
+                            a1[p] = sel(h16, hi(X[p + 2]), hi(X[p])) + __shfl_xor_sync(kAll, sel(h16, hi(X[p]), hi(X[p + 2])), 16);
+                        }
+                        first = sel(h8, a0[1], a0[0]) + __shfl_xor_sync(kAll, sel(h8, a0[0], a0[1]), 8);
+                        second = sel(h8, a1[1], a1[0]) + __shfl_xor_sync(kAll, sel(h8, a1[0], a1[1]), 8);
+                    };
+                    halve(Djk, Dt[0], Dt[1]);
+                    halve(Wjk, Wt[0], Wt[1]);
                 }
 #pragma unroll
                 for (int p = 0; p < 2; p++) {
@@ -787,11 +877,11 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
                     const int kl = qbase | ((j + t) & 7), back = qbase | ((j - t) & 7);
                     if (smooth_on && Wt[p] != R(0))
                         Dt[p] += Wt[p] * dln_switch<R>(rec[bjk * kRecs + kT8 * j + ((j + t) & 7)].x, cutoff, width);
-                    const R gx = Dt[p] * R(__shfl_sync(kAll, xk, kl) - xj), gy = Dt[p] * R(__shfl_sync(kAll, yk, kl) - yj),
-                            gz = Dt[p] * R(__shfl_sync(kAll, zk, kl) - zj);
+                    const double4 pj = sh.pj[j], pk_ = sh.pk[kl & 7];
+                    const R gx = Dt[p] * R(pk_.x - pj.x), gy = Dt[p] * R(pk_.y - pj.y), gz = Dt[p] * R(pk_.z - pj.z);
                     const Aux qa = aux[bjk * kRecs + kT8 * j + ((j + t) & 7)];
                     fj[0] -= gx; fj[1] -= gy; fj[2] -= gz;
-                    fj[3] = fma(Wt[p], qa.x, fj[3]);
+                    fj[3] = ::fma(Wt[p], qa.x, fj[3]);
                     fk[0] += __shfl_sync(kAll, gx, back);
                     fk[1] += __shfl_sync(kAll, gy, back);
                     fk[2] += __shfl_sync(kAll, gz, back);
@@ -820,9 +910,9 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
                     const int comp = lane >> 1;
                     const double kcc = __shfl_sync(kAll, kc, (8 * comp) & 31);
                     if (lane < 6 && !(lane & 1)) {
-                        fixed_add(fe + 2 * (1 + 3 * comp), fma(kcc, kx, vr[0]));
-                        fixed_add(fe + 2 * (2 + 3 * comp), fma(kcc, ky, vr[1]));
-                        fixed_add(fe + 2 * (3 + 3 * comp), fma(kcc, kz, vr[2]));
+                        fixed_add(fe + 2 * (1 + 3 * comp), ::fma(kcc, kx, vr[0]));
+                        fixed_add(fe + 2 * (2 + 3 * comp), ::fma(kcc, ky, vr[1]));
+                        fixed_add(fe + 2 * (3 + 3 * comp), ::fma(kcc, kz, vr[2]));
                     }
                 }
             }

@@ -1020,6 +1020,8 @@ void Engine::run_three_body(const Batch& b, const Species& s, const Damp& d, con
         }
     }
     if (!capturing_) {
+        // the triple kernel numbers the records with 32 bits
+        if (blocks > (0xffffffffLL >> 6)) throw Error("The system is too large for the three-body term");
         auto reserve = [&](void*& p, size_t& cap, size_t need) {
             if (need <= cap) return;
             free_block(p);
