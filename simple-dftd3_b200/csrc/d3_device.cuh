@@ -181,10 +181,11 @@ struct Tuning {
 
 // Pairwise decomposition (d3_pairwise.cu), FP64: energy2 and energy3 of every
 // system as [n_s][n_s] blocks at off[sys] (input atom order); c6 is scratch of
-// the same size.  Needs the sorted atoms and the reference weights.
+// the same size, factors of twice that (16-byte aligned; used for molecules: every
+// system has one lattice point).  Needs the sorted atoms and the reference weights.
 void launch_pairwise(const Batch& b, const Species& s, const Damp& d, const Config& c, const Work& w,
-                     const long long* off, long long total, double* c6, double* e2, double* e3,
-                     cudaStream_t stream);
+                     const long long* off, long long total, bool molecules, double* c6, double* factors, double* e2,
+                     double* e3, cudaStream_t stream);
 
 // Analytic Hessian of one structure (d3_hessian.cu), FP64, input atom order:
 // pos [n][3], sp, zid, ghost per atom; img_range = the [first, last) image

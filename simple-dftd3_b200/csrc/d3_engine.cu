@@ -635,7 +635,7 @@ void Engine::pairwise_host(const Damp& d, const double* positions, double* energ
     upload_pair_table(d, stream);
     const long long total = std::max<long long>(c6mat_total_, 1);
     if (!d_pw_) {
-        d_pw_ = dev_alloc<double>(3 * (size_t)total);
+        d_pw_ = dev_alloc<double>(5 * (size_t)total);
         d_pw_off_ = dev_alloc<long long>(nsys_);
         check(cudaMemcpy(d_pw_off_, c6mat_off_.data(), sizeof(long long) * nsys_, cudaMemcpyHostToDevice),
               "pairwise offsets");
@@ -651,17 +651,30 @@ void Engine::pairwise_host(const Damp& d, const double* positions, double* energ
     c.grad = false; c.mixed = false; c.param_grad = false; c.cn_partitioned = false;
     Work w = work_;
     w.counts = nullptr; w.e3_atom = nullptr; w.sig3_atom = nullptr; w.pg_atom = nullptr;
-    pu_.split = cn_split();
-    pu_.cn_store = nullptr;
-    pu_.cn_store_ok = nullptr;
-    order_atoms(d, d_pos_in_, b, false, stream);
-    launch_cn_units(b, s, c, Partition{}, w, pu_, false, stream);
-    launch_weights(b, s, c, w, stream);
-    launch_pairwise(b, s, d, c, w, d_pw_off_, c6mat_total_, d_pw_, d_pw_ + total, d_pw_ + 2 * total, stream);
+    if (small_systems()) {
+        // atoms in input order: one kernel for CN and weights in place of eight
+        b.sp = d_sp_;
+        b.ghost = d_ghost_;
+        b.local = d_local_;
+        b.zid = d_zid_;
+        b.perm = d_identity_;
+        b.tiles = nullptr;
+        const InputPositions in{d_pos_in_, d_x_, d_y_, d_z_, d_xhi_, d_xlo_};
+        launch_coordination_number(b, s, c, Partition{}, w, stream, &in, nullptr);
+    } else {
+        pu_.split = cn_split();
+        pu_.cn_store = nullptr;
+        pu_.cn_store_ok = nullptr;
+        order_atoms(d, d_pos_in_, b, false, stream);
+        launch_cn_units(b, s, c, Partition{}, w, pu_, false, stream);
+        launch_weights(b, s, c, w, stream);
+    }
+    launch_pairwise(b, s, d, c, w, d_pw_off_, c6mat_total_, !any_periodic_, d_pw_ + 2 * total, d_pw_, d_pw_ + 3 * total,
+                    d_pw_ + 4 * total, stream);
     check(cudaGetLastError(), "pairwise kernels");
-    check(cudaMemcpyAsync(energy2, d_pw_ + total, sizeof(double) * c6mat_total_, cudaMemcpyDeviceToHost, stream),
+    check(cudaMemcpyAsync(energy2, d_pw_ + 3 * total, sizeof(double) * c6mat_total_, cudaMemcpyDeviceToHost, stream),
           "pairwise energy2");
-    check(cudaMemcpyAsync(energy3, d_pw_ + 2 * total, sizeof(double) * c6mat_total_, cudaMemcpyDeviceToHost, stream),
+    check(cudaMemcpyAsync(energy3, d_pw_ + 4 * total, sizeof(double) * c6mat_total_, cudaMemcpyDeviceToHost, stream),
           "pairwise energy3");
     check(cudaStreamSynchronize(stream), "pairwise");
 }
@@ -725,6 +738,11 @@ bool Engine::direct_pairs(const Damp& d, bool pg) const
 {
     if (reducer_ || counting_ || pg || part_.nparts > 1) return false;
     if (d.kind != kRational && d.kind != kZero) return false;
+    return small_systems();
+}
+
+bool Engine::small_systems() const
+{
     return max_sys_atoms_ <= kDirectMaxAtoms && natoms_ <= kDirectMaxTotal;
 }
 

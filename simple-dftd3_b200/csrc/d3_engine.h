@@ -160,7 +160,7 @@ private:
     double* d_hs_ = nullptr;             // Hessian scratch and result
     double* d_rvdw_ = nullptr;           // [nid][nid] van der Waals radii (Hessian damping kernels)
     std::vector<int> img_off_host_;      // host copy of the image offsets
-    double* d_pw_ = nullptr;             // pairwise decomposition: C6, energy2, energy3 (3 x sum n_s^2)
+    double* d_pw_ = nullptr;             // pairwise decomposition: pair factors, C6, energy2, energy3 (5 x sum n_s^2)
     long long* d_pw_off_ = nullptr;
     void run(const Damp& d, const double* d_positions, double* d_energies, double* d_gradient,
              double* d_sigma9, double* d_param_grad, bool grad, cudaStream_t stream);
@@ -195,6 +195,7 @@ private:
     // systems small enough for the direct pair kernels (see direct_pairs)
     static constexpr int kDirectMaxAtoms = DIRECT_MAX_ATOMS;
     static constexpr int kDirectMaxTotal = DIRECT_MAX_TOTAL;
+    bool small_systems() const;
     bool direct_pairs(const Damp& d, bool pg) const;
     bool graph_on_ = false, capturing_ = false, graph_valid_ = false;
     cudaGraphExec_t graph_exec_ = nullptr;

@@ -4,14 +4,15 @@
 // triple, as the matrices energy2[i][j] and energy3[i][j] of every system
 // (input atom order, systems one after the other).
 //
-//   k_pw_c6        C6 of every ordered atom pair of each system (sorted order)
+//   k_pw_c6        C6 of every ordered atom pair of each system (sorted order), and for
+//                  systems of one lattice point the pair's factors of a triple
 //   k_pairwise2    one block per atom i: the lanes take the partners j and sum
 //                  the pair over all lattice translations; every (i, j) entry
 //                  is written once by its row, no atomics
-//   k_pairwise3    one thread per pair (i, j <= i) in the triple loop order of
-//                  atm.f90:829-950 (i >= j >= k, translations of j and k); a
-//                  sixth of each triple energy goes to each ordered pair of
-//                  the triple, summed per thread and added with FP64 atomics
+//   k_pairwise3    one warp per atom pair (i, j <= i): the energies of all triples
+//                  (atm.f90:829-950) that hold the pair, the lanes taking the third
+//                  atoms and images; a sixth of each triple energy belongs to each
+//                  ordered pair of the triple, so the entry is a sixth of that sum
 #include <cfloat>
 #include <cstdint>
 
@@ -34,9 +35,26 @@ __device__ __forceinline__ int system_of_offset(const long long* off, int nsys, 
     return lo;
 }
 
+// Factors of one pair of a triple (d3_atm.cu): m = sqrt(C6) r^-3 times the smooth
+// switch, and the pair's share P of (r0/r)^alp3, bounded so that the product of three
+// stays finite.  Zero outside the cutoff.
+__device__ __forceinline__ double2 pw_factor(double x, double c6, double r0, double alp3, const Config& c)
+{
+    if (x > c.cut3 * c.cut3 || x < DBL_EPSILON || c6 == 0.0) return make_double2(0.0, 0.0);
+    const double u = 1.0 / x;
+    double m = sqrt(fabs(c6)) * u * sqrt(u);
+    if (c.width3 > 0.0) {
+        double sw, dsw;
+        smooth<double>(sqrt(x), c.cut3, c.width3, sw, dsw);
+        m *= sw;
+    }
+    return make_double2(m, fmin(exp(0.5 * alp3 * log(r0 * r0 * u)), 1e100));
+}
+
 // C6 of the ordered pair (r, c) of each system (get_atomic_c6,
 // model.f90:340-431); ghost atoms give 0.
-__global__ void k_pw_c6(Batch b, Species s, Work w, const long long* off, long long total, double* c6)
+__global__ void k_pw_c6(Batch b, Species s, Config cf, Work w, const long long* off, long long total, double alp3,
+                        double* c6, double2* mp)
 {
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (t >= total) return;
@@ -45,8 +63,8 @@ __global__ void k_pw_c6(Batch b, Species s, Work w, const long long* off, long l
     const long long e = t - off[sys];
     const int r = a0 + (int)(e / n), c = a0 + (int)(e % n);
     double v = 0.0;
+    const int sr = b.sp[r], sc = b.sp[c];
     if (!(b.ghost && (b.ghost[r] || b.ghost[c]))) {
-        const int sr = b.sp[r], sc = b.sp[c];
         const double* ref = s.c6ref + (size_t)(sr * b.nid + sc) * kMaxRef * kMaxRef;
         for (int ir = 0; ir < s.nref[sr]; ir++) {
             double a = 0.0;
@@ -55,6 +73,9 @@ __global__ void k_pw_c6(Batch b, Species s, Work w, const long long* off, long l
         }
     }
     c6[t] = v;
+    if (!mp) return;
+    const double dx = b.x[r] - b.x[c], dy = b.y[r] - b.y[c], dz = b.z[r] - b.z[c];
+    mp[t] = pw_factor(dx * dx + dy * dy + dz * dz, v, s.atm_r0[sr * b.nid + sc], alp3, cf);
 }
 
 // edisp of one (i, j, T) term without the smooth cutoff: the energy
@@ -123,17 +144,23 @@ __global__ void __launch_bounds__(kPwThreads) k_pairwise2(Batch b, Species s, Da
     }
 }
 
-__device__ __forceinline__ double pw_triple_scale(int i, int j, int k)
+// Energy of a triple from its squared distances and the products of the pair factors.
+__device__ __forceinline__ double pw_triple(double x, double y, double z, double m, double P)
 {
-    // atm.f90:954-980
-    if (i == j) return i == k ? 1.0 / 6.0 : 0.5;
-    return (i != k && j != k) ? 1.0 : 0.5;
+    const double w = x * y * z;
+    const double A = 0.375 * (x + y - z) * (x - y + z) * (y + z - x) / w;
+    return m * (1.0 + A) / (1.0 + 6.0 * P);
 }
 
+// A site pair (i at 0, j at T_j) occurs once with every third site, also where sites
+// are images of one atom (atm.f90:954-980 then weights the repeated visits of the
+// reference's loop), so no weights are needed.  mp: pair factors (molecules), or null.
 __global__ void __launch_bounds__(kPwThreads) k_pairwise3(Batch b, Species s, Damp d, Config c, const long long* off,
-                                                           long long total, const double* c6, double* e3)
+                                                          long long total, const double* c6, const double2* mp,
+                                                          double* e3)
 {
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    const long long t = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     if (t >= total) return;
     const int sys = system_of_offset(off, b.nsys, t);
     const int a0 = b.atom_off[sys], n = b.atom_off[sys + 1] - a0;
@@ -143,86 +170,69 @@ __global__ void __launch_bounds__(kPwThreads) k_pairwise3(Batch b, Species s, Da
     const int p = a0 + pl, q = a0 + ql;
     const double* cm = c6 + off[sys];
     const double c6pq = cm[(long long)pl * n + ql];
-    if (c6pq == 0.0) return;
-    const int t0 = b.img_off[kImgDisp3 * (b.nsys + 1) + sys], t1 = b.img_off[kImgDisp3 * (b.nsys + 1) + sys + 1];
-    const double cut2 = c.cut3 * c.cut3;
-    const bool smooth_on = c.width3 > 0.0;
-    const double alp3 = (d.alp + 2.0) / 3.0;
-    const int sp = b.sp[p], sq = b.sp[q];
-    const double r0pq = s.atm_r0[sp * b.nid + sq];     // rs9 R0 (rs9 = 4/3)
-    const double xp = b.x[p], yp = b.y[p], zp = b.z[p];
-    double* eg = e3 + off[sys];
-    const long long lp = b.local[p], lq = b.local[q];
-    double epq = 0.0;
-    for (int tj = t0; tj < t1; tj++) {
-        const double ijx = b.x[q] + b.img[3 * tj] - xp, ijy = b.y[q] + b.img[3 * tj + 1] - yp,
-                     ijz = b.z[q] + b.img[3 * tj + 2] - zp;
-        const double r2ij = ijx * ijx + ijy * ijy + ijz * ijz;
-        if (r2ij > cut2 || r2ij < DBL_EPSILON) continue;
-        double swij = 1.0, dsw = 0.0;
-        if (smooth_on) smooth<double>(sqrt(r2ij), c.cut3, c.width3, swij, dsw);
-        for (int rl = 0; rl <= ql; rl++) {
-            const int r = a0 + rl;
-            const double c6pr = cm[(long long)pl * n + rl], c6qr = cm[(long long)ql * n + rl];
-            const double c9 = -d.s9 * sqrt(fabs(c6pq * c6pr * c6qr));
-            if (c9 == 0.0) continue;
-            const int sr = b.sp[r];
-            const double r0 = r0pq * s.atm_r0[sp * b.nid + sr] * s.atm_r0[sq * b.nid + sr];
-            const double triple = pw_triple_scale(pl, ql, rl);
-            double epr = 0.0, eqr = 0.0;
-            for (int tk = t0; tk < t1; tk++) {
-                const double ikx = b.x[r] + b.img[3 * tk] - xp, iky = b.y[r] + b.img[3 * tk + 1] - yp,
-                             ikz = b.z[r] + b.img[3 * tk + 2] - zp;
+    double sum = 0.0;
+    if (c6pq != 0.0) {
+        const int t0 = b.img_off[kImgDisp3 * (b.nsys + 1) + sys], nT = b.img_off[kImgDisp3 * (b.nsys + 1) + sys + 1] - t0;
+        const double* img = b.img + 3 * t0;
+        const double cut2 = c.cut3 * c.cut3, alp3 = (d.alp + 2.0) / 3.0;
+        const int sp = b.sp[p], sq = b.sp[q];
+        const double xp = b.x[p], yp = b.y[p], zp = b.z[p];
+        for (int tj = 0; tj < nT; tj++) {
+            const double ijx = b.x[q] + img[3 * tj] - xp, ijy = b.y[q] + img[3 * tj + 1] - yp,
+                         ijz = b.z[q] + img[3 * tj + 2] - zp;
+            const double r2ij = ijx * ijx + ijy * ijy + ijz * ijz;
+            if (r2ij > cut2 || r2ij < DBL_EPSILON) continue;
+            const double2 fij = mp ? mp[off[sys] + (long long)pl * n + ql]
+                                   : pw_factor(r2ij, c6pq, s.atm_r0[sp * b.nid + sq], alp3, c);
+            for (int f = lane; f < n * nT; f += 32) {
+                const int rl = nT == 1 ? f : f / nT, tk = f - rl * nT;
+                const int r = a0 + rl;
+                const double ikx = b.x[r] + img[3 * tk] - xp, iky = b.y[r] + img[3 * tk + 1] - yp,
+                             ikz = b.z[r] + img[3 * tk + 2] - zp;
                 const double r2ik = ikx * ikx + iky * iky + ikz * ikz;
                 if (r2ik > cut2 || r2ik < DBL_EPSILON) continue;
                 const double jkx = ikx - ijx, jky = iky - ijy, jkz = ikz - ijz;
                 const double r2jk = jkx * jkx + jky * jky + jkz * jkz;
                 if (r2jk > cut2 || r2jk < DBL_EPSILON) continue;
-                double sw = swij;
-                if (smooth_on) {
-                    double swik, swjk;
-                    smooth<double>(sqrt(r2ik), c.cut3, c.width3, swik, dsw);
-                    smooth<double>(sqrt(r2jk), c.cut3, c.width3, swjk, dsw);
-                    sw *= swik * swjk;
+                double2 fik, fjk;
+                if (mp) {
+                    fik = mp[off[sys] + (long long)rl * n + pl];
+                    fjk = mp[off[sys] + (long long)rl * n + ql];
+                } else {
+                    const int sr = b.sp[r];
+                    fik = pw_factor(r2ik, cm[(long long)rl * n + pl], s.atm_r0[sp * b.nid + sr], alp3, c);
+                    fjk = pw_factor(r2jk, cm[(long long)rl * n + ql], s.atm_r0[sq * b.nid + sr], alp3, c);
                 }
-                const double r2 = r2ij * r2ik * r2jk;
-                const double r1 = sqrt(r2), r3 = r2 * r1, r5 = r3 * r2;
-                const double fdmp = 1.0 / (1.0 + 6.0 * pow(r0 / r1, alp3));
-                const double ang = 0.375 * (r2ij + r2jk - r2ik) * (r2ij - r2jk + r2ik) * (-r2ij + r2jk + r2ik) / r5
-                                 + 1.0 / r3;
-                const double de = ang * fdmp * c9 * triple * sw / 6.0;
-                epq -= de;
-                epr -= de;
-                eqr -= de;
-            }
-            if (epr != 0.0) {
-                const long long lr = b.local[r];
-                atomicAdd(eg + lp * n + lr, epr);
-                atomicAdd(eg + lr * n + lp, epr);
-                atomicAdd(eg + lq * n + lr, eqr);
-                atomicAdd(eg + lr * n + lq, eqr);
+                sum += pw_triple(r2ij, r2ik, r2jk, fij.x * fik.x * fjk.x, fij.y * fik.y * fjk.y);
             }
         }
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        sum *= d.s9 / 6.0;
     }
-    if (epq != 0.0) {
-        atomicAdd(eg + lp * n + lq, epq);
-        atomicAdd(eg + lq * n + lp, epq);
-    }
+    if (lane != 0) return;
+    double* eg = e3 + off[sys];
+    const long long lp = b.local[p], lq = b.local[q];
+    eg[lp * n + lq] = sum;
+    eg[lq * n + lp] = sum;
 }
 
 }  // namespace
 
 void launch_pairwise(const Batch& b, const Species& s, const Damp& d, const Config& c, const Work& w,
-                     const long long* off, long long total, double* c6, double* e2, double* e3,
-                     cudaStream_t stream)
+                     const long long* off, long long total, bool molecules, double* c6, double* factors, double* e2,
+                     double* e3, cudaStream_t stream)
 {
     if (b.natoms <= 0 || total <= 0) return;
+    const bool threebody = std::fabs(d.s9) >= DBL_EPSILON;
     const unsigned blocks = (unsigned)((total + kPwThreads - 1) / kPwThreads);
-    k_pw_c6<<<blocks, kPwThreads, 0, stream>>>(b, s, w, off, total, c6);
+    double2* mp = threebody && molecules ? reinterpret_cast<double2*>(factors) : nullptr;
+    k_pw_c6<<<blocks, kPwThreads, 0, stream>>>(b, s, c, w, off, total, (d.alp + 2.0) / 3.0, c6, mp);
     k_pairwise2<<<b.natoms, kPwThreads, 0, stream>>>(b, s, d, c, off, c6, e2);
-    cudaMemsetAsync(e3, 0, sizeof(double) * total, stream);
-    if (std::fabs(d.s9) >= DBL_EPSILON)
-        k_pairwise3<<<blocks, kPwThreads, 0, stream>>>(b, s, d, c, off, total, c6, e3);
+    if (threebody)
+        k_pairwise3<<<(unsigned)((32 * total + kPwThreads - 1) / kPwThreads), kPwThreads, 0, stream>>>(b, s, d, c, off,
+                                                                                                   total, c6, mp, e3);
+    else
+        cudaMemsetAsync(e3, 0, sizeof(double) * total, stream);
 }
 
 }  // namespace d3
