@@ -43,6 +43,7 @@
 
 #include "d3_atm_common.cuh"
 #include "d3_device.cuh"
+#include "d3_math.cuh"
 
 namespace d3 {
 
@@ -98,22 +99,6 @@ __device__ __forceinline__ double fixed_value(const unsigned long long* acc2)
 {
     return double((long long)acc2[0]) * 2.3283064365386963e-10 +      // 2^-32
            double((long long)acc2[1]) * 2.117582368135751e-22;        // 2^-72
-}
-
-// 1/x: the hardware approximation (FP32, 1 ulp), or its FP64 form (relative
-// error e0 below 2^-20) with one cubic correction y (1 + e + e^2), e = 1 - x y.
-__device__ __forceinline__ float rcp_fast(float x)
-{
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ double rcp_fast(double x)
-{
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = ::fma(-x, y, 1.0);
-    return ::fma(y, ::fma(e, e, e), y);
 }
 
 // Two values worked on together: the packed FP32 instructions of sm_100 (one

@@ -16,6 +16,7 @@
 #include <cstdint>
 
 #include "d3_device.cuh"
+#include "d3_math.cuh"
 #include "d3_weights.cuh"
 
 namespace d3 {
@@ -115,7 +116,7 @@ __device__ __forceinline__ R rexp(R x) { if constexpr (sizeof(R) == 8) return ex
 template <class R>
 __device__ __forceinline__ R rsqrt_(R x) { if constexpr (sizeof(R) == 8) return sqrt(x); else return sqrtf(x); }
 template <class R>
-__device__ __forceinline__ R rinv_sqrt(R x) { if constexpr (sizeof(R) == 8) return rsqrt(x); else return rsqrtf(x); }
+__device__ __forceinline__ R rinv_sqrt(R x) { if constexpr (sizeof(R) == 8) return rsqrt_fast(x); else return rsqrtf(x); }
 template <class R>
 __device__ __forceinline__ R rpow(R x, R a) { if constexpr (sizeof(R) == 8) return pow(x, a); else return powf(x, a); }
 
@@ -214,7 +215,7 @@ __global__ void __launch_bounds__(kThreads) k_coordination_number(Batch b, Speci
                 displacement(sbuf[wib][k], xj, yj, zj, hj, lj, vx, vy, vz);
                 const R r2 = vx * vx + vy * vy + vz * vz;
                 if (!valid || r2 > cut2 || r2 < R(1.0e-12)) continue;
-                const R cf = R(1) / (R(1) + rexp(-R(kKcn) * (rc * rinv_sqrt(r2) - R(1))));
+                const R cf = inv<R>(R(1) + rexp(-R(kKcn) * (rc * rinv_sqrt(r2) - R(1))));
                 acc += double(cf);
                 nterm += (jj <= i);
             }
@@ -346,6 +347,7 @@ __global__ void __launch_bounds__(kThreads) k_two_body(Batch b, Species s, Damp 
     const bool smooth = c.width2 > 0.0 && c.width2 < c.cut2;
     const R s6 = R(d.s6), s8 = R(d.s8);
     const R alp6 = R(d.alp), alp8 = R(d.alp + 2.0);
+    const int h6 = half_even(d.alp);
     double e = 0, de = 0, gx = 0, gy = 0, gz = 0;
     double sxx = 0, syy = 0, szz = 0, sxy = 0, sxz = 0, syz = 0;
     double pg0 = 0, pg1 = 0, pg2 = 0, pg3 = 0;
@@ -413,9 +415,9 @@ __global__ void __launch_bounds__(kThreads) k_two_body(Batch b, Species s, Damp 
                     const R r4 = r2 * r2;
                     // one reciprocal for both denominators
                     const R a6 = r4 * r2 + q1, a8 = r4 * r4 + q2;
-                    const R inv = R(1) / (a6 * a8);
-                    const R t6 = a8 * inv;
-                    const R t8 = a6 * inv;
+                    const R ia = inv<R>(a6 * a8);
+                    const R t6 = a8 * ia;
+                    const R t8 = a6 * ia;
                     const R d6 = R(-6) * r4 * t6 * t6;
                     const R d8 = R(-8) * r4 * r2 * t8 * t8;
                     e6 = t6; e8 = rrij * t8;
@@ -430,22 +432,29 @@ __global__ void __launch_bounds__(kThreads) k_two_body(Batch b, Species s, Damp 
                     }
                 } else {
                     // q1 = rs6 * R0, q2 = rs8 * R0
-                    if (!smooth) r1 = rsqrt_(r2);
-                    const R r6 = r2 * r2 * r2;
-                    const R r8 = r6 * r2;
-                    const R t6 = rpow<R>(q1 / r1, alp6);
-                    const R t8 = rpow<R>(q2 / r1, alp8);
-                    const R f6 = R(1) / (R(1) + R(6) * t6);
-                    const R f8 = R(1) / (R(1) + R(6) * t8);
-                    const R d6 = R(-6) * f6 / r2 + R(6) * alp6 * t6 * (f6 * f6) / r2;
-                    const R d8 = R(-8) * f8 / r2 + R(6) * alp8 * t8 * (f8 * f8) / r2;
-                    e6 = f6 / r6; e8 = rrij * f8 / r8;
-                    edisp0 = s6 * f6 / r6 + s8 * rrij * f8 / r8;
-                    gdisp0 = s6 * d6 / r6 + s8 * rrij * d8 / r8;
+                    const R ir2 = inv<R>(r2);
+                    const R ir6 = ir2 * ir2 * ir2;
+                    R t6, t8;
+                    if (h6 >= 0) {
+                        t6 = ipow(q1 * q1 * ir2, h6);
+                        t8 = ipow(q2 * q2 * ir2, h6 + 1);
+                    } else {
+                        if (!smooth) r1 = rsqrt_(r2);
+                        t6 = rpow<R>(q1 / r1, alp6);
+                        t8 = rpow<R>(q2 / r1, alp8);
+                    }
+                    const R f6 = inv<R>(R(1) + R(6) * t6);
+                    const R f8 = inv<R>(R(1) + R(6) * t8);
+                    const R d6 = ir2 * f6 * (R(-6) + R(6) * alp6 * t6 * f6);
+                    const R d8 = ir2 * f8 * (R(-8) + R(6) * alp8 * t8 * f8);
+                    const R i8 = rrij * (ir6 * ir2);
+                    e6 = f6 * ir6; e8 = f8 * i8;
+                    edisp0 = s6 * e6 + s8 * e8;
+                    gdisp0 = s6 * d6 * ir6 + s8 * d8 * i8;
                     if (c.param_grad) {
                         // t = (rs R0 / r)^alp: dt/drs = alp t / rs, df/dt = -6 f^2
-                        dpa = d.rs6 != 0.0 ? s6 / r6 * R(-6) * f6 * f6 * alp6 * t6 / R(d.rs6) : R(0);
-                        dpb = d.rs8 != 0.0 ? s8 * rrij / r8 * R(-6) * f8 * f8 * alp8 * t8 / R(d.rs8) : R(0);
+                        dpa = d.rs6 != 0.0 ? s6 * ir6 * R(-6) * f6 * f6 * alp6 * t6 / R(d.rs6) : R(0);
+                        dpb = d.rs8 != 0.0 ? s8 * i8 * R(-6) * f8 * f8 * alp8 * t8 / R(d.rs8) : R(0);
                     }
                 }
                 const R edisp = sw * edisp0;
@@ -543,7 +552,7 @@ __global__ void __launch_bounds__(kThreads) k_cn_chain(Batch b, Species s, Confi
                 if (!valid || r2 > cut2 || r2 < R(1.0e-12)) continue;
                 const R ir = rinv_sqrt(r2);
                 const R expterm = rexp(-R(kKcn) * (rc * ir - R(1)));
-                const R cf = R(1) / (R(1) + expterm);
+                const R cf = inv<R>(R(1) + expterm);
                 // dcf / r with dcf = -cf (1 - cf) kcn rc / r^2 (ncoord.f90:198-201)
                 const R f = -cf * (R(1) - cf) * R(kKcn) * rc * (ir * ir * ir) * dsum;
                 const R cx = f * vx, cy = f * vy, cz = f * vz;

@@ -20,6 +20,7 @@
 #include <cstdint>
 
 #include "d3_device.cuh"
+#include "d3_math.cuh"
 #include "d3_weights.cuh"
 
 namespace d3 {
@@ -42,7 +43,7 @@ template <class R> struct T4;
 template <> struct T4<float> { using type = float4; };
 template <> struct T4<double> { using type = double4; };
 
-template <class R> __device__ __forceinline__ R tt_rcp(R x) { if constexpr (sizeof(R) == 8) return R(1) / x; else return __fdividef(1.0f, x); }
+template <class R> __device__ __forceinline__ R tt_rcp(R x) { if constexpr (sizeof(R) == 8) return rcp_fast(x); else return __fdividef(1.0f, x); }
 template <class R> __device__ __forceinline__ R tt_sqrt(R x) { if constexpr (sizeof(R) == 8) return sqrt(x); else return sqrtf(x); }
 template <class R> __device__ __forceinline__ R tt_pow(R x, R a) { if constexpr (sizeof(R) == 8) return pow(x, a); else return powf(x, a); }
 
@@ -266,29 +267,32 @@ __global__ void k_species_vectors(Batch b, Species s, Work w, R* UV)
 // FP32 form, so that no intermediate leaves the FP32 range.
 template <class R, int DAMP>
 __device__ __forceinline__ void tt_family(R r2, R r1, bool have_r1, R rrij, R q1, R q2, R q3, R q4, R q5, R zc,
-                                          R s6, R s8, R alp6, R alp8, R bet, R a1, R& edisp0, R& gdisp0,
-                                          R& cdisp0)
+                                          R s6, R s8, R alp6, R alp8, R bet, R a1, int h6, int hb, R& edisp0,
+                                          R& gdisp0, R& cdisp0)
 {
     if constexpr (DAMP == kMZero) {
         if (!have_r1) r1 = tt_sqrt<R>(r2);
-        const R r6 = r2 * r2 * r2;
-        const R r8 = r6 * r2;
-        const R t6 = tt_pow<R>(r1 * q1 + q3, -alp6);
-        const R t8 = tt_pow<R>(r1 * q2 + q3, -alp8);
-        const R f6 = R(1) / (R(1) + R(6) * t6);
-        const R f8 = R(1) / (R(1) + R(6) * t8);
-        const R d6 = R(-6) * f6 / r2 + R(6) * alp6 * t6 * (f6 * f6) / (r2 + q4 * r1);
-        const R d8 = R(-8) * f8 / r2 + R(6) * alp8 * t8 * (f8 * f8) / (r2 + q5 * r1);
-        edisp0 = s6 * f6 / r6 + s8 * rrij * f8 / r8;
-        gdisp0 = s6 * d6 / r6 + s8 * rrij * d8 / r8;
+        const R ir2 = inv<R>(r2);
+        const R ir6 = ir2 * ir2 * ir2;
+        const R x6 = inv<R>(r1 * q1 + q3), x8 = inv<R>(r1 * q2 + q3);
+        const R t6 = h6 >= 0 ? ipow(x6 * x6, h6) : tt_pow<R>(x6, alp6);
+        const R t8 = h6 >= 0 ? ipow(x8 * x8, h6 + 1) : tt_pow<R>(x8, alp8);
+        const R f6 = inv<R>(R(1) + R(6) * t6);
+        const R f8 = inv<R>(R(1) + R(6) * t8);
+        const R d6 = R(-6) * f6 * ir2 + R(6) * alp6 * t6 * (f6 * f6) * inv<R>(r2 + q4 * r1);
+        const R d8 = R(-8) * f8 * ir2 + R(6) * alp8 * t8 * (f8 * f8) * inv<R>(r2 + q5 * r1);
+        const R c6 = s6 * ir6, c8 = s8 * rrij * (ir6 * ir2);
+        edisp0 = c6 * f6 + c8 * f8;
+        gdisp0 = c6 * d6 + c8 * d8;
     } else if constexpr (DAMP == kOptimizedPower) {
         // t6 = r^b / (r^b r^6 + q1) = 1 / (r^6 + q1 r^-b)
-        const R ib = tt_pow<R>(r2, R(-0.5) * bet);
+        const R ir2 = inv<R>(r2);
+        const R ib = hb >= 0 ? ipow(ir2, hb) : tt_pow<R>(r2, R(-0.5) * bet);
         const R r4 = r2 * r2;
-        const R t6 = R(1) / (r4 * r2 + q1 * ib);
-        const R t8 = R(1) / (r4 * r4 + q2 * ib);
-        const R d6 = R(-6) * r4 * t6 * t6 + bet * q1 * t6 * t6 * ib / r2;
-        const R d8 = R(-8) * r4 * r2 * t8 * t8 + bet * q2 * t8 * t8 * ib / r2;
+        const R t6 = inv<R>(r4 * r2 + q1 * ib);
+        const R t8 = inv<R>(r4 * r4 + q2 * ib);
+        const R d6 = R(-6) * r4 * t6 * t6 + bet * q1 * t6 * t6 * ib * ir2;
+        const R d8 = R(-8) * r4 * r2 * t8 * t8 + bet * q2 * t8 * t8 * ib * ir2;
         edisp0 = s6 * t6 + s8 * rrij * t8;
         gdisp0 = s6 * d6 + s8 * rrij * d8;
     } else if constexpr (DAMP == kCSO) {
@@ -305,7 +309,7 @@ __device__ __forceinline__ void tt_family(R r2, R r1, bool have_r1, R rrij, R q1
         }
         const R sig = s6 + a1 * sf;
         const R r4 = r2 * r2;
-        const R t6 = R(1) / (r4 * r2 + q1);
+        const R t6 = inv<R>(r4 * r2 + q1);
         const R dsig = -a1 * sf * om / r1;
         const R dt6 = R(-6) * r4 * t6 * t6;
         edisp0 = sig * t6;
@@ -313,8 +317,8 @@ __device__ __forceinline__ void tt_family(R r2, R r1, bool have_r1, R rrij, R q1
     } else {
         const R r4 = r2 * r2;
         const R r6 = r4 * r2, r8 = r4 * r4;
-        const R t6 = R(1) / (r6 + zc);
-        const R t8 = R(1) / (r8 + zc * rrij);
+        const R t6 = inv<R>(r6 + zc);
+        const R t8 = inv<R>(r8 + zc * rrij);
         const R s8rr = s8 * rrij;
         edisp0 = s6 * t6 + s8rr * t8;
         gdisp0 = R(-6) * s6 * (r4 * t6) * t6 + R(-8) * s8rr * (r4 * r2 * t8) * t8;
@@ -385,6 +389,7 @@ k_two_body_tt(Batch b, Species s, Damp d, Config c, Partition p, Work w, const i
     const R cutoff = R(c.cut2), cut2 = R(c.cut2 * c.cut2), width = R(c.width2);
     const R s6 = R(d.s6), s8 = R(d.s8);
     const R alp6 = R(d.alp), alp8 = R(d.alp + 2.0);
+    const int h6 = half_even(d.alp), hb = half_even(d.bet);
     const R bet = R(d.bet), a1 = R(d.a1);
     const int zsi = DAMP == kZDamping ? b.zid[ic] : 0;
     const int nid = b.nid;
@@ -512,26 +517,33 @@ k_two_body_tt(Batch b, Species s, Damp d, Config c, Partition p, Work w, const i
                     }
                 } else if constexpr (DAMP == kZero) {
                     // zero.f90:490-536: q1 = rs6 R0, q2 = rs8 R0
-                    if (!SMOOTH) r1 = tt_sqrt<R>(r2);
-                    const R r6 = r2 * r2 * r2;
-                    const R r8 = r6 * r2;
-                    const R t6 = tt_pow<R>(q1 / r1, alp6);
-                    const R t8 = tt_pow<R>(q2 / r1, alp8);
-                    const R f6 = R(1) / (R(1) + R(6) * t6);
-                    const R f8 = R(1) / (R(1) + R(6) * t8);
-                    const R d6 = R(-6) * f6 / r2 + R(6) * alp6 * t6 * (f6 * f6) / r2;
-                    const R d8 = R(-8) * f8 / r2 + R(6) * alp8 * t8 * (f8 * f8) / r2;
-                    e6 = f6 / r6; e8 = rrij * f8 / r8;
-                    edisp0 = s6 * f6 / r6 + s8 * rrij * f8 / r8;
-                    gdisp0 = s6 * d6 / r6 + s8 * rrij * d8 / r8;
+                    const R ir2 = inv<R>(r2);
+                    const R ir6 = ir2 * ir2 * ir2;
+                    R t6, t8;
+                    if (h6 >= 0) {
+                        t6 = ipow(q1 * q1 * ir2, h6);
+                        t8 = ipow(q2 * q2 * ir2, h6 + 1);
+                    } else {
+                        if (!SMOOTH) r1 = tt_sqrt<R>(r2);
+                        t6 = tt_pow<R>(q1 / r1, alp6);
+                        t8 = tt_pow<R>(q2 / r1, alp8);
+                    }
+                    const R f6 = inv<R>(R(1) + R(6) * t6);
+                    const R f8 = inv<R>(R(1) + R(6) * t8);
+                    const R d6 = ir2 * f6 * (R(-6) + R(6) * alp6 * t6 * f6);
+                    const R d8 = ir2 * f8 * (R(-8) + R(6) * alp8 * t8 * f8);
+                    const R i8 = rrij * (ir6 * ir2);
+                    e6 = f6 * ir6; e8 = f8 * i8;
+                    edisp0 = s6 * e6 + s8 * e8;
+                    gdisp0 = s6 * d6 * ir6 + s8 * d8 * i8;
                     if (PG) {
-                        dpa = d.rs6 != 0.0 ? s6 / r6 * R(-6) * f6 * f6 * alp6 * t6 / R(d.rs6) : R(0);
-                        dpb = d.rs8 != 0.0 ? s8 * rrij / r8 * R(-6) * f8 * f8 * alp8 * t8 / R(d.rs8) : R(0);
+                        dpa = d.rs6 != 0.0 ? s6 * ir6 * R(-6) * f6 * f6 * alp6 * t6 / R(d.rs6) : R(0);
+                        dpb = d.rs8 != 0.0 ? s8 * i8 * R(-6) * f8 * f8 * alp8 * t8 / R(d.rs8) : R(0);
                     }
                 } else {
                     e6 = e8 = R(0);
                     tt_family<R, DAMP>(r2, r1, SMOOTH, rrij, q1, q2, q3, q4, q5, zc, s6, s8, alp6, alp8, bet, a1,
-                                       edisp0, gdisp0, cdisp0);
+                                       h6, hb, edisp0, gdisp0, cdisp0);
                 }
                 se += sw * edisp0;
                 if (DAMP == kZDamping) sc += sw * cdisp0;
@@ -708,6 +720,7 @@ k_two_body_rot(Batch b, Species s, Damp d, Config c, Work w, const int2* units, 
     const R cut2 = R(c.cut2 * c.cut2);
     const R s6 = R(d.s6), s8 = R(d.s8);
     const R alp6 = R(d.alp), alp8 = R(d.alp + 2.0);
+    const int h6 = half_even(d.alp);
     const bool iok = ivalid && !gi;
     const bool half = diag && lane >= 16;
     const int st0 = diag ? 1 : 0, st1 = diag ? 16 : 31;
@@ -761,18 +774,25 @@ k_two_body_rot(Batch b, Species s, Damp d, Config c, Work w, const int2* units, 
             } else {
                 // zero.f90:490-536 with q1 = rs6 R0, q2 = rs8 R0 (a rejected term at r^2 = 1, weight 0)
                 const R r2 = ok ? r2raw : R(1);
-                const R r1 = tt_sqrt<R>(r2);
-                const R r6 = r2 * r2 * r2;
-                const R r8 = r6 * r2;
-                const R t6 = tt_pow<R>(q1 / r1, alp6);
-                const R t8 = tt_pow<R>(q2 / r1, alp8);
-                const R f6 = R(1) / (R(1) + R(6) * t6);
-                const R f8 = R(1) / (R(1) + R(6) * t8);
-                const R d6 = R(-6) * f6 / r2 + R(6) * alp6 * t6 * (f6 * f6) / r2;
-                const R d8 = R(-8) * f8 / r2 + R(6) * alp8 * t8 * (f8 * f8) / r2;
+                const R ir2 = inv<R>(r2);
+                const R ir6 = ir2 * ir2 * ir2;
+                R t6, t8;
+                if (h6 >= 0) {
+                    t6 = ipow(q1 * q1 * ir2, h6);
+                    t8 = ipow(q2 * q2 * ir2, h6 + 1);
+                } else {
+                    const R r1 = tt_sqrt<R>(r2);
+                    t6 = tt_pow<R>(q1 / r1, alp6);
+                    t8 = tt_pow<R>(q2 / r1, alp8);
+                }
+                const R f6 = inv<R>(R(1) + R(6) * t6);
+                const R f8 = inv<R>(R(1) + R(6) * t8);
+                const R d6 = ir2 * f6 * (R(-6) + R(6) * alp6 * t6 * f6);
+                const R d8 = ir2 * f8 * (R(-8) + R(6) * alp8 * t8 * f8);
                 const R sw = ok ? R(1) : R(0);
-                edisp0 = sw * (s6 * f6 / r6 + s8 * rrij * f8 / r8);
-                gdisp0 = sw * (s6 * d6 / r6 + s8 * rrij * d8 / r8);
+                const R w6 = sw * s6 * ir6, w8 = sw * s8 * rrij * (ir6 * ir2);
+                edisp0 = w6 * f6 + w8 * f8;
+                gdisp0 = w6 * d6 + w8 * d8;
             }
             // E_pair = -C6 edisp (both halves to i), dE/dCN = -dC6/dCN edisp, gradient -C6 gdisp v
             // (rational.f90:488-497)
@@ -901,9 +921,9 @@ k_cn_rot(Batch b, Species s, Config c, Work w, const int2* units, int nunits, do
             const R rc = R(rci + rcj);
             const R rr = ok ? r2 : R(1);
             if constexpr (sizeof(R) == 8) {
-                const R r1 = sqrt(rr);
-                cf = R(1) / (R(1) + exp(-R(kKcnTT) * (rc / r1 - R(1))));
-                f = -cf * (R(1) - cf) * R(kKcnTT) * rc / rr / r1;
+                const R ir = rsqrt_fast(rr);
+                cf = rcp_fast(R(1) + exp(-R(kKcnTT) * (rc * ir - R(1))));
+                f = -cf * (R(1) - cf) * R(kKcnTT) * rc * (ir * ir * ir);
             } else {
                 const R ir = rsqrtf(rr);
                 cf = __fdividef(1.0f, 1.0f + expf(-R(kKcnTT) * (rc * ir - R(1))));
@@ -1187,9 +1207,9 @@ __device__ __forceinline__ void cn_tt(const Batch& b, const Species& s, const Co
                     // the count and the chain rule's countd of the same term (ncoord.f90:198-206)
                     R cf, f;
                     if constexpr (sizeof(R) == 8) {
-                        const R r1 = sqrt(r2);
-                        cf = R(1) / (R(1) + exp(-R(kKcnTT) * (rc / r1 - R(1))));
-                        f = -cf * (R(1) - cf) * R(kKcnTT) * rc / r2 / r1;
+                        const R ir = rsqrt_fast(r2);
+                        cf = rcp_fast(R(1) + exp(-R(kKcnTT) * (rc * ir - R(1))));
+                        f = -cf * (R(1) - cf) * R(kKcnTT) * rc * (ir * ir * ir);
                     } else {
                         const R ir = rsqrtf(r2);
                         cf = __fdividef(1.0f, 1.0f + expf(-R(kKcnTT) * (rc * ir - R(1))));
@@ -1203,7 +1223,7 @@ __device__ __forceinline__ void cn_tt(const Batch& b, const Species& s, const Co
                     sxy += cx * vy; sxz += cx * vz; syz += cy * vz;
                 } else {
                     R cf;
-                    if constexpr (sizeof(R) == 8) cf = R(1) / (R(1) + exp(-R(kKcnTT) * (rc / sqrt(r2) - R(1))));
+                    if constexpr (sizeof(R) == 8) cf = rcp_fast(R(1) + exp(-R(kKcnTT) * (rc * rsqrt_fast(r2) - R(1))));
                     else cf = __fdividef(1.0f, 1.0f + expf(-R(kKcnTT) * (rc * rsqrtf(r2) - R(1))));
                     sc += ok ? cf : R(0);
                 }
