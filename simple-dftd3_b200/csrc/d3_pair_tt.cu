@@ -97,12 +97,13 @@ __device__ __forceinline__ R wsum4_tt(R a, R b, R c, R d, int lane)
     return z;
 }
 
-// The FP32 sweeps take two translations per step (the second masked off
-// when a mask word has an odd count), branch-free, for instruction-level
-// parallelism.  The FP64 sweeps, at the register limit, take one, and only
-// the lanes whose term is taken run the FP64 math (its library sqrt, exp and
-// divisions cost more issue slots than the divergence; measured on B200).
-template <class R> constexpr bool kPairStep = sizeof(R) == 4;
+// The sweeps take two translations per step, for instruction-level parallelism.
+// FP32: always, the second masked off when a mask word has an odd count; a
+// rejected lane evaluates its term at r^2 = 1 with weight 0.  FP64: where a second
+// one is left (a periodic 2000-atom cell 512 -> 472 us with the branch-free
+// reciprocals); a single one, as every partner in a molecule has, is evaluated by
+// the lanes whose term is taken alone.
+template <class R> constexpr bool kSingleStep = sizeof(R) == 8;
 
 // Distance vector v = x_i - x_j - T of a staged translation q (head and
 // tail in the mixed form) and whether its term is taken: r^2 in [eps, cut2v]
@@ -567,7 +568,7 @@ k_two_body_tt(Batch b, Species s, Damp d, Config c, Partition p, Work w, const i
                 for (unsigned mm = jm[h]; mm;) {
                     const int qa = qh + __ffs(mm);
                     mm &= mm - 1;
-                    if constexpr (kPairStep<R>) {
+                    if (!kSingleStep<R> || mm) {
                         const bool two = mm != 0u;
                         const int qb = two ? qh + __ffs(mm) : qa;
                         mm &= mm - 1;
@@ -1237,7 +1238,7 @@ __device__ __forceinline__ void cn_tt(const Batch& b, const Species& s, const Co
                 for (unsigned mm = jm[h]; mm;) {
                     const int qa = qh + __ffs(mm);
                     mm &= mm - 1;
-                    if constexpr (kPairStep<R>) {
+                    if (!kSingleStep<R> || mm) {
                         const bool two = mm != 0u;
                         const int qb = two ? qh + __ffs(mm) : qa;
                         mm &= mm - 1;
