@@ -155,8 +155,9 @@ dftd3_b200_set_batch_graph(dftd3_error /* error */,
  * the default, Morton order with 3 Bohr cells for systems above 16384 atoms;
  * > 0: Morton order with keys quantised to cells of that many Bohr),
  * tuning[1] work items per tile pair of the pair sweeps (1, 2
- * or 4; 0 chooses 1 for batches of molecules, else 2, and 1 for the CN
- * sweeps of the mixed form when the tile pairs give every SM eight warps),
+ * or 4; 0 chooses 1 for batches of molecules, else 2, 1 for the CN sweeps of
+ * the mixed form when the tile pairs give every SM eight warps, and 8 to 32
+ * where the tile pairs are too few to give every SM work),
  * tuning[2] resident blocks per SM of the three-body kernel (0 = occupancy
  * limit), tuning[3] 0, 1 or 2, accepted for callers that set it: one
  * three-body kernel serves molecules and periodic systems. */

@@ -87,7 +87,8 @@ struct PairUnits {
     const int2* units = nullptr;         // [nunits] global tile indices (it, jt)
     int nunits = 0;
     const int* unit_base = nullptr;      // [nsys]
-    int split = 4;                       // items per unit: 1, 2 (j-tile halves), 4 (and translation halves)
+    int split = 4;                       // items per unit: 1, 2 (j-tile halves), 4 (and translation halves),
+                                         // 8, 16, 32 (that many parts of the j tile)
     bool single_image = false;           // every system has the lattice point T = 0 only (molecules) and
                                          // the two-body sum takes the diagonal walk (k_two_body_rot)
     void* U = nullptr;                   // [natoms][nid][16] species vectors U (7 + pad) and dU (7 + pad) (R)
@@ -173,8 +174,8 @@ struct Tuning {
     double morton_cell = 0.0;      // spatial order: 0 = column order (compact tiles; Morton with 3 Bohr
                                    // cells for systems above kRankOrderMax atoms), > 0 = Morton order
                                    // with keys quantised to cells of this many Bohr
-    int pair_split = 0;            // work items per tile pair of the pair sweeps: 1, 2 or 4; 0 = 1 for
-                                   // molecules, else 2 (mixed form) or 4 (FP64 form)
+    int pair_split = 0;            // work items per tile pair of the pair sweeps: 1, 2 or 4; 0 = chosen by
+                                   // the number of tile pairs (Engine::pair_split)
     int atm_blocks_per_sm = 0;     // resident blocks per SM of the triple kernel; 0 = occupancy
     int atm_mol = 0;               // 0, 1 or 2: accepted for callers that set it, one kernel serves all systems
 };
@@ -273,8 +274,8 @@ size_t cn_store_bytes(const PairUnits& pu, bool mixed);   // d3_pair_tt.cu
 constexpr int kCnStoreChunk = 128; // translations of a system the stored chain rule covers
 void launch_cn_units(const Batch& b, const Species& s, const Config& c, const Partition& p, const Work& w,
                      const PairUnits& pu, bool chain, cudaStream_t stream, bool weights = false, void* uv = nullptr);
-size_t pair_unit_slot_doubles();   // per unit: i and j slots
-size_t pair_unit_i_doubles();      // per unit: i slots
+size_t pair_unit_slot_doubles();   // per item: i and j slots
+size_t pair_unit_i_doubles();      // per item: i slots
 size_t species_vector_doubles(int natoms, int nid);   // PairUnits::U (FP64 size)
 // Species vectors U[a][s][r] = sum_q C6ref(r of s, q of atom a's species) gw_a[q]
 // and dU with dgw (zero for ghosts), in the arithmetic type of the form.

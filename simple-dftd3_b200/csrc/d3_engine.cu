@@ -276,8 +276,12 @@ Engine::Engine(int nsys, const int* natoms, const int* numbers, const double* la
     pu_.units = d_units_;
     pu_.unit_base = d_unit_base_;
     pu_.U = dev_alloc<double>(species_vector_doubles(natoms_, nid));
-    pu_.unit_i = dev_alloc<double>((size_t)std::max(pu_.nunits, 1) * pair_unit_slot_doubles());
-    pu_.unit_j = pu_.unit_i + (size_t)std::max(pu_.nunits, 1) * pair_unit_i_doubles();
+    // slots for the largest split: four, or more for few tile pairs
+    max_split_ = 4;
+    while (max_split_ < 32 && (long long)pu_.nunits * max_split_ < 6LL * sms_) max_split_ *= 2;
+    const size_t items = (size_t)std::max(pu_.nunits, 1) * max_split_;
+    pu_.unit_i = dev_alloc<double>(items * pair_unit_slot_doubles());
+    pu_.unit_j = pu_.unit_i + items * pair_unit_i_doubles();
     d_tile_off_ = dev_alloc<int>(nsys + 1);
     d_tile_sys_ = dev_alloc<int>(std::max(ntiles_, 1));
     up(d_tile_off_, tile_off.data(), sizeof(int) * (nsys + 1));
@@ -291,10 +295,8 @@ Engine::Engine(int nsys, const int* natoms, const int* numbers, const double* la
     }
     c6mat_total_ = off;
     sys_natoms_.assign(natoms, natoms + nsys);
-    auto_split_ = 1;
-    for (int sy = 0; sy < nsys; sy++)
-        if (per_[3 * sy] || per_[3 * sy + 1] || per_[3 * sy + 2]) auto_split_ = 2;
-    any_periodic_ = auto_split_ == 2;
+    any_periodic_ = false;
+    for (int sy = 0; sy < nsys; sy++) any_periodic_ = any_periodic_ || periodic_any(sy);
     t8_off_.assign(nsys + 1, 0);
     for (int sy = 0; sy < nsys; sy++) t8_off_[sy + 1] = t8_off_[sy] + (natoms[sy] + 7) / 8;
     ntiles8_ = t8_off_[nsys];
@@ -679,20 +681,40 @@ void Engine::pairwise_host(const Damp& d, const double* positions, double* energ
     check(cudaStreamSynchronize(stream), "pairwise");
 }
 
-// Items per tile pair with tuning 0 (measured on B200): one for batches of
-// molecules; for periodic systems two, and for the CN sweeps of the mixed
-// form one once the units alone give every SM eight warps.
+// Items per tile pair with tuning 0 (measured on B200): one for molecules, two for
+// periodic systems, and for the CN sweeps of the mixed form one once the tile pairs
+// alone give every SM eight warps.  Where that leaves SMs without work, the j tile is
+// cut into 8, 16 or 32 parts until the items give every SM so many warps: six in the
+// FP64 form and four in the mixed form of periodic systems, two for molecules, whose
+// items have one term per partner.  Whole calls with two (one) items against that:
+// 60-atom slab 637 -> 116 us, cells of 300, 500 and 900 atoms 530 -> 167, 432 -> 202
+// and 294 -> 254 us, 300-atom cluster 161 -> 104 us (with four warps 108, eight 127),
+// 400-atom frame, mixed, 313 -> 295 us (with eight warps 369).
+int Engine::auto_split(int least) const
+{
+    const long long want = (long long)sms_ * (any_periodic_ ? (mixed_ ? 4 : 6) : 2);
+    int split = least;
+    while (split < max_split_ && pu_.nunits * (long long)split < want) split = split < 8 ? 8 : 2 * split;
+    return std::min(split, max_split_);
+}
+
+// Molecules: the two-body and CN diagonal walks (FP64 only for systems of at most
+// 256 atoms, where few tile pairs lie beyond the cutoff), which take whole units.
+bool Engine::diagonal_walks() const { return !any_periodic_ && (mixed_ || max_sys_atoms_ <= 256); }
+
 int Engine::pair_split() const
 {
     if (tune_.pair_split) return tune_.pair_split;
-    return auto_split_ == 1 ? 1 : 2;
+    if (diagonal_walks()) return 1;
+    return auto_split(any_periodic_ ? 2 : 1);
 }
 
 int Engine::cn_split() const
 {
     if (tune_.pair_split) return tune_.pair_split;
-    if (auto_split_ == 1) return 1;
-    return mixed_ && pu_.nunits >= 8 * sms_ ? 1 : 2;
+    if (diagonal_walks()) return 1;
+    if (!any_periodic_) return auto_split(1);
+    return mixed_ && pu_.nunits >= 8 * sms_ ? 1 : auto_split(2);
 }
 
 void Engine::hessian_host(const Damp& d, const double* positions, double* hessian)
@@ -766,9 +788,7 @@ void Engine::run(const Damp& d, const double* d_positions, double* d_energies, d
     c.grad = grad; c.mixed = mixed_; c.param_grad = pg; c.cn_partitioned = cn_partitioned_;
     // the CN sweeps and the two-body sweep split the tile pairs each their own way
     pu_.split = pair_split();
-    // molecules: the two-body diagonal walk (FP64 only for systems of at most
-    // 256 atoms, where few tile pairs lie beyond the cutoff)
-    pu_.single_image = !any_periodic_ && (mixed_ || max_sys_atoms_ <= 256);
+    pu_.single_image = diagonal_walks();
     PairUnits pcn = pu_;
     pcn.split = cn_split();
     // the CN pass keeps the chain rule's per-pair sums when every system's CN
@@ -783,7 +803,7 @@ void Engine::run(const Damp& d, const double* d_positions, double* d_energies, d
                 void* ok = d_cn_store_ok_;
                 free_block(ok);
                 d_cn_store_ = dev_alloc<unsigned char>(bytes);
-                d_cn_store_ok_ = dev_alloc<unsigned char>((size_t)pu_.nunits * 4);
+                d_cn_store_ok_ = dev_alloc<unsigned char>((size_t)pu_.nunits * max_split_);
                 cn_store_cap_ = bytes;
             }
             pcn.cn_store = d_cn_store_;

@@ -188,7 +188,9 @@ private:
     int2* d_units_ = nullptr;
     int* d_unit_base_ = nullptr;
     std::vector<int> sys_natoms_;
-    int auto_split_ = 1;                 // pair split of tuning 0
+    int max_split_ = 4;                  // items per tile pair the slots are sized for
+    int auto_split(int least) const;
+    bool diagonal_walks() const;
     int pair_split() const;              // items per tile pair of the two-body sweep
     int cn_split() const;                // items per tile pair of the CN sweeps
     bool any_periodic_ = false;          // a system has a periodic direction

@@ -36,8 +36,6 @@ constexpr int kCnStore = 3;       // stored chain-rule sums per (i, j): countd (
 constexpr double kKcnTT = 16.0;   // ncoord.f90:31
 constexpr int kCnSigJ = 8;        // stored-sum CN pass: unit_i slots 8 .. 14 hold the j sums
                                   // (cn, countd v^T (6)) of the column atoms
-constexpr int kSplitMax = 4;      // a unit is evaluated as 1, 2 (j-tile halves) or 4 items
-                                  // (and translation halves); slots are sized for the largest split
 
 template <class R> struct T4;
 template <> struct T4<float> { using type = float4; };
@@ -135,9 +133,10 @@ __device__ __forceinline__ TTGeo<R> tt_geo(const V* sth, const V* stl, int q, R 
 }
 
 // Items of a unit: split 2 halves the j tile, split 4 also halves the
-// translations; item sub of a unit takes j half sub % splitJ and
-// translation half sub / splitJ.
-__host__ __device__ __forceinline__ int tt_split_j(int split) { return split >= 2 ? 2 : 1; }
+// translations; 8, 16 and 32 (small systems, whose units alone leave most SMs
+// idle) cut the j tile into that many parts.  Item sub of a unit takes j part
+// sub % splitJ and translation half sub / splitJ.
+__host__ __device__ __forceinline__ int tt_split_j(int split) { return split > 4 ? split : split >= 2 ? 2 : 1; }
 
 // Species vectors U and dU of one (atom, species) entry, padded to 8.
 template <class R>
@@ -1033,7 +1032,7 @@ __device__ __forceinline__ double tt_gather_atom(long long base, int tl, int nt,
 {
     constexpr int VI = KI <= 1 ? 1 : KI <= 2 ? 2 : KI <= 4 ? 4 : KI <= 8 ? 8 : 16;
     constexpr int VJ = KJ <= 1 ? 1 : KJ <= 2 ? 2 : KJ <= 4 ? 4 : 8;
-    const int sh = split >> 1;   // log2 of the split (1, 2 or 4)
+    const int sh = __ffs(split) - 1;   // log2 of the split
     double si = 0.0, sj = 0.0;
     if (lane % VI < KI) {
         const long long i0 = (base + (long long)tl * (tl + 1) / 2) * split;
@@ -1599,8 +1598,8 @@ size_t cn_store_bytes(const PairUnits& pu, bool mixed)
            (mixed ? sizeof(float) : sizeof(double));
 }
 
-size_t pair_unit_slot_doubles() { return (size_t)kSplitMax * kTile * (kUnitI + kUnitJ); }
-size_t pair_unit_i_doubles() { return (size_t)kSplitMax * kTile * kUnitI; }
+size_t pair_unit_slot_doubles() { return (size_t)kTile * (kUnitI + kUnitJ); }
+size_t pair_unit_i_doubles() { return (size_t)kTile * kUnitI; }
 size_t species_vector_doubles(int natoms, int nid) { return (size_t)natoms * nid * 2 * kRefPad; }
 
 void launch_species_vectors(const Batch& b, const Species& s, const Config& c, const Work& w, void* U,
