@@ -144,7 +144,9 @@ dftd3_b200_get_batch_graph_kernels(dftd3_error /* error */,
  * later evaluations launch the graph on the caller's stream.  Inputs and
  * outputs are staged through buffers the batch owns.  Per-stage times are
  * not recorded for graph replays.  A replay whose three-body blocks outgrow
- * the captured buffers is detected and evaluated again without the graph. */
+ * the captured buffers is detected and evaluated again without the graph.
+ * Host-buffer evaluations of a few molecules of at most 256 atoms take one to
+ * four launches without copies and are not captured. */
 SDFTD3_API_ENTRY void SDFTD3_API_CALL
 dftd3_b200_set_batch_graph(dftd3_error /* error */,
                            dftd3_b200_batch /* batch */,

@@ -594,10 +594,15 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
             }
             zx[p] = pk(r0.x, r1.x); zu[p] = pk(r0.y, r1.y); zm[p] = pk(r0.z, r1.z); zp[p] = pk(r0.w, r1.w);
         }
-        const int2 range = v.range[id.t8 + J];
-        const int4* list = v.list + v.list_off[id.sys] + (long long)J * nt8 * nT;
-        const int nE = range.y;
-        int e0 = (same ? 0 : range.x) + piece;
+        // root tiles from the lists of J, or (one lattice point, no lists) all tiles
+        const int4* list = nullptr;
+        int nE = nt8, e0 = (same ? 0 : J + 1) + piece;
+        if (PER || v.list) {
+            const int2 range = v.range[id.t8 + J];
+            list = v.list + v.list_off[id.sys] + (long long)J * nt8 * nT;
+            nE = range.y;
+            e0 = (same ? 0 : range.x) + piece;
+        }
         int head = 0, cnt = 0;
         while (true) {
             // roots: tiles I (and images) with a pair in reach of both J and K
@@ -607,10 +612,20 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
                 unsigned m = 0;
                 int bij = 0, bik = 0, I = 0, fl = 0;
                 if (e < nE) {
-                    const int4 en = list[e];
-                    bij = en.x;
-                    I = en.y & 0xffffff;
-                    const int tI = en.z;
+                    int tI = 0;
+                    unsigned mij;
+                    if (PER || list) {
+                        const int4 en = list[e];
+                        bij = en.x;
+                        I = en.y & 0xffffff;
+                        mij = (unsigned)en.y >> 24;
+                        tI = en.z;
+                    } else {
+                        I = e;
+                        bij = (int)(I < J ? cbase + (long long)J * (J + 1) / 2 + I : cbase + (long long)I * (I + 1) / 2 + J);
+                        mij = v.mask[bij];
+                        mij = I < J ? mij >> 8 : mij & 0xffu;
+                    }
                     int d = 0;
                     bool in = true;
                     const bool tr = I < J;                  // block stored as (J, I)
@@ -627,7 +642,7 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
                         const long long cik = tr ? cbase + ((long long)J * (J + 1) / 2 + I) * nT + d
                                                  : cbase + ((long long)I * (I + 1) / 2 + K) * nT + d;
                         m = v.mask[cik];
-                        m = ((unsigned)en.y >> 24) & (tr ? m >> 8 : m & 0xffu);
+                        m = mij & (tr ? m >> 8 : m & 0xffu);
                         if (m) bik = (int)(v.map ? v.map[cik] : cik);
                         fl = (tr ? 1 : 0) | (same && I == J ? 2 : 0) | tI << 2;
                     }

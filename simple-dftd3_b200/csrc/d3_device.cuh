@@ -302,7 +302,8 @@ struct AtmView {
     int* sub = nullptr;                    // [ntiles8][8] atom of each tile slot, or -1
     double4* pos = nullptr;                // [ntiles8][8] its position, and the atom
     const long long* list_off = nullptr;   // [nsys] first root list entry
-    const int4* list = nullptr;            // root tiles of tile J of a system: from list_off + J nt8 nT
+    const int4* list = nullptr;            // root tiles of tile J of a system: from list_off + J nt8 nT; null
+                                           // (one lattice point): all tiles
     const int2* range = nullptr;           // [ntiles8] first entry with I > J, number of entries
     const int* map = nullptr;              // [ncand + 1] block of each candidate (a kept one raises the next
                                            // entry), or null: every candidate has its block
@@ -345,6 +346,32 @@ void launch_atm_pairs(const Batch& b, const Species& s, const Config& c, const W
 void launch_atm_lists(const AtmView& v, int ntiles8, const int* tile8_sys, const long long* list_off, int4* list,
                       int2* range, const int* guard, cudaStream_t stream);
 void launch_atm_triples(const AtmLaunch& l);
+// Small molecules (d3_molecule.cu): systems of one lattice point and at most
+// kMolAtoms atoms, in input order, one cluster of blocks per system.
+constexpr int kMolAtoms = 256;
+constexpr int kMolSlots = 8;      // atoms per three-body tile
+constexpr int kMolSpecies = 12;   // species of the batch at most (48 KB of shared memory)
+struct MolArgs {
+    Batch b;
+    Species s;
+    Damp d;
+    Config c;
+    Work w;
+    AtmView v;
+    int two_body = 1;                    // the two-body sum contributes
+    const double* pos = nullptr;         // [natoms][3] device or pinned host memory
+    double *x = nullptr, *y = nullptr, *z = nullptr;
+    void* UV = nullptr;                  // species vectors
+    void* fstore = nullptr;              // [natoms][kMolAtoms] CN derivatives of the pairs (with the three-body term)
+    unsigned long long *fxf = nullptr, *fxe = nullptr, *queue = nullptr;
+    double *energies = nullptr, *sigma9 = nullptr, *grad_out = nullptr;   // device or pinned host memory
+};
+int mol_cluster_size(int max_atoms);
+bool mol_cluster_fits(int cluster);      // the device can hold such a cluster
+// last: without the three-body term, up to the results; otherwise the state for the
+// three-body kernels (no launch_atm_order), followed by launch_mol_finish.
+void launch_mol_pairs(const MolArgs& a, int cluster, bool last, cudaStream_t stream);
+void launch_mol_finish(const MolArgs& a, int cluster, cudaStream_t stream);
 // Adds the gradient and dE/dCN, writes e3 and sig3 (and the triple count).
 void launch_atm_finish(const Batch& b, const Config& c, const AtmView& v, int ntiles8, double s9,
                        const unsigned long long* fxf, const unsigned long long* fxe, const unsigned long long* queue,

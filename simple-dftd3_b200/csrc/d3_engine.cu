@@ -763,6 +763,59 @@ bool Engine::direct_pairs(const Damp& d, bool pg) const
     return small_systems();
 }
 
+// Blocks per system of the small-molecule kernels (d3_molecule.cu), 0 where they do
+// not apply: systems of one lattice point and at most kMolAtoms atoms of at most
+// kMolSpecies species, up to about
+// one block per SM in all (more systems than that fill the GPU with the kernels of
+// the batches), no partition, reducer, parameter derivatives or counters; with
+// profiling the staged kernels run, whose times are asked for.
+int Engine::molecule_cluster(const Damp&, bool pg) const
+{
+    if (reducer_ || counting_ || profiling_ || pg || part_.nparts > 1 || any_periodic_) return 0;
+    if (natoms_ == 0 || max_sys_atoms_ > kMolAtoms || tab_.nid() > kMolSpecies) return 0;
+    const int cluster = mol_cluster_size(max_sys_atoms_);
+    if ((long long)nsys_ * cluster > 128 || !mol_cluster_fits(cluster)) return 0;
+    return cluster;
+}
+
+void Engine::run_molecules(const Batch& b_, const Species& s, const Damp& d, const Config& c, int cluster,
+                           const double* positions, double* energies, double* gradient, double* sigma9,
+                           cudaStream_t stream)
+{
+    const bool threebody = std::fabs(d.s9) >= DBL_EPSILON;
+    Batch b = b_;
+    b.sp = d_sp_;
+    b.ghost = d_ghost_;
+    b.local = d_local_;
+    b.zid = d_zid_;
+    b.perm = d_identity_;
+    b.tiles = nullptr;
+    MolArgs a;
+    a.b = b; a.s = s; a.d = d; a.c = c;
+    a.w = work_;
+    a.w.counts = nullptr;
+    a.two_body = two_body_active(d) ? 1 : 0;
+    a.pos = positions;
+    a.x = d_x_; a.y = d_y_; a.z = d_z_;
+    a.UV = pu_.U;
+    a.energies = energies; a.sigma9 = sigma9; a.grad_out = gradient;
+    if (threebody) {
+        ensure_atm_layout(stream);
+        if (!d_mol_fstore_) d_mol_fstore_ = dev_alloc<double>((size_t)kMolAtoms * natoms_);
+        a.v = atm_;
+        a.fstore = d_mol_fstore_;
+        a.fxf = d_fxf_; a.fxe = d_fxe_; a.queue = d_atm_queue_;
+    }
+    launch_mol_pairs(a, cluster, !threebody, stream);
+    if (threebody) {
+        species_ready_ = true;
+        run_three_body(b, s, d, c, a.w, stream, true);
+        launch_mol_finish(a, cluster, stream);
+    }
+    if (!capturing_) ev_recorded_ = false;
+    check(cudaGetLastError(), "kernel launch");
+}
+
 bool Engine::small_systems() const
 {
     return max_sys_atoms_ <= kDirectMaxAtoms && natoms_ <= kDirectMaxTotal;
@@ -786,6 +839,10 @@ void Engine::run(const Damp& d, const double* d_positions, double* d_energies, d
     c.cut_cn = cut_.cn; c.cut2 = cut_.disp2; c.cut3 = cut_.disp3;
     c.width2 = cut_.width2; c.width3 = cut_.width3;
     c.grad = grad; c.mixed = mixed_; c.param_grad = pg; c.cn_partitioned = cn_partitioned_;
+    if (const int cluster = molecule_cluster(d, pg)) {
+        run_molecules(b, s, d, c, cluster, d_positions, d_energies, d_gradient, d_sigma9, stream);
+        return;
+    }
     // the CN sweeps and the two-body sweep split the tile pairs each their own way
     pu_.split = pair_split();
     pu_.single_image = diagonal_walks();
@@ -1028,7 +1085,7 @@ bool Engine::atm_compact(bool mixed) const
 }
 
 void Engine::run_three_body(const Batch& b, const Species& s, const Damp& d, const Config& c, Work& w,
-                            cudaStream_t stream)
+                            cudaStream_t stream, bool prepared)
 {
     ensure_atm_layout(stream);
     // the two-body pass computed the species vectors; without it they are computed here
@@ -1036,8 +1093,10 @@ void Engine::run_three_body(const Batch& b, const Species& s, const Damp& d, con
     const bool compact = atm_compact(c.mixed);
     const size_t rec = atm_rec_bytes(c.mixed), aux = atm_block_bytes(c.mixed, true) - rec;
     AtmView v = atm_;
-    launch_atm_order(b, d_tile_off_, d_tile_sys_, ntiles_, v, compact ? d_spheres8_ : nullptr,
-                     c.grad ? d_fxf_ : nullptr, d_fxe_, d_atm_queue_, stream);
+    if (prepared) v.list = nullptr;
+    else
+        launch_atm_order(b, d_tile_off_, d_tile_sys_, ntiles_, v, compact ? d_spheres8_ : nullptr,
+                         c.grad ? d_fxf_ : nullptr, d_fxe_, d_atm_queue_, stream);
     long long blocks = v.ncand;
     if (compact) {
         if (v.ncand > atm_flag_cap_) {
@@ -1097,13 +1156,14 @@ void Engine::run_three_body(const Batch& b, const Species& s, const Damp& d, con
     const long long units = v.ncand * l.split;
     l.blocks = (int)std::max<long long>(1, std::min<long long>((long long)sms_ * occ, (units + atm_warps_per_block() - 1) / atm_warps_per_block()));
     launch_atm_pairs(b, s, c, w, v, pu_.U, l.alp3, guard, stream);
-    launch_atm_lists(v, ntiles8_, d_tile8_sys_, d_list_off_, d_atm_list_, d_atm_range_, guard, stream);
+    if (!prepared) launch_atm_lists(v, ntiles8_, d_tile8_sys_, d_list_off_, d_atm_list_, d_atm_range_, guard, stream);
     if (profiling_ && !capturing_) check(cudaEventRecord(kev_[2], stream), "cudaEventRecord");
     launch_atm_triples(l);
     if (profiling_ && !capturing_) {
         check(cudaEventRecord(kev_[3], stream), "cudaEventRecord");
         kev3_recorded_ = true;
     }
+    if (prepared) return;
     launch_atm_finish(b, c, v, ntiles8_, d.s9, d_fxf_, d_fxe_, d_atm_queue_, guard, w, d_e3_, d_sig3_, stream);
     w.e3_atom = d_e3_;
     w.sig3_atom = c.grad ? d_sig3_ : nullptr;
@@ -1357,6 +1417,16 @@ void Engine::evaluate_host(const Damp& d, const double* positions, double* energ
     double* hg = he + nsys_;
     double* hs = hg + 3 * (size_t)natoms_;
     std::memcpy(hin, positions, sizeof(double) * nin);
+    if (molecule_cluster(d, false)) {
+        // small molecules: the kernels read and write the pinned buffers (no copies),
+        // one or four launches that a captured sequence would not make cheaper
+        run(d, hin, he, grad ? hg : nullptr, grad ? hs : nullptr, nullptr, grad, stream_);
+        check(cudaStreamSynchronize(stream_), "evaluate");
+        std::memcpy(energies, he, sizeof(double) * nsys_);
+        if (gradient) std::memcpy(gradient, hg, sizeof(double) * 3 * natoms_);
+        if (sigma9) std::memcpy(sigma9, hs, sizeof(double) * 9 * nsys_);
+        return;
+    }
     check(cudaMemcpyAsync(d_pos_in_, hin, sizeof(double) * nin, cudaMemcpyHostToDevice, stream_), "positions");
     if (graph_on_) run_graphed(d, grad, false, stream_);
     else run(d, d_pos_in_, d_energies_, grad ? d_grad_out_ : nullptr, grad ? d_sigma_ : nullptr, nullptr, grad, stream_);

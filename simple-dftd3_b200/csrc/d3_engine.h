@@ -269,8 +269,14 @@ private:
     size_t h_stage_len_ = 0;
     unsigned long long* d_counts_ = nullptr;
     // three-body
+    // prepared: k_mol_pairs has ordered the tiles; launch_mol_finish takes the sums
     void run_three_body(const Batch& b, const Species& s, const Damp& d, const Config& c, Work& w,
-                        cudaStream_t stream);
+                        cudaStream_t stream, bool prepared = false);
+    int molecule_cluster(const Damp& d, bool pg) const;
+    void run_molecules(const Batch& b, const Species& s, const Damp& d, const Config& c, int cluster,
+                       const double* positions, double* energies, double* gradient, double* sigma9,
+                       cudaStream_t stream);
+    void* d_mol_fstore_ = nullptr;       // CN derivatives of small molecules' pairs
     void ensure_atm_layout(cudaStream_t stream);
     bool atm_compact(bool mixed) const;
     void free_block(void*& p);
