@@ -153,9 +153,18 @@ __device__ __forceinline__ D2 fma(D2 x, D2 y, D2 z) { return D2{::fma(x.a, y.a, 
 // tile indices) and translation index.
 struct BlockId { int sys, t8, A, B, t; };
 
-__device__ __forceinline__ BlockId block_id(const AtmView& v, long long c, int lane)
+// Largest a with a (a + 1) / 2 <= p.
+__device__ __forceinline__ int triangle_row(unsigned p)
 {
-    // 32-way search of the system (whole warp)
+    int a = (int)((sqrtf(8.0f * (float)p + 1.0f) - 1.0f) * 0.5f);
+    while ((unsigned)(a + 1) * (unsigned)(a + 2) / 2 <= p) a++;
+    while ((unsigned)a * (unsigned)(a + 1) / 2 > p) a--;
+    return a;
+}
+
+// System at candidate c: a 32-way search by the whole warp; returns its position.
+__device__ __forceinline__ int find_system(const AtmView& v, long long c, int lane)
+{
     int lo = 0, hi = v.nord;
     while (hi - lo > 1) {
         const int step = (hi - lo + 31) >> 5;
@@ -164,19 +173,44 @@ __device__ __forceinline__ BlockId block_id(const AtmView& v, long long c, int l
         lo += (__popc(ok) - 1) * step;
         hi = min(hi, lo + step);
     }
+    return lo;
+}
+
+__device__ __forceinline__ BlockId block_id(const AtmView& v, long long c, int lane)
+{
+    const int at = find_system(v, c, lane);
     BlockId id;
-    id.sys = v.ord[lo];
+    id.sys = v.ord[at];
     id.t8 = v.t8_off[id.sys];
-    const long long e = c - v.cand_off[lo];
+    const long long e = c - v.cand_off[at];
     const int nT = v.rep[4 * id.sys + 3];
     const unsigned p = (unsigned)(e / nT);
     id.t = (int)(e - (long long)p * nT);
-    int a = (int)((sqrtf(8.0f * (float)p + 1.0f) - 1.0f) * 0.5f);
-    while ((unsigned)(a + 1) * (unsigned)(a + 2) / 2 <= p) a++;
-    while ((unsigned)a * (unsigned)(a + 1) / 2 > p) a--;
-    id.A = a;
-    id.B = (int)(p - (unsigned)a * (unsigned)(a + 1) / 2);
+    id.A = triangle_row(p);
+    id.B = (int)(p - (unsigned)id.A * (unsigned)(id.A + 1) / 2);
     return id;
+}
+
+// Unit u of the triple kernel, in the order of their work: for every system first
+// the pairs of a tile with itself, whose roots are all tiles, then the others by
+// rising A, whose roots are the tiles above A.  Returns the candidate.
+__device__ __forceinline__ long long unit_id(const AtmView& v, long long u, int lane, BlockId& id)
+{
+    const int at = find_system(v, u, lane);
+    id.sys = v.ord[at];
+    id.t8 = v.t8_off[id.sys];
+    const int nt8 = v.t8_off[id.sys + 1] - id.t8, nT = v.rep[4 * id.sys + 3];
+    const long long base = v.cand_off[at];
+    const unsigned p = (unsigned)((u - base) / nT);
+    id.t = (int)((u - base) - (long long)p * nT);
+    if (p < (unsigned)nt8) {
+        id.A = id.B = (int)p;
+    } else {
+        const unsigned r = p - (unsigned)nt8;
+        id.A = triangle_row(r) + 1;
+        id.B = (int)(r - (unsigned)id.A * (unsigned)(id.A - 1) / 2);
+    }
+    return base + ((long long)id.A * (id.A + 1) / 2 + id.B) * nT + id.t;
 }
 
 // ------------------------------------------------------------- tile order --
@@ -547,11 +581,11 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
             if (u >= nunits) break;
             u_end = min(u + grab, nunits);
         }
-        const long long cand = (long long)(u / split);
+        BlockId id;
+        const long long cand = unit_id(v, (long long)(u / split), lane, id);
         const int piece = (int)(u % split);
         u++;
         if (v.mask[cand] == 0) continue;
-        const BlockId id = block_id(v, cand, lane);
         const int nT = PER ? v.rep[4 * id.sys + 3] : 1;
         const bool same = id.A == id.B;
         if (PER && same && 2 * id.t < nT - 1) continue;      // the other half space

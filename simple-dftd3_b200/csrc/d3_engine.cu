@@ -1152,7 +1152,7 @@ void Engine::run_three_body(const Batch& b, const Species& s, const Damp& d, con
     for (int sy = 0; sy < nsys_; sy++)
         most = std::max(most, (long long)(t8_off_[sy + 1] - t8_off_[sy]) * img_rep_[4 * (size_t)sy + 3]);
     l.split = (int)std::max<long long>(1, std::min(most, (2 * warps + v.ncand) / std::max<long long>(v.ncand, 1)));
-    l.grab = v.ncand > 256 * warps ? 8 : 1;
+    l.grab = v.ncand > 256 * warps ? 4 : 1;
     const long long units = v.ncand * l.split;
     l.blocks = (int)std::max<long long>(1, std::min<long long>((long long)sms_ * occ, (units + atm_warps_per_block() - 1) / atm_warps_per_block()));
     launch_atm_pairs(b, s, c, w, v, pu_.U, l.alp3, guard, stream);
