@@ -538,6 +538,14 @@ __device__ __forceinline__ void async_copy_value(V* dst, const V* src)
     }
 }
 
+// Columns of the pair p of a step: with gradients the lanes of a quarter take
+// different k, (j + p) mod 8 and k ^ 4, and the column sums travel with k; energies
+// have no column sums, so that all lanes take the same k, p and p + 4, and its records
+// are broadcast reads (141-atom slab 339 -> 299 us; with gradients the exchanges of
+// the column sums cost what the reads save: eight frames 51.2 against 52.5 ms).
+template <bool GRAD>
+__device__ __forceinline__ int column(int j, int p) { return GRAD ? (j + p) & 7 : p; }
+
 // What bounds it: dependent latencies and the issue of the work per four roots (22
 // of 47 instructions per step of 32 slots; FP32 2.2 instructions per cycle and SM;
 // FP64 1.6, the FP64 pipe at 46%).  A step of two partners (k and k ^ 4) is 39
@@ -616,15 +624,17 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
             oj = aj >= 0 ? b.local[aj] : 0;
             ok = ak >= 0 ? b.local[ak] : 0;
         }
-        // the (j, k) records of this lane; pair p: k = (j + p) mod 8 and k ^ 4.
-        // Half of the walk (diag): steps 1..3, and 4 in the lower lanes.
+        // the (j, k) records of this lane; pair p: k = column(j, p) and k ^ 4.  A tile
+        // with itself (diag): every unordered pair once.
         Pair zx[4], zu[4], zm[4], zp[4];
 #pragma unroll
         for (int p = 0; p < 4; p++) {
-            Rec r0 = rec[bjk * kRecs + kT8 * j + ((j + p) & 7)], r1 = rec[bjk * kRecs + kT8 * j + ((j + p + 4) & 7)];
+            const int k0 = column<GRAD>(j, p);
+            Rec r0 = rec[bjk * kRecs + kT8 * j + k0], r1 = rec[bjk * kRecs + kT8 * j + (k0 ^ 4)];
             if (diag) {
-                if (p == 0) { r0.z = R(0); if (GEN) r0.y = R(0); }
-                if (p > 0 || j >= 4) { r1.z = R(0); if (GEN) r1.y = R(0); }
+                // the rotated walk takes steps 1..3, and 4 in the lower lanes
+                if (GRAD ? p == 0 : k0 >= j) { r0.z = R(0); if (GEN) r0.y = R(0); }
+                if (GRAD ? p > 0 || j >= 4 : k0 + 4 >= j) { r1.z = R(0); if (GEN) r1.y = R(0); }
             }
             zx[p] = pk(r0.x, r1.x); zu[p] = pk(r0.y, r1.y); zm[p] = pk(r0.z, r1.z); zp[p] = pk(r0.w, r1.w);
         }
@@ -755,7 +765,7 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
                 Pair rK = pk(R(0), R(0)), rV = rK, rE = rK, kS = rK, kE = rK;
 #pragma unroll
                 for (int p = 0; p < 4; p++) {
-                    const int kl = qbase | ((j + p) & 7);
+                    const int kl = qbase | column<GRAD>(j, p);
                     Pair y, yu, ym, yp;
                     if constexpr (sizeof(R) == 4) {
                         const float4 b0 = sh.xu[kl], b1 = sh.mp[kl];
