@@ -216,7 +216,19 @@ __global__ void __launch_bounds__(kPwThreads) k_pairwise3(Batch b, Species s, Da
     eg[lq * n + lp] = sum;
 }
 
+__global__ void k_copy_out(const double* __restrict__ src, double* __restrict__ dst, long long n)
+{
+    pdl_wait();
+    const long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (k < n) dst[k] = src[k];
+}
+
 }  // namespace
+
+void launch_copy_out(const double* src, double* dst, long long n, cudaStream_t stream)
+{
+    if (n > 0) launch_pdl(k_copy_out, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, stream, src, dst, n);
+}
 
 void launch_pairwise(const Batch& b, const Species& s, const Damp& d, const Config& c, const Work& w,
                      const long long* off, long long total, bool molecules, double* c6, double* factors, double* e2,
