@@ -45,7 +45,8 @@ sys.path.insert(0, str(ROOT / "simple-dftd3_b200"))
 L2_FLUSH_BYTES = 256 << 20     # larger than the 126 MB L2
 # algorithmic flops per unit of work (FMA = 2); fixed between the two forms
 FLOPS_PER_PAIR = 65            # two-body BJ term with gradient, virial and dE/dCN
-FLOPS_PER_TRIPLE = 220         # ATM term with gradient, virial and dE/dCN
+FLOPS_PER_TRIPLE = 220         # ATM term with gradient, virial and dE/dCN in the reference's form (the pair form
+                               # of k_atm_triples spends about 110)
 METRIC = "pair-terms/s, D3(BJ) two-body E+grad+virial (mixed FP32/FP64, <=1e-7 rel. E error)"
 # DRAM bytes (read + write) of one k_two_body_tt<float, rational> launch on cell2000, from
 # an ncu capture of that launch
@@ -630,7 +631,7 @@ def run_ours(args, rank, world, dist):
     # the dominant kernel alone, timed with CUDA events around its launch
     stage = "three_body_kernel" if atm else "two_body_kernel"
     flops = FLOPS_PER_TRIPLE if atm else FLOPS_PER_PAIR
-    kern = "k_triples" if atm else "k_two_body_tt"
+    kern = "k_atm_triples" if atm else "k_two_body_tt"
     line = {
         "metric": METRIC if args.workload == "cell2000" else f"{unit} ({args.workload})",
         "value": (1 if shard else world) * units / (ms * 1e-3),
@@ -683,12 +684,10 @@ def run_ours(args, rank, world, dist):
                 continue
             entry["roofline_mixed"] = roofline(entry["work"]["triple_terms"], FLOPS_PER_TRIPLE,
                                                entry["mixed"]["stage_ms"]["three_body_kernel"], peak32,
-                                               "k_triples_mol<float>" if name == "batch4096" else "k_triples<float>",
-                                               "fp32")
+                                               "k_atm_triples<float>", "fp32")
             entry["roofline_fp64"] = roofline(entry["work"]["triple_terms"], FLOPS_PER_TRIPLE,
                                               entry["fp64"]["stage_ms"]["three_body_kernel"], peak64,
-                                              "k_triples_mol<double>" if name == "batch4096" else "k_triples<double>",
-                                              "fp64")
+                                              "k_atm_triples<double>", "fp64")
     if want_cpu:
         if args.workload in ("cell2000", "cluster5000", "batch4096", "frames256"):
             if args.workload == "frames256":

@@ -25,13 +25,14 @@
 // common translation) is visited once.  A unit is a pair block (J, K, T) whose
 // third atoms, the roots, run over the tiles I > J and their images; for J = K
 // (T in one half space, T = 0 as half of the walk) over all tiles, and then the
-// triples inside one tile index are met three times and weighted by 1/3.  One
-// (k_atm_lists: the tile images in reach of J.)  One warp takes a unit: four quarters of eight lanes hold four roots, the lane one
-// atom j, its eight (j, k) records and their sums D, W in registers, and the
-// quarter walks k = (j + t) mod 8; the sums of (i, k) move one lane down per step
-// with k.  Roots without a partner in J or K inside the cutoff are dropped
-// before (8-bit masks of the blocks).  Per four roots D and W of (i, j) and
-// (i, k) become forces; every 128 roots the (j, k) sums do.
+// triples inside one tile index are met three times and weighted by 1/3
+// (k_atm_lists: the tile images in reach of J).  One warp takes a unit: four
+// quarters of eight lanes hold four roots, the lane one atom j, its eight (j, k)
+// records and their sums D, W in registers, and the quarter walks
+// k = (j + t) mod 8; the sums of (i, k) move one lane down per step with k.  Roots
+// without a partner in J or K inside the cutoff are dropped before (8-bit masks of
+// the blocks).  Per four roots D and W of (i, j) and (i, k) become forces; every
+// 128 roots the (j, k) sums do.
 //
 // All sums over units go to fixed-point accumulators (integer additions), so the
 // results do not depend on the order of the warps and repeat bit for bit.
@@ -59,7 +60,8 @@ constexpr int kRootChunk = 128;         // roots between two flushes: FP32 sums 
 // 168 registers and 12 warps beat 128 registers (spills) and 16 warps, 54.8
 // against 59.1 ms on eight frames; FP64 with gradient: 254 registers and 8 warps
 // beat 168 and 12 (cluster of 5000 atoms 15.5 against 17.7 ms); energies: 16 and
-// 12 warps beat 20 and 16 (slab 0.63 against 0.74 ms).
+// 12 warps beat 20 and 16 (slab 0.63 against 0.74 ms, before its pair sweeps were
+// cut into more items).
 template <class R, bool GRAD>
 constexpr int kTripleBlocks = sizeof(R) == 4 ? (GRAD ? 3 : 4) : (GRAD ? 2 : 3);
 
@@ -546,18 +548,21 @@ __device__ __forceinline__ void async_copy_value(V* dst, const V* src)
 template <bool GRAD>
 __device__ __forceinline__ int column(int j, int p) { return GRAD ? (j + p) & 7 : p; }
 
-// What bounds it: dependent latencies and the issue of the work per four roots (22
-// of 47 instructions per step of 32 slots; FP32 2.2 instructions per cycle and SM;
-// FP64 1.6, the FP64 pipe at 46%).  A step of two partners (k and k ^ 4) is 39
-// packed FP32 instructions, two reciprocals, four shuffles and two 16-byte shared
-// loads; the (j, k) records and sums stay in registers.  One partner at a time and
+// What bounds it: the data pipe of L1 and shared memory (74% busy in FP32, 86% in
+// FP64: the (i, k) records of a step, staged roots, shuffles of the column sums),
+// with 12 or 8 warps per SM to hide its latency and that of the FMA chains (2.2 and
+// 1.7 instructions per cycle and SM; FMA pipe 44%, FP64 pipe 51%).  A step of two
+// partners (k and k ^ 4) is 39 packed FP32 instructions, two reciprocals, four
+// shuffles and two 16-byte shared loads; the (j, k) records and sums stay in
+// registers.  One partner at a time and
 // plain FP32 instructions (62 per step) took 67.8 instead of 54.8 ms on eight
-// frames and, in FP64, 16.7 instead of 15.3 ms on the cluster.  Whole evaluations
-// with the neighbour-list and block-per-molecule kernels that this one replaced
-// (185 instructions per slot, exp, log and divisions per triple in FP64) against
-// now: cluster of 5000 atoms (FP64) 54.0 -> 15.3 ms, 512 molecules (FP64) 21.4 ->
-// 2.1 ms, 4096 molecules (mixed) 13.9 -> 7.6 ms, eight periodic frames (mixed) 149
-// -> 54.8 ms, one molecule of 100 atoms 216 -> 85 us, slab energy 2.6 -> 0.63 ms.
+// frames and, in FP64, 16.7 instead of 15.3 ms on the cluster (both before the unit
+// order).  Whole evaluations with the neighbour-list and block-per-molecule kernels
+// that this one replaced (185 instructions per slot, exp, log and divisions per
+// triple in FP64) against now: cluster of 5000 atoms (FP64) 54.4 -> 15.1 ms, 512
+// molecules (FP64) 21.2 -> 2.1 ms, 4096 molecules (mixed) 13.6 -> 5.8 ms, eight
+// periodic frames (mixed) 163 -> 51 ms, one molecule of 100 atoms 220 -> 67 us, slab
+// energy 2.8 -> 0.31 ms.
 // GEN: work partition and term counting (the owner test of every triple).
 template <class R, bool GRAD, bool PER, bool GEN>
 __global__ void __launch_bounds__(32 * kAtmWarps, kTripleBlocks<R, GRAD>)
