@@ -935,15 +935,20 @@ k_cn_chain_rot(Batch b, Work w, const int2* units, int nunits, const R* store, c
 // l / VI, l / VI + 32 / VI, ...) and value l % VJ of its j slots, VI and VJ
 // the powers of two >= KI and KJ, so that a warp load reads a few contiguous
 // slot rows; the i slots of an atom are the items of the units (tl, jt <= tl),
-// consecutive, its j slots those of the units (it >= tl, tl).  The j total of
+// consecutive, its j slots those of the units (it >= tl, tl), of whose items only
+// those of the atom's own part of the j tile hold more than zeros.  The j total of
 // value m is added to i value JOFF + m; lanes 0 .. KI - 1 return the totals.
+// Bound by the latency of the slot loads: rows of zeros left out, and two of the
+// fifteen values read for energies, took a 300-atom cell (split 16 and 32) from 158 to
+// 151 us and a 141-atom slab energy from 301 to 297 us.  The kernels are held to 32
+// registers: at 40, and three quarters of the warps, the gathers of 4096 molecules
+// took 80 us more.
 template <int KI, int KJ, int JOFF, int SJ = kUnitJ>
 __device__ __forceinline__ double tt_gather_atom(long long base, int tl, int nt, int sl, int split,
                                                  const double* unit_i, const double* unit_j, int lane)
 {
     constexpr int VI = KI <= 1 ? 1 : KI <= 2 ? 2 : KI <= 4 ? 4 : KI <= 8 ? 8 : 16;
     constexpr int VJ = KJ <= 1 ? 1 : KJ <= 2 ? 2 : KJ <= 4 ? 4 : 8;
-    const int sh = __ffs(split) - 1;   // log2 of the split
     double si = 0.0, sj = 0.0;
     if (lane % VI < KI) {
         const long long i0 = (base + (long long)tl * (tl + 1) / 2) * split;
@@ -955,12 +960,15 @@ __device__ __forceinline__ double tt_gather_atom(long long base, int tl, int nt,
 #pragma unroll
     for (int o = VI; o < 32; o <<= 1) si += __shfl_xor_sync(0xffffffffu, si, o);
     if (lane % VJ < KJ) {
-        const int nj = (nt - tl) * split;
+        const int sh = split == 4 ? 1 : 0;                     // two translation parts, or one
+        const int lj = __ffs(split) - 1 - sh;                  // log2 of the parts of the j tile
+        const int nj = (nt - tl) << sh;
+        const double* p = unit_j + ((((base + tl) * split + (sl >> (5 - lj))) * kTile) + sl) * SJ + lane % VJ;
 #pragma unroll 8
         for (int q = lane / VJ; q < nj; q += 32 / VJ) {
-            const int it = tl + (q >> sh);
-            const long long item = (base + (long long)it * (it + 1) / 2 + tl) * split + (q & (split - 1));
-            sj += unit_j[(item * kTile + sl) * SJ + lane % VJ];
+            const unsigned it = tl + (q >> sh);
+            const unsigned row = (it * (it + 1) / 2 << (lj + sh)) + ((q & sh) << lj);
+            sj += p[(size_t)row * (kTile * SJ)];
         }
     }
 #pragma unroll
@@ -971,9 +979,10 @@ __device__ __forceinline__ double tt_gather_atom(long long base, int tl, int nt,
     return si;
 }
 
-// Per-atom sums of the two-body unit slots: energy, dE/dCN, gradient,
-// virial and parameter derivatives (lanes 0 .. 14 of tt_gather_atom).
-__global__ void k_unit_gather(Batch b, Config c, const int* unit_base, int split, const double* unit_i,
+// Per-atom sums of the two-body unit slots: energy and dE/dCN, or (FULL) these,
+// gradient, virial and parameter derivatives (lanes 0 .. 14 of tt_gather_atom).
+template <bool FULL>
+__global__ void __launch_bounds__(256, 8) k_unit_gather(Batch b, Config c, const int* unit_base, int split, const double* unit_i,
                               const double* unit_j, Work w)
 {
     pdl_wait();
@@ -985,9 +994,11 @@ __global__ void k_unit_gather(Batch b, Config c, const int* unit_base, int split
     const int t0 = b.tile_off[sys], t1 = b.tile_off[sys + 1];
     const int tl = (a - as) / kTile;              // tile of a, local to the system
     const int sl = (a - as) % kTile;              // slot lane
-    const double v = tt_gather_atom<kUnitI, kUnitJ, 1>(unit_base[sys], tl, t1 - t0, sl, split, unit_i, unit_j, lane);
+    const double v = tt_gather_atom<FULL ? kUnitI : 2, FULL ? kUnitJ : 1, 1>(unit_base[sys], tl, t1 - t0, sl, split,
+                                                                            unit_i, unit_j, lane);
     if (lane == 0) w.e_atom[a] = v;
     else if (lane == 1) { if (w.dEdcn) w.dEdcn[a] = v; }
+    else if (!FULL) return;
     else if (lane < 5) { if (c.grad) w.grad[3 * a + lane - 2] = v; }
     else if (lane < 5 + kSigma) { if (c.grad) w.sig_atom[kSigma * a + lane - 5] = v; }
     else if (lane < kUnitI) { if (c.param_grad && w.pg_atom) w.pg_atom[kParamGrad * a + lane - 11] = v; }
@@ -1318,7 +1329,7 @@ k_cn_chain_stored(Batch b, Config c, Partition p, Work w, const int2* units, int
 // of the stored-sum passes, with the atom's S sums (CN) and its chain-rule
 // virial dE/dCN_i S_i (chain rule).
 template <bool CHAIN, bool STORED>
-__global__ void k_cn_gather(Batch b, const int* unit_base, int split, const double* unit_i, const double* unit_j,
+__global__ void __launch_bounds__(256, 8) k_cn_gather(Batch b, const int* unit_base, int split, const double* unit_i, const double* unit_j,
                             Work w)
 {
     pdl_wait();
@@ -1580,7 +1591,9 @@ void launch_two_body_units(const Batch& b, const Species& s, const Damp& d, cons
         }
     }
     if (ev_end) cudaEventRecord(ev_end, stream);
-    launch_pdl(k_unit_gather, dim3((b.natoms + 7) / 8), dim3(256), 0, stream, b, c, pu.unit_base, pu.split, pu.unit_i, pu.unit_j, w);
+    const auto gather = c.grad || c.param_grad ? k_unit_gather<true> : k_unit_gather<false>;
+    launch_pdl(gather, dim3((b.natoms + 7) / 8), dim3(256), 0, stream, b, c, pu.unit_base, pu.split, pu.unit_i, pu.unit_j,
+               w);
 }
 
 }  // namespace d3

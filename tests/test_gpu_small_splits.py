@@ -58,3 +58,24 @@ def test_few_tile_pairs_parameter_derivatives(natoms, precision, etol):
     assert abs(e.item() - ref["energy"]) <= etol * abs(ref["energy"])
     gtol = GTOL64 * np.abs(ref["gradient"]).max() if precision == "fp64" else 1e-7
     assert np.abs(x.grad.cpu().numpy() - ref["gradient"]).max() <= gtol
+
+
+@pytest.mark.parametrize("split", [0, 1, 2, 4])
+@pytest.mark.parametrize("natoms", [1, 33, 200])
+def test_slot_sums_energy_only(natoms, split):
+    """Energies of a pass without derivatives, whose gather reads two values per slot,
+    against the pass with them (1e-14 of the energy: the same sums), for every way the
+    tile pairs are cut."""
+    from dftd3 import library as lib, synthetic as S
+    from dftd3.interface import BatchedDispersion, ModifiedZeroDampingParam
+    rng = np.random.default_rng(natoms)
+    edge = (natoms / 0.02) ** (1 / 3) + 2.0
+    num = rng.choice([1, 6, 7, 8], size=natoms).astype(np.int32)
+    pos = S.pack_cell(rng, natoms, edge * np.eye(3), 2.0)
+    keys = ("s6", "s8", "rs6", "rs8", "bet", "alp", "s9")
+    param = ModifiedZeroDampingParam(**{k: MZERO[k] for k in keys})
+    model = BatchedDispersion([num], [pos], edge * np.eye(3)[None], np.ones((1, 3), dtype=bool))
+    lib.set_batch_tuning(model._batch, 0.0, split, 0)
+    full = model.get_dispersion(param, grad=True)["energy"]
+    only = model.get_dispersion(param, grad=False)["energy"]
+    assert np.abs(np.asarray(only) - np.asarray(full)).max() <= 1e-14 * np.abs(full).max()
