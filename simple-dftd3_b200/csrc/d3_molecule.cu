@@ -42,6 +42,12 @@ constexpr int kMolSteps = kMolAtoms / 32;            // partners of a lane
 constexpr double kKcnMol = 16.0;                     // ncoord.f90:31
 static_assert(kMolCluster <= 16, "cluster size");
 
+// The two halves of a cluster barrier.  A block's shared memory may be touched by the
+// others only once the block has started, which nothing but a barrier of the cluster
+// tells: a kernel arrives at its entry and waits before its first remote store.
+__device__ __forceinline__ void mol_cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void mol_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
 __device__ __forceinline__ double mol_wsum(double v)
 {
 #pragma unroll
@@ -125,6 +131,7 @@ __device__ __forceinline__ void mol_chain(const MolShared& sh, const R (&fk)[kMo
 template <class R, int DAMP, bool GRAD, bool LAST>
 __global__ void __launch_bounds__(kMolThreads, 1) k_mol_pairs(MolArgs a)
 {
+    mol_cluster_arrive();
     pdl_wait();
     __shared__ MolShared sh;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -137,14 +144,13 @@ __global__ void __launch_bounds__(kMolThreads, 1) k_mol_pairs(MolArgs a)
     const int a0 = b.atom_off[sys], n = b.atom_off[sys + 1] - a0;
     R* sv = sgw + kMolAtoms * kMaxRef + (size_t)wid * b.nid * 2 * kMaxRef;   // [nid][V 7, dV 7]
     // the block's atoms to every block of the cluster
-    if (tid < 3 * kMolWarps) {
-        const int k = 3 * kMolWarps * rank + tid;
-        if (k < 3 * n) {
-            const double v = a.pos[3 * (size_t)a0 + k];
-            for (int r = 0; r < nranks; r++) cluster.map_shared_rank(&sh.pos[k], r)[0] = v;
-        }
-    }
+    const int kpos = 3 * kMolWarps * rank + tid;
+    const bool has_pos = tid < 3 * kMolWarps && kpos < 3 * n;
+    const double vpos = has_pos ? a.pos[3 * (size_t)a0 + kpos] : 0.0;
     for (int k = tid; k < n; k += kMolThreads) sh.sp[k] = b.sp[a0 + k];
+    mol_cluster_wait();
+    if (has_pos)
+        for (int r = 0; r < nranks; r++) cluster.map_shared_rank(&sh.pos[kpos], r)[0] = vpos;
     cluster.sync();
 
     const int i = kMolWarps * rank + wid;
