@@ -231,6 +231,14 @@ __device__ __forceinline__ int longest_axis(double x, double y, double z, bool m
     return ex >= ey && ex >= ez ? 0 : ey >= ez ? 1 : 2;
 }
 
+// The coordinate as an integer of the same order, NaN at the ends: ranks by it are a
+// permutation for any input, so that every slot of a tile is written.
+__device__ __forceinline__ long long order_bits(double c)
+{
+    const long long u = __double_as_longlong(c);
+    return u ^ ((u >> 63) & 0x7fffffffffffffffLL);
+}
+
 // Compact tiles of 8 atoms inside each 32-atom tile (one warp each): the atoms
 // are ordered along the longest axis of their box and cut into tiles of 8, above
 // 16 atoms into two halves that are ordered along their own longest axis (fill
@@ -252,10 +260,10 @@ __global__ void k_atm_order(Batch b, const int* tile_off, const int* tile_sys, i
     const int a = a0 + (in ? lane : 0);
     const double x = b.x[a], y = b.y[a], z = b.z[a];
     auto rank_in = [&](int axis, int group) {
-        const double c = axis == 0 ? x : axis == 1 ? y : z;
+        const long long c = order_bits(axis == 0 ? x : axis == 1 ? y : z);
         int r = 0;
         for (int k = 0; k < n; k++) {
-            const double ck = __shfl_sync(0xffffffffu, c, k);
+            const long long ck = __shfl_sync(0xffffffffu, c, k);
             const int gk = __shfl_sync(0xffffffffu, group, k);
             r += gk == group && (ck < c || (ck == c && k < lane));
         }
