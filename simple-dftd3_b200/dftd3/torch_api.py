@@ -82,6 +82,10 @@ class D3Batch:
 
     def strained(self, positions: torch.Tensor, strain: Optional[torch.Tensor]):
         """Strained positions and host lattices for a (nsys, 3, 3) strain."""
+        # the evaluation reads one row per atom: any other shape is refused here
+        if positions.dim() != 2:
+            raise ValueError("Positions must have the shape (natoms, 3)")
+        positions = positions.expand(len(self._sys_index), 3)
         if strain is None:
             return positions, self.lattices
         idx = self.sys_index(positions.device)
@@ -100,7 +104,7 @@ class D3Batch:
 
 def _evaluate(model: D3Batch, positions, params, strain, derivatives: bool, param_derivatives: bool):
     pos, lat = model.strained(positions.detach(), None if strain is None else strain.detach())
-    pos = pos.contiguous()
+    pos = pos.to(torch.float64).contiguous()     # the kernels read doubles
     nsys = len(model)
     dev = positions.device
     energies = torch.zeros(nsys, dtype=torch.float64, device=dev)
