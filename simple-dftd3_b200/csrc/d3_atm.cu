@@ -76,31 +76,12 @@ __device__ __forceinline__ double norm2(double x, double y, double z)
     return __fma_rn(z, z, __fma_rn(y, y, __dmul_rn(x, x)));
 }
 
-// Deterministic accumulation of sums from many warps: a value is added as two
-// 64-bit integers, its multiple of 2^-32 (floor) and the rest rounded to units
-// of 2^-72, so that the total does not depend on the order of the additions.
-// Range +-2^31 per addition; the rest word takes up to 2^23 additions (each
-// below 2^40 + 1) before it could overflow.
-__device__ __forceinline__ void fixed_split(double v, long long& hi, long long& lo)
-{
-    const double sv = v * 4294967296.0;                 // 2^32
-    const double h = floor(sv);
-    hi = (long long)h;
-    lo = __double2ll_rn((sv - h) * 1099511627776.0);    // 2^40
-}
-
 __device__ __forceinline__ void fixed_add(unsigned long long* acc2, double v)
 {
     long long hi, lo;
     fixed_split(v, hi, lo);
     atomicAdd(acc2, (unsigned long long)hi);
     atomicAdd(acc2 + 1, (unsigned long long)lo);
-}
-
-__device__ __forceinline__ double fixed_value(const unsigned long long* acc2)
-{
-    return double((long long)acc2[0]) * 2.3283064365386963e-10 +      // 2^-32
-           double((long long)acc2[1]) * 2.117582368135751e-22;        // 2^-72
 }
 
 // Two values worked on together: the packed FP32 instructions of sm_100 (one

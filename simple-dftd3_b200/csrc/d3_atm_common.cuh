@@ -1,5 +1,6 @@
 // Smooth cutoff and triple ownership of the three-body kernels (d3_atm.cu) and
-// of the pairwise decomposition (d3_pairwise.cu).
+// of the pairwise decomposition (d3_pairwise.cu), and the fixed-point sums of the
+// former (read by d3_molecule.cu as well).
 #pragma once
 
 #include <cfloat>
@@ -28,6 +29,27 @@ __device__ __forceinline__ bool owns_pair_atm(const Partition& p, int i, int j)
 {
     long long hi = i > j ? i : j, lo = i > j ? j : i;
     return (hi * (hi + 1) / 2 + lo) % p.nparts == p.part;
+}
+
+// Deterministic accumulation of sums from many warps: a value is added as two
+// 64-bit integers, its nearest multiple of 2^-40 and the rest rounded to units of
+// 2^-72, so that the total does not depend on the order of the additions.  The rest
+// is at most 2^31 units either way: its word takes 2^32 additions before it could
+// overflow.  An atom of a cell of one atom with N neighbours gets about N^2 / 4 of
+// them (fcc Cu: 2.6e6 at a three-body cutoff of 40 Bohr, 3.0e7 at 60, 2^32 at 135),
+// an atom of a larger cell fewer.  Sums reach to +-2^23.
+__device__ __forceinline__ void fixed_split(double v, long long& hi, long long& lo)
+{
+    const double sv = v * 1099511627776.0;              // 2^40
+    const double h = rint(sv);
+    hi = (long long)h;
+    lo = __double2ll_rn((sv - h) * 4294967296.0);       // 2^32
+}
+
+__device__ __forceinline__ double fixed_value(const unsigned long long* acc2)
+{
+    return double((long long)acc2[0]) * 9.094947017729282e-13 +       // 2^-40
+           double((long long)acc2[1]) * 2.117582368135751e-22;        // 2^-72
 }
 
 }  // namespace

@@ -24,6 +24,7 @@
 #include <mutex>
 #include <set>
 
+#include "d3_atm_common.cuh"
 #include "d3_damping.cuh"
 #include "d3_device.cuh"
 #include "d3_math.cuh"
@@ -53,12 +54,6 @@ __device__ __forceinline__ double mol_wsum(double v)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
-}
-
-// The two 64-bit words of d3_atm.cu's fixed-point sums (units of 2^-32 and 2^-72).
-__device__ __forceinline__ double mol_fixed(const unsigned long long* f)
-{
-    return double((long long)f[0]) * 2.3283064365386963e-10 + double((long long)f[1]) * 2.117582368135751e-22;
 }
 
 // Dynamic part of k_mol_pairs: the reference weights of every atom, and of every
@@ -359,14 +354,14 @@ __global__ void __launch_bounds__(kMolThreads, 1) k_mol_finish(MolArgs a)
     if (GRAD)
         for (int k = tid; k < n; k += kMolThreads) {
             sh.pos[3 * k] = a.x[a0 + k]; sh.pos[3 * k + 1] = a.y[a0 + k]; sh.pos[3 * k + 2] = a.z[a0 + k];
-            sh.de[k] = a.w.dEdcn[a0 + k] + s9 * mol_fixed(a.fxf + (size_t)8 * (a0 + k) + 6);
+            sh.de[k] = a.w.dEdcn[a0 + k] + s9 * fixed_value(a.fxf + (size_t)8 * (a0 + k) + 6);
         }
     cluster.sync();
     const int i = kMolWarps * rank + wid;
     double v[7] = {0, 0, 0, 0, 0, 0, 0};
     if (i < n) {
         v[0] = a.w.e_atom[a0 + i];
-        if (i % kMolSlots == 0) v[0] += s9 * mol_fixed(a.fxe + (size_t)20 * (a.v.t8_off[sys] + i / kMolSlots));
+        if (i % kMolSlots == 0) v[0] += s9 * fixed_value(a.fxe + (size_t)20 * (a.v.t8_off[sys] + i / kMolSlots));
         if (GRAD) {
             R fk[kMolSteps];
             const R* fs = (const R*)a.fstore + (size_t)(a0 + i) * kMolAtoms;
@@ -377,7 +372,7 @@ __global__ void __launch_bounds__(kMolThreads, 1) k_mol_finish(MolArgs a)
             gx = mol_wsum(gx); gy = mol_wsum(gy); gz = mol_wsum(gz);
             for (int k = 0; k < kSigma; k++) sg[k] = mol_wsum(sg[k]);
             const unsigned long long* f = a.fxf + (size_t)8 * (a0 + i);
-            const double tx = 2.0 * s9 * mol_fixed(f), ty = 2.0 * s9 * mol_fixed(f + 2), tz = 2.0 * s9 * mol_fixed(f + 4);
+            const double tx = 2.0 * s9 * fixed_value(f), ty = 2.0 * s9 * fixed_value(f + 2), tz = 2.0 * s9 * fixed_value(f + 4);
             // the three-body virial is sum F_a (x) x_a, the origin being free
             const double x = sh.pos[3 * i] - sh.pos[0], y = sh.pos[3 * i + 1] - sh.pos[1], z = sh.pos[3 * i + 2] - sh.pos[2];
             const double t3[kSigma] = {tx * x, ty * y, tz * z, 0.5 * (tx * y + ty * x), 0.5 * (tx * z + tz * x),
