@@ -47,8 +47,8 @@ __device__ __forceinline__ void tt_family(R r2, R r1, bool have_r1, R rrij, R q1
         const R ir2 = inv<R>(r2);
         const R ir6 = ir2 * ir2 * ir2;
         const R x6 = inv<R>(r1 * q1 + q3), x8 = inv<R>(r1 * q2 + q3);
-        const R t6 = h6 >= 0 ? ipow(x6 * x6, h6) : tt_pow<R>(x6, alp6);
-        const R t8 = h6 >= 0 ? ipow(x8 * x8, h6 + 1) : tt_pow<R>(x8, alp8);
+        const R t6 = damping_power(h6 >= 0 ? ipow(x6 * x6, h6) : tt_pow<R>(x6, alp6));
+        const R t8 = damping_power(h6 >= 0 ? ipow(x8 * x8, h6 + 1) : tt_pow<R>(x8, alp8));
         const R f6 = inv<R>(R(1) + R(6) * t6);
         const R f8 = inv<R>(R(1) + R(6) * t8);
         const R d6 = R(-6) * f6 * ir2 + R(6) * alp6 * t6 * (f6 * f6) * inv<R>(r2 + q4 * r1);
@@ -59,7 +59,7 @@ __device__ __forceinline__ void tt_family(R r2, R r1, bool have_r1, R rrij, R q1
     } else if constexpr (DAMP == kOptimizedPower) {
         // t6 = r^b / (r^b r^6 + q1) = 1 / (r^6 + q1 r^-b)
         const R ir2 = inv<R>(r2);
-        const R ib = hb >= 0 ? ipow(ir2, hb) : tt_pow<R>(r2, R(-0.5) * bet);
+        const R ib = damping_power(hb >= 0 ? ipow(ir2, hb) : tt_pow<R>(r2, R(-0.5) * bet));
         const R r4 = r2 * r2;
         const R t6 = inv<R>(r4 * r2 + q1 * ib);
         const R t8 = inv<R>(r4 * r4 + q2 * ib);

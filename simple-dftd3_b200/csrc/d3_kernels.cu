@@ -443,6 +443,7 @@ __global__ void __launch_bounds__(kThreads) k_two_body(Batch b, Species s, Damp 
                         t6 = rpow<R>(q1 / r1, alp6);
                         t8 = rpow<R>(q2 / r1, alp8);
                     }
+                    t6 = damping_power(t6); t8 = damping_power(t8);
                     const R f6 = inv<R>(R(1) + R(6) * t6);
                     const R f8 = inv<R>(R(1) + R(6) * t8);
                     const R d6 = ir2 * f6 * (R(-6) + R(6) * alp6 * t6 * f6);

@@ -1,11 +1,14 @@
 // Reciprocals, reciprocal square roots and even powers of the pair terms.
 //
-// FP64: the hardware approximation (relative error e0 below 2^-20) with one step
-// of the series of (1 - e)^-1 or (1 - e)^-1/2 in the residual e, cut after e^2
-// (error e0^3, below the rounding): 4 and 6 instructions without branches, in
-// place of the library's division and square root with their special cases.  The
-// arguments are squared distances and sums of positive terms: positive, normal
-// and far from the ends of the range.  Measured (B200, FP64): the CN sweep of a
+// FP64: the hardware approximation y (relative error e0 below 2^-20) and one
+// third-order Householder step: with the residual e = 1 - x y (1 - x y^2) the result
+// is y (1 - e)^-1 (y (1 - e)^-1/2), its binomial series cut after e^2, error of order
+// e0^3 = 2^-60, below the rounding.  4 and 6 instructions without branches, in
+// place of the library's division and square root with their special cases; within
+// one and two units in the last place for normal arguments whose result is normal.
+// An infinite argument gives NaN: the callers' arguments are squared distances and
+// sums of positive terms far from the ends of the range, and the powers of the
+// damping functions, which are not, are bounded first (damping_power).  Measured (B200, FP64): the CN sweep of a
 // periodic 2000-atom cell 161 -> 108 us (two divisions and a square root less per
 // term), its rational two-body sweep 232 -> 210 us, the optimized power sweep of a
 // 141-atom slab 247 -> 114 us (no pow).
@@ -65,5 +68,11 @@ __device__ __forceinline__ R ipow(R x, int h)
     }
     return y;
 }
+
+// A damping power t = (R0/r)^alp (r^-bet), bounded so that 1 + 6 t, 6 alp t (R0^(bet + 8) t) stay finite for any
+// exponent and distance (the rejected terms of a sweep take r = 1, where a large alp
+// overflows first): the damping 1 / (1 + 6 t) has vanished long before.
+template <class R>
+__device__ __forceinline__ R damping_power(R t) { if constexpr (sizeof(R) == 8) return fmin(t, 1e150); else return fminf(t, 1e30f); }
 
 }  // namespace d3

@@ -265,6 +265,7 @@ __global__ void __launch_bounds__(kMolThreads, 1) k_mol_pairs(MolArgs a)
                     t6 = tt_pow<R>(q1 / r1, alp6);
                     t8 = tt_pow<R>(q2 / r1, alp8);
                 }
+                t6 = damping_power(t6); t8 = damping_power(t8);
                 const R f6 = inv<R>(R(1) + R(6) * t6), f8 = inv<R>(R(1) + R(6) * t8);
                 const R w6 = s6 * ir6, w8 = s8 * rrij * (ir6 * ir2);
                 ed = w6 * f6 + w8 * f8;

@@ -439,6 +439,7 @@ k_two_body_tt(Batch b, Species s, Damp d, Config c, Partition p, Work w, const i
                         t6 = tt_pow<R>(q1 / r1, alp6);
                         t8 = tt_pow<R>(q2 / r1, alp8);
                     }
+                    t6 = damping_power(t6); t8 = damping_power(t8);
                     const R f6 = inv<R>(R(1) + R(6) * t6);
                     const R f8 = inv<R>(R(1) + R(6) * t8);
                     const R d6 = ir2 * f6 * (R(-6) + R(6) * alp6 * t6 * f6);
@@ -696,6 +697,7 @@ k_two_body_rot(Batch b, Species s, Damp d, Config c, Work w, const int2* units, 
                     t6 = tt_pow<R>(q1 / r1, alp6);
                     t8 = tt_pow<R>(q2 / r1, alp8);
                 }
+                t6 = damping_power(t6); t8 = damping_power(t8);
                 const R f6 = inv<R>(R(1) + R(6) * t6);
                 const R f8 = inv<R>(R(1) + R(6) * t8);
                 const R d6 = ir2 * f6 * (R(-6) + R(6) * alp6 * t6 * f6);
