@@ -45,6 +45,7 @@
 #include "d3_atm_common.cuh"
 #include "d3_device.cuh"
 #include "d3_math.cuh"
+#include "d3_per_device.h"
 
 namespace d3 {
 
@@ -997,14 +998,17 @@ __global__ void k_atm_finish(Batch b, Config c, AtmView v, int ntiles8, double s
 template <class R, bool GRAD, bool PER, bool GEN>
 int atm_configure()
 {
-    static const int blocks = [] {
+    // an error here stays the last one, which the engine checks after its launches
+    static PerDevice<int> blocks;
+    int device = 0;
+    cudaGetDevice(&device);
+    const auto kernel = k_atm_triples<R, GRAD, PER, GEN>;
+    const int n = blocks.get(device, (const void*)kernel, [&](int& n) {
         const int smem = (int)sizeof(AtmShared<R>) * kAtmWarps;
-        cudaFuncSetAttribute(k_atm_triples<R, GRAD, PER, GEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        int n = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_atm_triples<R, GRAD, PER, GEN>, 32 * kAtmWarps, smem);
-        return n > 0 ? n : 1;
-    }();
-    return blocks;
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
+               cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, 32 * kAtmWarps, smem) == cudaSuccess && n > 0;
+    });
+    return n > 0 ? n : 1;
 }
 
 template <class R, bool GRAD, bool PER>

@@ -21,13 +21,12 @@
 
 #include <cfloat>
 #include <cstdint>
-#include <mutex>
-#include <set>
 
 #include "d3_atm_common.cuh"
 #include "d3_damping.cuh"
 #include "d3_device.cuh"
 #include "d3_math.cuh"
+#include "d3_per_device.h"
 #include "d3_weights.cuh"
 
 namespace d3 {
@@ -389,17 +388,21 @@ __global__ void __launch_bounds__(kMolThreads, 1) k_mol_finish(MolArgs a)
 
 using MolKernel = void (*)(MolArgs);
 
-// Clusters above eight blocks need a kernel's consent, given once.
-void mol_consent(MolKernel kernel)
+// Clusters above eight blocks need a kernel's consent, given once on each device.
+bool mol_consent(MolKernel kernel)
 {
-    static std::mutex lock;
-    static std::set<MolKernel> done;
-    std::lock_guard<std::mutex> guard(lock);
-    if (done.insert(kernel).second) cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    static PerDevice<bool> consent;
+    int device = 0;
+    cudaGetDevice(&device);
+    return consent.get(device, (const void*)kernel, [&](bool& ok) {
+        ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+        return ok;
+    });
 }
 
 void mol_launch(MolKernel kernel, const MolArgs& a, int cluster, size_t smem, cudaStream_t stream)
 {
+    // without consent the launch fails, and the engine reports its error
     if (cluster > 8) mol_consent(kernel);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(a.b.nsys * cluster);
@@ -450,9 +453,11 @@ int mol_cluster_size(int max_atoms)
 bool mol_cluster_fits(int cluster)
 {
     if (cluster <= 8) return true;
-    static const bool fits = [] {
-        const MolKernel kernel = k_mol_pairs<double, kRational, true, true>;
-        mol_consent(kernel);
+    static PerDevice<bool> fits;
+    int device = 0;
+    cudaGetDevice(&device);
+    const MolKernel kernel = k_mol_pairs<double, kRational, true, true>;
+    const bool ok = fits.get(device, (const void*)kernel, [&](bool& ok) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(kMolCluster);
         cfg.blockDim = dim3(kMolThreads);
@@ -465,9 +470,11 @@ bool mol_cluster_fits(int cluster)
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         int n = 0;
-        return cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0;
-    }();
-    return fits;
+        ok = mol_consent(kernel) && cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0;
+        return ok;
+    });
+    if (!ok) (void)cudaGetLastError();        // the staged kernels serve these systems
+    return ok;
 }
 
 void launch_mol_pairs(const MolArgs& a, int cluster, bool last, cudaStream_t stream)
