@@ -1055,8 +1055,8 @@ int atm_blocks_per_sm(bool mixed, bool grad, bool periodic, bool gen)
 size_t atm_scan_temp_bytes(long long n)
 {
     size_t bytes = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, bytes, (const int*)nullptr, (int*)nullptr, (int)(n + 1));
-    return bytes;
+    const cudaError_t e = cub::DeviceScan::ExclusiveSum(nullptr, bytes, (const int*)nullptr, (int*)nullptr, n + 1);
+    return e == cudaSuccess ? bytes : 0;
 }
 
 void launch_atm_order(const Batch& b, const int* tile_off, const int* tile_sys, int ntiles, const AtmView& v,
@@ -1068,12 +1068,13 @@ void launch_atm_order(const Batch& b, const int* tile_off, const int* tile_sys, 
                fxe, queue);
 }
 
-void launch_atm_mark(const Batch& b, const Config& c, const AtmView& v, const double4* spheres, int* flag, int* map,
-                     void* temp, size_t temp_bytes, cudaStream_t stream)
+cudaError_t launch_atm_mark(const Batch& b, const Config& c, const AtmView& v, const double4* spheres, int* flag, int* map,
+                            void* temp, size_t temp_bytes, cudaStream_t stream)
 {
-    cudaMemsetAsync(flag + v.ncand, 0, sizeof(int), stream);
+    const cudaError_t e = cudaMemsetAsync(flag + v.ncand, 0, sizeof(int), stream);
+    if (e != cudaSuccess) return e;
     k_atm_mark<<<(unsigned)((v.ncand + 127) / 128), 128, 0, stream>>>(b, c, v, spheres, flag);
-    cub::DeviceScan::ExclusiveSum(temp, temp_bytes, flag, map, (int)(v.ncand + 1), stream);
+    return cub::DeviceScan::ExclusiveSum(temp, temp_bytes, flag, map, v.ncand + 1, stream);
 }
 
 void launch_atm_guard(const int* total, long long cap, int* guard, cudaStream_t stream)

@@ -335,14 +335,14 @@ size_t atm_block_bytes(bool mixed, bool grad);   // records and CN derivatives o
 size_t atm_rec_bytes(bool mixed);                // the records alone
 int atm_warps_per_block();
 int atm_blocks_per_sm(bool mixed, bool grad, bool periodic, bool gen);
-size_t atm_scan_temp_bytes(long long ncand);
+size_t atm_scan_temp_bytes(long long ncand);      // 0: the scan refuses the size
 // Tile order; clears the accumulators and the queue.  spheres: [ntiles8] or null.
 void launch_atm_order(const Batch& b, const int* tile_off, const int* tile_sys, int ntiles, const AtmView& v,
                       double4* spheres, unsigned long long* fxf, unsigned long long* fxe, unsigned long long* queue,
                       cudaStream_t stream);
 // Candidates in reach of the cutoff and their block numbers: map[ncand] is the total.
-void launch_atm_mark(const Batch& b, const Config& c, const AtmView& v, const double4* spheres, int* flag, int* map,
-                     void* temp, size_t temp_bytes, cudaStream_t stream);
+cudaError_t launch_atm_mark(const Batch& b, const Config& c, const AtmView& v, const double4* spheres, int* flag, int* map,
+                            void* temp, size_t temp_bytes, cudaStream_t stream);
 // Sets *guard when the total exceeds cap; the kernels below then return at once.
 void launch_atm_guard(const int* total, long long cap, int* guard, cudaStream_t stream);
 void launch_atm_pairs(const Batch& b, const Species& s, const Config& c, const Work& w, const AtmView& v, const void* U,

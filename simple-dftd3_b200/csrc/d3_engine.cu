@@ -1140,9 +1140,11 @@ void Engine::run_three_body(const Batch& b, const Species& s, const Damp& d, con
             d_atm_flag_ = dev_alloc<int>(atm_flag_cap_ + 1);
             d_atm_map_ = dev_alloc<int>(atm_flag_cap_ + 1);
             scan_bytes_ = atm_scan_temp_bytes(atm_flag_cap_);
+            if (scan_bytes_ == 0) throw Error("The system is too large for the three-body term");
             d_scan_temp_ = dev_alloc<unsigned char>(scan_bytes_);
         }
-        launch_atm_mark(b, c, v, d_spheres8_, d_atm_flag_, d_atm_map_, d_scan_temp_, scan_bytes_, stream);
+        check(launch_atm_mark(b, c, v, d_spheres8_, d_atm_flag_, d_atm_map_, d_scan_temp_, scan_bytes_, stream),
+              "block numbers");
         v.map = d_atm_map_;
         if (!capturing_) {
             check(cudaMemcpyAsync(h_atm_total_, d_atm_map_ + v.ncand, sizeof(int), cudaMemcpyDeviceToHost, stream), "total");
