@@ -87,9 +87,13 @@ dftd3_b200_get_dispersion_batched(dftd3_error /* error */,
  * Evaluations are asynchronous with respect to the host, except with the
  * three-body term when its pair blocks of all tile pairs and translations
  * exceed 1 GiB (3 KiB each, 1.5 KiB in the mixed form): then only those in
- * reach of the cutoff are kept and the call waits for the device once, for
- * their number (ordinary sequence) or for the capacity check at the end
- * (captured sequence, dftd3_b200_set_batch_graph). */
+ * reach of the cutoff are kept and the call waits for the device, for their
+ * number (ordinary sequence; once for every group of systems with 2^24 tile
+ * pairs and translations, whose blocks are held together) or for the capacity
+ * check at the end (captured sequence, dftd3_b200_set_batch_graph).
+ * The three-body term of one system is refused above 524272 atoms, 2^26 tile
+ * pairs (8 x 8 atoms, with their translations) within the cutoff or 2^33 of
+ * them in all; the number of systems has no limit but memory. */
 SDFTD3_API_ENTRY void SDFTD3_API_CALL
 dftd3_b200_get_dispersion_device(dftd3_error /* error */,
                                  dftd3_b200_batch /* batch */,

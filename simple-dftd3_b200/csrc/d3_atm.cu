@@ -17,7 +17,8 @@
 // Tiles and blocks.  Every 32-atom tile of the spatial order is cut into compact
 // tiles of 8 atoms (k_atm_order).  A block holds the 64 records of a tile pair
 // (A, B <= A) for one lattice translation (k_atm_pairs; batches whose blocks
-// exceed kAtmDenseCap keep only those whose spheres are in reach, k_atm_mark).
+// exceed kAtmDenseCap keep only those whose spheres are in reach, k_atm_mark, and
+// above kAtmGroupCands candidates take groups of systems one after the other).
 // Tiles of 8 fill 0.6 of their triple slots with accepted triples on periodic
 // frames (cutoff 40 Bohr), tiles of 16 0.44 and of 32 0.30 (CPU replay).
 //
@@ -333,7 +334,10 @@ __global__ void k_atm_mark(Batch b, Config c, AtmView v, const double4* spheres,
     flag[cand] = norm2(sb.x + T[0] - sa.x, sb.y + T[1] - sa.y, sb.z + T[2] - sa.z) <= reach * reach ? 1 : 0;
 }
 
-__global__ void k_atm_guard(const int* total, long long cap, int* guard) { *guard = *total > cap ? 1 : 0; }
+__global__ void k_atm_guard(const int* total, long long cap, int* guard, bool first)
+{
+    *guard = *total > cap || (!first && *guard) ? 1 : 0;
+}
 
 // The 64 records {x, u, m, P} of a block and, with gradients, {dlnC6/dCN_a / 2,
 // dlnC6/dCN_b / 2} of (row atom a of A, column atom b of B + T): one warp per
@@ -445,14 +449,15 @@ k_atm_pairs(Batch b, Species s, Config c, Work w, AtmView v, const R* UV, double
 // Root tiles of every tile J, ascending: the tile images (I, T_I) whose block
 // with J has a pair inside the cutoff, {block, mask of the roots << 24 | I, T_I,
 // candidate}.  One warp per tile; gt[J] is the first entry with I > J.
-__global__ void k_atm_lists(AtmView v, int ntiles8, const int* tile8_sys, const long long* list_off, int4* list,
-                            int2* range, const int* guard)
+__global__ void k_atm_lists(AtmView v, int ntiles8, const int* tile8_sys, const int* sys_group, int group,
+                            const long long* list_off, int4* list, int2* range, const int* guard)
 {
     pdl_wait();
     const int lane = threadIdx.x & 31;
     const int tile = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (tile >= ntiles8 || (guard && *guard)) return;
     const int sys = tile8_sys[tile];
+    if (sys_group && sys_group[sys] != group) return;
     const int t8 = v.t8_off[sys], nt8 = v.t8_off[sys + 1] - t8, J = tile - t8;
     const int nT = v.rep[4 * sys + 3];
     const long long cbase = v.cand_off_sys[sys];
@@ -1077,9 +1082,9 @@ cudaError_t launch_atm_mark(const Batch& b, const Config& c, const AtmView& v, c
     return cub::DeviceScan::ExclusiveSum(temp, temp_bytes, flag, map, v.ncand + 1, stream);
 }
 
-void launch_atm_guard(const int* total, long long cap, int* guard, cudaStream_t stream)
+void launch_atm_guard(const int* total, long long cap, int* guard, bool first, cudaStream_t stream)
 {
-    k_atm_guard<<<1, 1, 0, stream>>>(total, cap, guard);
+    k_atm_guard<<<1, 1, 0, stream>>>(total, cap, guard, first);
 }
 
 void launch_atm_pairs(const Batch& b, const Species& s, const Config& c, const Work& w, const AtmView& v, const void* U,
@@ -1091,12 +1096,12 @@ void launch_atm_pairs(const Batch& b, const Species& s, const Config& c, const W
     else launch_pdl(k_atm_pairs<double>, dim3(blocks), dim3(256), 0, stream, b, s, c, w, v, (const double*)U, alp3, guard);
 }
 
-void launch_atm_lists(const AtmView& v, int ntiles8, const int* tile8_sys, const long long* list_off, int4* list,
-                      int2* range, const int* guard, cudaStream_t stream)
+void launch_atm_lists(const AtmView& v, int ntiles8, const int* tile8_sys, const int* sys_group, int group,
+                      const long long* list_off, int4* list, int2* range, const int* guard, cudaStream_t stream)
 {
     if (ntiles8 <= 0) return;
-    launch_pdl(k_atm_lists, dim3((ntiles8 + 3) / 4), dim3(128), 0, stream, v, ntiles8, tile8_sys, list_off, list, range,
-               guard);
+    launch_pdl(k_atm_lists, dim3((ntiles8 + 3) / 4), dim3(128), 0, stream, v, ntiles8, tile8_sys, sys_group, group,
+               list_off, list, range, guard);
 }
 
 void launch_atm_triples(const AtmLaunch& l)

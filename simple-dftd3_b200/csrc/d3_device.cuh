@@ -294,9 +294,10 @@ void launch_two_body_units(const Batch& b, const Species& s, const Damp& d, cons
 // Three-body term (d3_atm.cu).  Tiles of 8 atoms and candidate blocks: the
 // systems in processing order (largest first) have, for every tile pair
 // (A, B <= A) and every three-body lattice translation, one candidate block of
-// 64 pair records.
+// 64 pair records.  Large batches are taken in groups of systems, one view each:
+// cand_off, cand_off_sys and list_off count from the start of the group.
 struct AtmView {
-    int nord = 0;                          // systems
+    int nord = 0;                          // systems of the group
     long long ncand = 0;                   // candidate blocks
     const long long* cand_off = nullptr;   // [nord] first candidate of each system, in processing order
     const int* ord = nullptr;              // [nord] system at each processing position
@@ -343,12 +344,14 @@ void launch_atm_order(const Batch& b, const int* tile_off, const int* tile_sys, 
 // Candidates in reach of the cutoff and their block numbers: map[ncand] is the total.
 cudaError_t launch_atm_mark(const Batch& b, const Config& c, const AtmView& v, const double4* spheres, int* flag, int* map,
                             void* temp, size_t temp_bytes, cudaStream_t stream);
-// Sets *guard when the total exceeds cap; the kernels below then return at once.
-void launch_atm_guard(const int* total, long long cap, int* guard, cudaStream_t stream);
+// Sets *guard when the total exceeds cap, or leaves an earlier group's (not first); the
+// kernels below then return at once.
+void launch_atm_guard(const int* total, long long cap, int* guard, bool first, cudaStream_t stream);
 void launch_atm_pairs(const Batch& b, const Species& s, const Config& c, const Work& w, const AtmView& v, const void* U,
                       double alp3, const int* guard, cudaStream_t stream);
-void launch_atm_lists(const AtmView& v, int ntiles8, const int* tile8_sys, const long long* list_off, int4* list,
-                      int2* range, const int* guard, cudaStream_t stream);
+// sys_group: [nsys] group of each system, or null (one group)
+void launch_atm_lists(const AtmView& v, int ntiles8, const int* tile8_sys, const int* sys_group, int group,
+                      const long long* list_off, int4* list, int2* range, const int* guard, cudaStream_t stream);
 void launch_atm_triples(const AtmLaunch& l);
 // Small molecules (d3_molecule.cu): systems of one lattice point and at most
 // kMolAtoms atoms, in input order, one cluster of blocks per system.

@@ -1031,6 +1031,7 @@ void Engine::ensure_atm_layout(cudaStream_t stream)
         d_cand_off_ = dev_alloc<long long>(nsys_);
         d_cand_off_sys_ = dev_alloc<long long>(nsys_);
         d_list_off_ = dev_alloc<long long>(nsys_);
+        d_atm_group_ = dev_alloc<int>(nsys_);
         d_pos8_ = dev_alloc<double4>(8 * n8);
         d_tile8_sys_ = dev_alloc<int>(n8);
         d_atm_range_ = dev_alloc<int2>(n8);
@@ -1063,15 +1064,28 @@ void Engine::ensure_atm_layout(cudaStream_t stream)
     std::iota(ord.begin(), ord.end(), 0);
     std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return sys_natoms_[a] > sys_natoms_[b]; });
     std::vector<long long> off(nsys_), off_sys(nsys_), list_off(nsys_);
-    long long total = 0, entries = 0;
+    std::vector<int> group_of(nsys_);
+    std::vector<AtmGroup> groups;
+    long long most_cand = 0, most_entries = 0, all = 0;
     for (int k = 0; k < nsys_; k++) {
-        const long long nt = t8_off_[ord[k] + 1] - t8_off_[ord[k]], nT = img_rep_[4 * (size_t)ord[k] + 3];
-        off[k] = off_sys[ord[k]] = total;
-        list_off[ord[k]] = entries;
-        total += nt * (nt + 1) / 2 * nT;
-        entries += nt * nt * nT;
+        const int sy = ord[k];
+        const long long nt = t8_off_[sy + 1] - t8_off_[sy], nT = img_rep_[4 * (size_t)sy + 3];
+        const long long cand = nt * (nt + 1) / 2 * nT;
+        // tile pairs of a system are numbered with 32 bits, the candidates by blocks of eight
+        if (nt > 65534 || cand > (1LL << 33)) throw Error("The system is too large for the three-body term");
+        if (groups.empty() || groups.back().ncand + cand > kAtmGroupCands) groups.push_back({k, 0, 0, 0, 1});
+        AtmGroup& g = groups.back();
+        off[k] = off_sys[sy] = g.ncand;
+        list_off[sy] = g.entries;
+        group_of[sy] = (int)groups.size() - 1;
+        g.count++;
+        g.ncand += cand;
+        g.entries += nt * nt * nT;
+        g.most = std::max(g.most, nt * nT);
+        most_cand = std::max(most_cand, g.ncand);
+        most_entries = std::max(most_entries, g.entries);
+        all += cand;
     }
-    if (total > 0x7ffffff0LL) throw Error("The system is too large for the three-body term");
     check(cudaMemcpyAsync(d_atm_ord_, ord.data(), sizeof(int) * nsys_, cudaMemcpyHostToDevice, stream), "order");
     check(cudaMemcpyAsync(d_cand_off_, off.data(), sizeof(long long) * nsys_, cudaMemcpyHostToDevice, stream),
           "candidates");
@@ -1081,24 +1095,28 @@ void Engine::ensure_atm_layout(cudaStream_t stream)
           "root lists");
     check(cudaMemcpyAsync(d_atm_rep_, img_rep_.data(), sizeof(int) * 4 * nsys_, cudaMemcpyHostToDevice, stream),
           "translations");
-    if (total > atm_cand_cap_) {
+    check(cudaMemcpyAsync(d_atm_group_, group_of.data(), sizeof(int) * nsys_, cudaMemcpyHostToDevice, stream), "groups");
+    // room for other lattices, not where it would take gigabytes
+    auto padded = [](long long n) { return n + std::min(n / 4, kAtmGroupCands) + 16; };
+    if (most_cand > atm_cand_cap_) {
         void* p = d_atm_mask_;
         free_block(p);
-        atm_cand_cap_ = total + total / 4 + 16;
+        atm_cand_cap_ = padded(most_cand);
         d_atm_mask_ = dev_alloc<unsigned short>(atm_cand_cap_);
     }
-    if (entries > atm_list_cap_) {
+    if (most_entries > atm_list_cap_) {
         void* p = d_atm_list_;
         free_block(p);
-        atm_list_cap_ = entries + entries / 4 + 16;
+        atm_list_cap_ = padded(most_entries);
         d_atm_list_ = dev_alloc<int4>(atm_list_cap_);
     }
     // the host vectors go out of scope: make the copies complete first
     check(cudaStreamSynchronize(stream), "three-body layout");
     atm_.nord = nsys_;
-    // kernel arguments of a captured sequence: a new number of candidates needs a new capture
-    if (total != atm_.ncand) graph_valid_ = false;
-    atm_.ncand = total;
+    // kernel arguments of a captured sequence: other numbers of candidates need a new capture
+    if (!(groups == atm_groups_)) graph_valid_ = false;
+    atm_groups_ = std::move(groups);
+    atm_.ncand = all;
     atm_.cand_off = d_cand_off_;
     atm_.cand_off_sys = d_cand_off_sys_;
     atm_.pos = d_pos8_;
@@ -1124,13 +1142,32 @@ void Engine::run_three_body(const Batch& b, const Species& s, const Damp& d, con
     ensure_atm_layout(stream);
     // the two-body pass computed the species vectors; without it they are computed here
     if (!species_ready_) launch_species_vectors(b, s, c, w, pu_.U, stream);
+    AtmView v = atm_;
+    if (!prepared)
+        launch_atm_order(b, d_tile_off_, d_tile_sys_, ntiles_, v, atm_compact(c.mixed) ? d_spheres8_ : nullptr,
+                         c.grad ? d_fxf_ : nullptr, d_fxe_, d_atm_queue_, stream);
+    for (const AtmGroup& g : atm_groups_) run_three_body_group(g, b, s, d, c, w, stream, prepared);
+    if (prepared) return;
+    launch_atm_finish(b, c, v, ntiles8_, d.s9, d_fxf_, d_fxe_, d_atm_queue_, atm_compact(c.mixed) ? d_guard_ : nullptr, w,
+                      d_e3_, d_sig3_, stream);
+    w.e3_atom = d_e3_;
+    w.sig3_atom = c.grad ? d_sig3_ : nullptr;
+}
+
+// Blocks and triples of one group of systems, in buffers that the groups share.
+void Engine::run_three_body_group(const AtmGroup& g, const Batch& b, const Species& s, const Damp& d, const Config& c,
+                                  const Work& w, cudaStream_t stream, bool prepared)
+{
+    const bool first = &g == &atm_groups_.front(), last = &g == &atm_groups_.back();
     const bool compact = atm_compact(c.mixed);
     const size_t rec = atm_rec_bytes(c.mixed), aux = atm_block_bytes(c.mixed, true) - rec;
     AtmView v = atm_;
+    v.nord = g.count;
+    v.ncand = g.ncand;
+    v.cand_off += g.first;
+    v.ord += g.first;
     if (prepared) v.list = nullptr;
-    else
-        launch_atm_order(b, d_tile_off_, d_tile_sys_, ntiles_, v, compact ? d_spheres8_ : nullptr,
-                         c.grad ? d_fxf_ : nullptr, d_fxe_, d_atm_queue_, stream);
+    if (!first) check(cudaMemsetAsync(d_atm_queue_, 0, sizeof(unsigned long long), stream), "queue");
     long long blocks = v.ncand;
     if (compact) {
         if (v.ncand > atm_flag_cap_) {
@@ -1168,7 +1205,7 @@ void Engine::run_three_body(const Batch& b, const Species& s, const Damp& d, con
     if (compact) {
         size_t cap = atm_rec_cap_ / rec;
         if (c.grad) cap = std::min(cap, atm_aux_cap_ / aux);
-        launch_atm_guard(d_atm_map_ + v.ncand, (long long)cap, d_guard_, stream);
+        launch_atm_guard(d_atm_map_ + v.ncand, (long long)cap, d_guard_, first, stream);
         guard = d_guard_;
     }
     v.rec = d_atm_rec_;
@@ -1184,25 +1221,20 @@ void Engine::run_three_body(const Batch& b, const Species& s, const Damp& d, con
     if (tune_.atm_blocks_per_sm > 0) occ = std::min(occ, tune_.atm_blocks_per_sm);
     const long long warps = (long long)sms_ * occ * atm_warps_per_block();
     // few units: several warps share the roots of one
-    long long most = 1;
-    for (int sy = 0; sy < nsys_; sy++)
-        most = std::max(most, (long long)(t8_off_[sy + 1] - t8_off_[sy]) * img_rep_[4 * (size_t)sy + 3]);
-    l.split = (int)std::max<long long>(1, std::min(most, (2 * warps + v.ncand) / std::max<long long>(v.ncand, 1)));
+    l.split = (int)std::max<long long>(1, std::min(g.most, (2 * warps + v.ncand) / std::max<long long>(v.ncand, 1)));
     l.grab = v.ncand > 256 * warps ? 4 : 1;
     const long long units = v.ncand * l.split;
     l.blocks = (int)std::max<long long>(1, std::min<long long>((long long)sms_ * occ, (units + atm_warps_per_block() - 1) / atm_warps_per_block()));
     launch_atm_pairs(b, s, c, w, v, pu_.U, l.alp3, guard, stream);
-    if (!prepared) launch_atm_lists(v, ntiles8_, d_tile8_sys_, d_list_off_, d_atm_list_, d_atm_range_, guard, stream);
-    if (profiling_ && !capturing_) check(cudaEventRecord(kev_[2], stream), "cudaEventRecord");
+    if (!prepared)
+        launch_atm_lists(v, ntiles8_, d_tile8_sys_, atm_groups_.size() > 1 ? d_atm_group_ : nullptr,
+                         int(&g - atm_groups_.data()), d_list_off_, d_atm_list_, d_atm_range_, guard, stream);
+    if (profiling_ && !capturing_ && first) check(cudaEventRecord(kev_[2], stream), "cudaEventRecord");
     launch_atm_triples(l);
-    if (profiling_ && !capturing_) {
+    if (profiling_ && !capturing_ && last) {
         check(cudaEventRecord(kev_[3], stream), "cudaEventRecord");
         kev3_recorded_ = true;
     }
-    if (prepared) return;
-    launch_atm_finish(b, c, v, ntiles8_, d.s9, d_fxf_, d_fxe_, d_atm_queue_, guard, w, d_e3_, d_sig3_, stream);
-    w.e3_atom = d_e3_;
-    w.sig3_atom = c.grad ? d_sig3_ : nullptr;
 }
 
 void Engine::stage_times(double out[kTimes])

@@ -290,6 +290,23 @@ private:
     void free_block(void*& p);
     // blocks above this size are kept for the tile pairs in reach only
     static constexpr size_t kAtmDenseCap = size_t(1) << 30;
+    // Systems of a batch whose blocks are held at a time: consecutive ones in processing
+    // order with at most this many candidates (a larger system alone).  A candidate has 42
+    // bytes of scratch, a kept block 1.5 or 3 KiB: 0.7 GB and, with a quarter in reach as
+    // on periodic frames, 6 or 13 GB; the triples of a full group take a third of a second.
+    static constexpr long long kAtmGroupCands = 1LL << 24;
+    struct AtmGroup {
+        int first, count;                // processing positions
+        long long ncand, entries;        // candidate blocks, root list entries
+        long long most;                  // largest number of tile images of a system
+        bool operator==(const AtmGroup& o) const
+        {
+            return first == o.first && count == o.count && ncand == o.ncand && entries == o.entries && most == o.most;
+        }
+    };
+    std::vector<AtmGroup> atm_groups_;
+    void run_three_body_group(const AtmGroup& g, const Batch& b, const Species& s, const Damp& d, const Config& c,
+                              const Work& w, cudaStream_t stream, bool prepared);
     std::vector<long long> c6mat_off_;   // dense [n_s][n_s] blocks of the pairwise decomposition
     long long c6mat_total_ = 0;
     int ntiles8_ = 0;
@@ -298,6 +315,7 @@ private:
     bool atm_layout_valid_ = false;
     AtmView atm_;
     long long *d_cand_off_ = nullptr, *d_cand_off_sys_ = nullptr, *d_list_off_ = nullptr;
+    int* d_atm_group_ = nullptr;
     double4* d_pos8_ = nullptr;
     int* d_tile8_sys_ = nullptr;
     int4* d_atm_list_ = nullptr;
