@@ -15,8 +15,9 @@ namespace {
 
 void check(cudaError_t e, const char* what)
 {
-    if (e != cudaSuccess)
-        throw Error(std::string("CUDA error in ") + what + ": " + cudaGetErrorString(e));
+    if (e == cudaSuccess) return;
+    (void)cudaGetLastError();      // reported here, not by the next call's launches as well
+    throw Error(std::string("CUDA error in ") + what + ": " + cudaGetErrorString(e));
 }
 
 void cross(const double* a, const double* b, double* c)
@@ -183,6 +184,19 @@ T* Engine::dev_alloc(size_t n)
     allocations_.push_back(p);
     alloc_epoch_++;   // captured graphs hold device pointers
     return static_cast<T*>(p);
+}
+
+// A buffer of n entries in place of p.  cap is what p holds, also when the allocation
+// fails: the engine stays usable, and a later call allocates again.
+template <class T, class C>
+void Engine::regrow(T*& p, C& cap, size_t n)
+{
+    void* old = p;
+    p = nullptr;
+    cap = 0;
+    free_block(old);
+    p = dev_alloc<T>(n);
+    cap = (C)n;
 }
 
 Engine::Engine(int nsys, const int* natoms, const int* numbers, const double* lattices,
@@ -442,15 +456,8 @@ void Engine::ensure_images(cudaStream_t stream)
         off[k * (nsys_ + 1) + nsys_] = (int)(all.size() / 3);
     }
     if (all.size() > img_capacity_) {
-        if (d_img_) {
-            check(cudaStreamSynchronize(stream), "images sync");
-            auto it = std::find(allocations_.begin(), allocations_.end(), (void*)d_img_);
-            if (it != allocations_.end()) allocations_.erase(it);
-            check(cudaFree(d_img_), "cudaFree");
-            alloc_epoch_++;
-        }
-        img_capacity_ = all.size() + all.size() / 4 + 3;
-        d_img_ = dev_alloc<double>(img_capacity_);
+        check(cudaStreamSynchronize(stream), "images sync");
+        regrow(d_img_, img_capacity_, all.size() + all.size() / 4 + 3);
     }
     check(cudaMemcpyAsync(d_img_, all.data(), sizeof(double) * all.size(), cudaMemcpyHostToDevice, stream), "images");
     check(cudaMemcpyAsync(d_img_off_, off.data(), sizeof(int) * off.size(), cudaMemcpyHostToDevice, stream), "img_off");
@@ -653,7 +660,7 @@ void Engine::pairwise_host(const Damp& d, const double* positions, double* energ
     ensure_workspace(false, false, false);
     upload_pair_table(d, stream);
     const long long total = std::max<long long>(c6mat_total_, 1);
-    if (!d_pw_) {
+    if (!d_pw_off_) {
         d_pw_ = dev_alloc<double>(5 * (size_t)total);
         d_pw_off_ = dev_alloc<long long>(nsys_);
         check(cudaMemcpy(d_pw_off_, c6mat_off_.data(), sizeof(long long) * nsys_, cudaMemcpyHostToDevice),
@@ -755,7 +762,7 @@ void Engine::hessian_host(const Damp& d, const double* positions, double* hessia
     upload_pair_table(d, stream);
     const int n = natoms_;
     const size_t nh = 9 * (size_t)n * n;
-    if (!d_hs_) {
+    if (!d_rvdw_) {
         d_hs_ = dev_alloc<double>(hessian_scratch_doubles(n) + nh);
         const int nid = tab_.nid();
         d_rvdw_ = dev_alloc<double>((size_t)nid * nid);
@@ -890,12 +897,9 @@ void Engine::run(const Damp& d, const double* d_positions, double* d_energies, d
         const size_t bytes = cn_store_bytes(pcn, mixed_);
         if (bytes <= kCnStoreCap && (bytes <= cn_store_cap_ || !capturing_)) {
             if (bytes > cn_store_cap_) {
-                free_block(d_cn_store_);
-                void* ok = d_cn_store_ok_;
-                free_block(ok);
-                d_cn_store_ = dev_alloc<unsigned char>(bytes);
-                d_cn_store_ok_ = dev_alloc<unsigned char>((size_t)pu_.nunits * max_split_);
-                cn_store_cap_ = bytes;
+                cn_store_cap_ = 0;
+                if (!d_cn_store_ok_) d_cn_store_ok_ = dev_alloc<unsigned char>((size_t)pu_.nunits * max_split_);
+                regrow(d_cn_store_, cn_store_cap_, bytes);
             }
             pcn.cn_store = d_cn_store_;
             pcn.cn_store_ok = d_cn_store_ok_;
@@ -1098,18 +1102,8 @@ void Engine::ensure_atm_layout(cudaStream_t stream)
     check(cudaMemcpyAsync(d_atm_group_, group_of.data(), sizeof(int) * nsys_, cudaMemcpyHostToDevice, stream), "groups");
     // room for other lattices, not where it would take gigabytes
     auto padded = [](long long n) { return n + std::min(n / 4, kAtmGroupCands) + 16; };
-    if (most_cand > atm_cand_cap_) {
-        void* p = d_atm_mask_;
-        free_block(p);
-        atm_cand_cap_ = padded(most_cand);
-        d_atm_mask_ = dev_alloc<unsigned short>(atm_cand_cap_);
-    }
-    if (most_entries > atm_list_cap_) {
-        void* p = d_atm_list_;
-        free_block(p);
-        atm_list_cap_ = padded(most_entries);
-        d_atm_list_ = dev_alloc<int4>(atm_list_cap_);
-    }
+    if (most_cand > atm_cand_cap_) regrow(d_atm_mask_, atm_cand_cap_, padded(most_cand));
+    if (most_entries > atm_list_cap_) regrow(d_atm_list_, atm_list_cap_, padded(most_entries));
     // the host vectors go out of scope: make the copies complete first
     check(cudaStreamSynchronize(stream), "three-body layout");
     atm_.nord = nsys_;
@@ -1171,14 +1165,15 @@ void Engine::run_three_body_group(const AtmGroup& g, const Batch& b, const Speci
     long long blocks = v.ncand;
     if (compact) {
         if (v.ncand > atm_flag_cap_) {
-            void *pf = d_atm_flag_, *pm = d_atm_map_;
-            free_block(pf); free_block(pm); free_block(d_scan_temp_);
-            atm_flag_cap_ = atm_cand_cap_;
-            d_atm_flag_ = dev_alloc<int>(atm_flag_cap_ + 1);
-            d_atm_map_ = dev_alloc<int>(atm_flag_cap_ + 1);
-            scan_bytes_ = atm_scan_temp_bytes(atm_flag_cap_);
-            if (scan_bytes_ == 0) throw Error("The system is too large for the three-body term");
-            d_scan_temp_ = dev_alloc<unsigned char>(scan_bytes_);
+            const long long n = atm_cand_cap_;
+            const size_t bytes = atm_scan_temp_bytes(n);
+            if (bytes == 0) throw Error("The system is too large for the three-body term");
+            atm_flag_cap_ = 0;
+            long long held;
+            regrow(d_atm_flag_, held, n + 1);
+            regrow(d_atm_map_, held, n + 1);
+            regrow(d_scan_temp_, scan_bytes_, bytes);
+            atm_flag_cap_ = n;
         }
         check(launch_atm_mark(b, c, v, d_spheres8_, d_atm_flag_, d_atm_map_, d_scan_temp_, scan_bytes_, stream),
               "block numbers");
@@ -1192,11 +1187,8 @@ void Engine::run_three_body_group(const AtmGroup& g, const Batch& b, const Speci
     if (!capturing_) {
         // the triple kernel numbers the records with 32 bits
         if (blocks > (0xffffffffLL >> 6)) throw Error("The system is too large for the three-body term");
-        auto reserve = [&](void*& p, size_t& cap, size_t need) {
-            if (need <= cap) return;
-            free_block(p);
-            cap = compact ? need + need / 4 : need;
-            p = dev_alloc<unsigned char>(cap);
+        auto reserve = [&](unsigned char*& p, size_t& cap, size_t need) {
+            if (need > cap) regrow(p, cap, compact ? need + need / 4 : need);
         };
         reserve(d_atm_rec_, atm_rec_cap_, (size_t)std::max<long long>(blocks, 1) * rec);
         if (c.grad) reserve(d_atm_aux_, atm_aux_cap_, (size_t)std::max<long long>(blocks, 1) * aux);
@@ -1477,8 +1469,10 @@ void Engine::evaluate_host(const Damp& d, const double* positions, double* energ
     const size_t nout = nsys_ + 3 * (size_t)natoms_ + 9 * (size_t)nsys_;
     if (h_stage_len_ < nin + nout) {
         if (h_stage_) cudaFreeHost(h_stage_);
+        h_stage_ = nullptr;
+        h_stage_len_ = 0;
+        check(cudaMallocHost(&h_stage_, sizeof(double) * (nin + nout)), "cudaMallocHost");
         h_stage_len_ = nin + nout;
-        check(cudaMallocHost(&h_stage_, sizeof(double) * h_stage_len_), "cudaMallocHost");
     }
     double* hin = h_stage_;
     double* he = h_stage_ + nin;

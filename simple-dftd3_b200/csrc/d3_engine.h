@@ -153,8 +153,7 @@ private:
     bool cn_single_chunk() const;
     static constexpr size_t kCnStoreCap = size_t(768) << 20;   // bytes of stored chain-rule sums at most
     static constexpr int kFusedWeightsMaxAtoms = 65536;          // CN gather fused with weights and species vectors
-    void* d_cn_store_ = nullptr;
-    unsigned char* d_cn_store_ok_ = nullptr;
+    unsigned char *d_cn_store_ = nullptr, *d_cn_store_ok_ = nullptr;
     size_t cn_store_cap_ = 0;
     void order_atoms(const Damp& d, const double* d_positions, const Batch& b, bool mixed, cudaStream_t stream);
     double* d_hs_ = nullptr;             // Hessian scratch and result
@@ -165,6 +164,7 @@ private:
     void run(const Damp& d, const double* d_positions, double* d_energies, double* d_gradient,
              double* d_sigma9, double* d_param_grad, bool grad, cudaStream_t stream);
     template <class T> T* dev_alloc(size_t n);
+    template <class T, class C> void regrow(T*& p, C& cap, size_t n);
 
     void reduce(double* buffer, int count, cudaStream_t stream);
     Reducer reducer_ = nullptr;
@@ -326,10 +326,10 @@ private:
     unsigned short* d_atm_mask_ = nullptr;
     long long atm_cand_cap_ = 0;
     int *d_atm_flag_ = nullptr, *d_atm_map_ = nullptr;
-    void* d_scan_temp_ = nullptr;
+    unsigned char* d_scan_temp_ = nullptr;
     size_t scan_bytes_ = 0;
     long long atm_flag_cap_ = 0;
-    void *d_atm_rec_ = nullptr, *d_atm_aux_ = nullptr;
+    unsigned char *d_atm_rec_ = nullptr, *d_atm_aux_ = nullptr;
     size_t atm_rec_cap_ = 0, atm_aux_cap_ = 0;        // bytes
     double* d_e3_ = nullptr;
     double* d_sig3_ = nullptr;
