@@ -409,8 +409,10 @@ k_atm_pairs(Batch b, Species s, Config c, Work w, AtmView v, const R* UV, double
         if (ok[h]) {
             const int a = ar[h];
             const int sa = b.sp[a], sb = b.sp[bc];
+            // FP64 up to the record, whose values are rounded once each in the mixed form
+            const double u = rcp_fast(x2[h]);
             o.x = R(x2[h]);
-            o.y = R(1) / o.x;
+            o.y = R(u);
             const R* gw = gw_all + (size_t)a * kMaxRef;
             const R* dgw = dgw_all + (size_t)a * kMaxRef;
             const R* up = UV + ((size_t)bc * b.nid + sa) * (2 * kRefPad);
@@ -423,13 +425,19 @@ k_atm_pairs(Batch b, Species s, Config c, Work w, AtmView v, const R* UV, double
                 dc += gw[r] * __ldg(up + kRefPad + r);
             }
             if (b.ghost && b.ghost[a]) c6 = R(0);
-            const R r0 = R(__ldg(s.atm_r0 + sa * b.nid + sb));
+            const double r0 = __ldg(s.atm_r0 + sa * b.nid + sb);
             // the pair's share of (r0/r)^alp3, bounded so that the product of
             // three stays finite (the damping has vanished long before)
-            if constexpr (sizeof(R) == 8) o.w = fmin(exp(0.5 * alp3 * log(r0 * r0 * o.y)), 1e100);
-            else o.w = fminf(exp2f(0.5f * float(alp3) * log2f(r0 * r0 * o.y)), 1e12f);
+            if constexpr (sizeof(R) == 8) {
+                o.w = fmin(exp(0.5 * alp3 * log(r0 * r0 * u)), 1e100);
+            } else {
+                const double l = 0.5 * alp3 * log2(r0 * r0 * u);
+                const float lh = (float)l, ll = (float)(l - (double)lh);
+                const float p = exp2f(lh);
+                o.w = fminf(::fma(0.69314718f * ll, p, p), 1e12f);
+            }
             if (c6 != R(0)) {
-                R m = sqrt(c6) * o.y * sqrt(o.y);
+                R m = R(double(sqrt(c6)) * (u * rsqrt_fast(x2[h])));
                 if (c.width3 > 0.0) {
                     R sw, dsw;
                     smooth<R>(R(sqrt(x2[h])), R(c.cut3), R(c.width3), sw, dsw);
@@ -722,6 +730,7 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
             Pair fjk[4];                       // force and dE/dCN of j and of k
             double vr[3] = {0, 0, 0};          // component (lane >> 1) & 3 of sum F_i (x) T_I
             R esum = R(0);
+            double etot = 0.0;
             int ntrip = 0;
             if (GRAD)
 #pragma unroll
@@ -833,7 +842,9 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
                     }
                 }
                 const R sumE = lo(rE) + hi(rE);
+                // FP32: sums of 32 triples (four steps of eight) at most
                 esum += sumE;
+                if (sizeof(R) == 4 && (r0 & 12) == 12) { etot += double(esum); esum = R(0); }
                 if constexpr (GRAD) {
                     // after four moves the lane holds column j (upper value) and column j ^ 4 (lower)
                     const R Wik = hi(kE) + __shfl_xor_sync(kAll, lo(kE), 4);
@@ -885,7 +896,7 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
             // ---- flush: energy, then the (j, k) sums and the forces of j and k
             unsigned long long* fe = fxe + (size_t)20 * (id.t8 + J);
             {
-                double es = double(esum);
+                double es = etot + double(esum);
                 for (int o = 16; o > 0; o >>= 1) es += __shfl_xor_sync(kAll, es, o);
                 if (lane == 0) fixed_add(fe, es);
                 if (GEN && counting) {
