@@ -426,15 +426,15 @@ k_atm_pairs(Batch b, Species s, Config c, Work w, AtmView v, const R* UV, double
             }
             if (b.ghost && b.ghost[a]) c6 = R(0);
             const double r0 = __ldg(s.atm_r0 + sa * b.nid + sb);
-            // the pair's share of (r0/r)^alp3, bounded so that the product of
-            // three stays finite (the damping has vanished long before)
+            // the pair's share of (r0/r)^alp3, bounded so that the product of three (FP32:
+            // of two; the third may take it to infinity, where f is zero) stays finite
             if constexpr (sizeof(R) == 8) {
                 o.w = fmin(exp(0.5 * alp3 * log(r0 * r0 * u)), 1e100);
             } else {
                 const double l = 0.5 * alp3 * log2(r0 * r0 * u);
                 const float lh = (float)l, ll = (float)(l - (double)lh);
                 const float p = exp2f(lh);
-                o.w = fminf(::fma(0.69314718f * ll, p, p), 1e12f);
+                o.w = fminf(::fma(0.69314718f * ll, p, p), 1e18f);
             }
             if (c6 != R(0)) {
                 R m = R(double(sqrt(c6)) * (u * rsqrt_fast(x2[h])));
@@ -822,8 +822,8 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
                     } else {
                         const Pair E = Mf * B1;
                         const Pair q2 = a2 * a3, q3 = a1 * a3;
-                        // K = (1 + A) w - A with w = alp/2 6Pf - 3/2: (1 + A)(w - 1) + 1
-                        const Pair KM = fma(B1, fma(p6 * f, ahalf, pk(R(-2.5), R(-2.5))), one) * Mf;
+                        // K = (1 + A) w - A with w = alp/2 6Pf - 3/2: (1 + A)(w - 1) + 1, 6Pf = 1 - f
+                        const Pair KM = fma(B1, fma(one - f, ahalf, pk(R(-2.5), R(-2.5))), one) * Mf;
                         const Pair V = U * Mf;
                         const Pair dq = q2 - q1, sq = q2 + q1;
                         rK = rK + KM;

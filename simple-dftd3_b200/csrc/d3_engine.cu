@@ -1130,12 +1130,15 @@ bool Engine::atm_compact(bool mixed) const
     return (size_t)atm_.ncand * atm_block_bytes(mixed, true) > kAtmDenseCap;
 }
 
-void Engine::run_three_body(const Batch& b, const Species& s, const Damp& d, const Config& c, Work& w,
+void Engine::run_three_body(const Batch& b, const Species& s, const Damp& d, const Config& c_, Work& w,
                             cudaStream_t stream, bool prepared)
 {
     ensure_atm_layout(stream);
-    // the two-body pass computed the species vectors; without it they are computed here
-    if (!species_ready_) launch_species_vectors(b, s, c, w, pu_.U, stream);
+    Config c = c_;
+    c.mixed = atm_mixed(d);
+    // the two-body pass computed the species vectors; without it, or in another precision, they
+    // are computed here (after that pass, which has no more use for them)
+    if (!species_ready_ || c.mixed != c_.mixed) launch_species_vectors(b, s, c, w, pu_.U, stream);
     AtmView v = atm_;
     if (!prepared)
         launch_atm_order(b, d_tile_off_, d_tile_sys_, ntiles_, v, atm_compact(c.mixed) ? d_spheres8_ : nullptr,
@@ -1377,7 +1380,7 @@ void Engine::run_graphed(const Damp& d, bool grad, bool pg, cudaStream_t stream)
     if (threebody) ensure_atm_layout(stream);
     if (graph_valid_ && graph_epoch_ == alloc_epoch_ && std::memcmp(&key, &graph_key_, sizeof(key)) == 0) {
         check(cudaGraphLaunch(graph_exec_, stream), "cudaGraphLaunch");
-        if (!threebody || !atm_compact(mixed_)) return;
+        if (!threebody || !atm_compact(atm_mixed(d))) return;
         // the three-body blocks must have fitted the buffers the graph was captured with
         check(cudaMemcpyAsync(h_guard_, d_guard_, sizeof(int), cudaMemcpyDeviceToHost, stream), "guard");
         check(cudaStreamSynchronize(stream), "graph");
@@ -1439,7 +1442,7 @@ double Engine::autotune(const Damp& d, const double* d_positions, bool grad, cud
         for (int sp : {1, 2, 4})
             if (sp != best.pair_split) { Tuning t = best; t.pair_split = sp; consider(t); }
         if (threebody) {
-            const int occ = atm_blocks_per_sm(mixed_, grad, any_periodic_, part_.nparts > 1);
+            const int occ = atm_blocks_per_sm(atm_mixed(d), grad, any_periodic_, part_.nparts > 1);
             const int cur = best.atm_blocks_per_sm > 0 ? std::min(best.atm_blocks_per_sm, occ) : occ;
             for (int bps = 1; bps <= occ; bps++)
                 if (bps != cur) { Tuning t = best; t.atm_blocks_per_sm = bps; consider(t); }

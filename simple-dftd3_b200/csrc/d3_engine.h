@@ -287,6 +287,11 @@ private:
     void* d_mol_fstore_ = nullptr;       // CN derivatives of small molecules' pairs
     void ensure_atm_layout(cudaStream_t stream);
     bool atm_compact(bool mixed) const;
+    // FP32 triples up to this exponent: a pair's share (r0/r)^((alp + 2) / 3) of the damping
+    // is bounded at 1e18 in FP32, which at 50 is passed below a twelfth of r0 (0.7 Bohr at
+    // most), and at 100, where the bound would bite at a third of r0, costs the energy.
+    static constexpr double kAtmMixedMaxAlp = 50.0;
+    bool atm_mixed(const Damp& d) const { return mixed_ && d.alp <= kAtmMixedMaxAlp; }
     void free_block(void*& p);
     // blocks above this size are kept for the tile pairs in reach only
     static constexpr size_t kAtmDenseCap = size_t(1) << 30;
