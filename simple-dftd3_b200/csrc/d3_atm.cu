@@ -38,6 +38,7 @@
 // All sums over units go to fixed-point accumulators (integer additions), so the
 // results do not depend on the order of the warps and repeat bit for bit.
 #include <cub/cub.cuh>
+#include <math_constants.h>
 
 #include <algorithm>
 #include <cfloat>
@@ -78,10 +79,11 @@ __device__ __forceinline__ double norm2(double x, double y, double z)
     return __fma_rn(z, z, __fma_rn(y, y, __dmul_rn(x, x)));
 }
 
-__device__ __forceinline__ void fixed_add(unsigned long long* acc2, double v)
+__device__ __forceinline__ void fixed_add(unsigned long long* acc2, double v, unsigned long long* tile)
 {
     long long hi, lo;
     fixed_split(v, hi, lo);
+    if (!fixed_fits(hi)) tile[kTileMark] = 1;
     atomicAdd(acc2, (unsigned long long)hi);
     atomicAdd(acc2 + 1, (unsigned long long)lo);
 }
@@ -273,9 +275,9 @@ __global__ void k_atm_order(Batch b, const int* tile_off, const int* tile_sys, i
         for (int k = 0; k < 8; k++) f[k] = 0;
     }
     if (lane < n8) {
-        unsigned long long* f = fxe + (size_t)20 * (base8 + lane);
+        unsigned long long* f = fxe + (size_t)kTileSums * (base8 + lane);
 #pragma unroll
-        for (int k = 0; k < 20; k++) f[k] = 0;
+        for (int k = 0; k < kTileSums; k++) f[k] = 0;
     }
     if (!spheres) return;
     // bounding spheres (box centre, largest distance)
@@ -884,6 +886,7 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
                         if (rin) {
                             long long hi, lo;
                             fixed_split(g, hi, lo);
+                            if (!fixed_fits(hi)) fxe[(size_t)kTileSums * (e.z >> 3) + kTileMark] = 1;
                             atomicAdd(fxf + (size_t)8 * (int)pi.w + 2 * comp + (lane & 1),
                                       (unsigned long long)((lane & 1) ? lo : hi));
                         }
@@ -894,11 +897,11 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
             head = (head + nroot) & (kRing - 1);
             cnt -= nroot;
             // ---- flush: energy, then the (j, k) sums and the forces of j and k
-            unsigned long long* fe = fxe + (size_t)20 * (id.t8 + J);
+            unsigned long long* fe = fxe + (size_t)kTileSums * (id.t8 + J);
             {
                 double es = etot + double(esum);
                 for (int o = 16; o > 0; o >>= 1) es += __shfl_xor_sync(kAll, es, o);
-                if (lane == 0) fixed_add(fe, es);
+                if (lane == 0) fixed_add(fe, es, fe);
                 if (GEN && counting) {
                     for (int o = 16; o > 0; o >>= 1) ntrip += __shfl_xor_sync(kAll, ntrip, o);
                     if (lane == 0) atomicAdd(queue + 1, (unsigned long long)ntrip);
@@ -953,8 +956,8 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
                     p1 = sel(h16, fk[3], fk[1]) + __shfl_xor_sync(kAll, sel(h16, fk[1], fk[3]), 16);
                     ck = double(sel(h8, p1, p0) + __shfl_xor_sync(kAll, sel(h8, p0, p1), 8));
                 }
-                if (aj >= 0) fixed_add(fxf + (size_t)8 * aj + 2 * q, cj);
-                if (ak >= 0) fixed_add(fxf + (size_t)8 * ak + 2 * q, ck);
+                if (aj >= 0) fixed_add(fxf + (size_t)8 * aj + 2 * q, cj, fe);
+                if (ak >= 0) fixed_add(fxf + (size_t)8 * ak + 2 * q, ck, fxe + (size_t)kTileSums * (id.t8 + K));
                 if (PER) {
                     // sum of F (x) T over the images: the roots' and k's
                     double kc = ck;
@@ -965,9 +968,9 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
                     const int comp = lane >> 1;
                     const double kcc = __shfl_sync(kAll, kc, (8 * comp) & 31);
                     if (lane < 6 && !(lane & 1)) {
-                        fixed_add(fe + 2 * (1 + 3 * comp), ::fma(kcc, kx, vr[0]));
-                        fixed_add(fe + 2 * (2 + 3 * comp), ::fma(kcc, ky, vr[1]));
-                        fixed_add(fe + 2 * (3 + 3 * comp), ::fma(kcc, kz, vr[2]));
+                        fixed_add(fe + 2 * (1 + 3 * comp), ::fma(kcc, kx, vr[0]), fe);
+                        fixed_add(fe + 2 * (2 + 3 * comp), ::fma(kcc, ky, vr[1]), fe);
+                        fixed_add(fe + 2 * (3 + 3 * comp), ::fma(kcc, kz, vr[2]), fe);
                     }
                 }
             }
@@ -991,13 +994,16 @@ __global__ void k_atm_finish(Batch b, Config c, AtmView v, int ntiles8, double s
     const int a = v.sub[slot];
     if (a < 0) return;
     const bool first = (slot & 7) == 0;
-    const unsigned long long* fe = fxe + (size_t)20 * (slot >> 3);
-    e3[a] = first ? s9 * fixed_value(fe) : 0.0;
+    const unsigned long long* fe = fxe + (size_t)kTileSums * (slot >> 3);
+    // NaN for a marked tile (and for an atom without a position, whose tile may be out of reach)
+    const double nan = fe[kTileMark] || !isfinite(b.x[a] + b.y[a] + b.z[a]) ? CUDART_NAN : 0.0;
+    e3[a] = (first ? s9 * fixed_value(fe) : 0.0) + nan;
     if (!c.grad) return;
     const unsigned long long* f = fxf + (size_t)8 * a;
-    const double g[3] = {2.0 * s9 * fixed_value(f), 2.0 * s9 * fixed_value(f + 2), 2.0 * s9 * fixed_value(f + 4)};
+    const double g[3] = {2.0 * s9 * fixed_value(f) + nan, 2.0 * s9 * fixed_value(f + 2) + nan,
+                         2.0 * s9 * fixed_value(f + 4) + nan};
     for (int k = 0; k < 3; k++) w.grad[3 * a + k] += g[k];
-    w.dEdcn[a] += s9 * fixed_value(f + 6);
+    w.dEdcn[a] += s9 * fixed_value(f + 6) + nan;
     const int o = b.atom_off[b.sys_of_atom[a]];
     const double x = b.x[a] - b.x[o], y = b.y[a] - b.y[o], z = b.z[a] - b.z[o];
     double s[kSigma] = {g[0] * x, g[1] * y, g[2] * z, 0.5 * (g[0] * y + g[1] * x), 0.5 * (g[0] * z + g[2] * x),

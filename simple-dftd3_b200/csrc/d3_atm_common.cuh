@@ -37,7 +37,8 @@ __device__ __forceinline__ bool owns_pair_atm(const Partition& p, int i, int j)
 // is at most 2^31 units either way: its word takes 2^32 additions before it could
 // overflow.  An atom of a cell of one atom with N neighbours gets about N^2 / 4 of
 // them (fcc Cu: 2.6e6 at a three-body cutoff of 40 Bohr, 3.0e7 at 60, 2^32 at 135),
-// an atom of a larger cell fewer.  Sums reach to +-2^23.
+// an atom of a larger cell fewer.  Sums reach to +-2^23.  A value of 2^22 or more, an
+// infinity or a NaN has no such form: the caller marks the tile (fixed_fits).
 __device__ __forceinline__ void fixed_split(double v, long long& hi, long long& lo)
 {
     const double sv = v * 1099511627776.0;              // 2^40
@@ -45,6 +46,16 @@ __device__ __forceinline__ void fixed_split(double v, long long& hi, long long& 
     hi = (long long)h;
     lo = __double2ll_rn((sv - h) * 4294967296.0);       // 2^32
 }
+
+__device__ __forceinline__ bool fixed_fits(long long hi)
+{
+    return (unsigned long long)(hi + (1LL << 62)) < (1ULL << 63);
+}
+
+// Sums of a three-body tile: energy, the nine sums of F (x) T, two words each, and the
+// mark that a sum of the tile or of its atoms met a value without fixed-point form:
+// the results it enters are NaN.
+constexpr int kTileSums = kAtmTileSums, kTileMark = kAtmTileSums - 1;
 
 __device__ __forceinline__ double fixed_value(const unsigned long long* acc2)
 {

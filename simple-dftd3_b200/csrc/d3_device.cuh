@@ -316,6 +316,7 @@ struct AtmView {
     void* rec = nullptr;                   // [blocks][64] pair records (4 values)
     void* aux = nullptr;                   // [blocks][64] CN derivatives (2 values)
 };
+constexpr int kAtmTileSums = 21;           // words: ten fixed-point sums and the mark of a value without one
 struct AtmLaunch {
     Batch b;
     Config c;
@@ -328,7 +329,7 @@ struct AtmLaunch {
     bool periodic = false, counting = false;
     unsigned long long *queue = nullptr;   // [2] next unit, counted triples x 3
     unsigned long long *fxf = nullptr;     // [natoms][4][2] fixed-point force / (2 s9), dE/dCN / s9
-    unsigned long long *fxe = nullptr;     // [ntiles8][10][2] energy / s9, sum of F (x) T / (2 s9)
+    unsigned long long *fxe = nullptr;     // [ntiles8][kAtmTileSums] energy / s9, sum of F (x) T / (2 s9), mark
     const int* guard = nullptr;            // set: the blocks did not fit, skip the work
     cudaStream_t stream = nullptr;
 };

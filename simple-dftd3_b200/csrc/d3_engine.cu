@@ -1047,7 +1047,7 @@ void Engine::ensure_atm_layout(cudaStream_t stream)
         d_e3_ = dev_alloc<double>(n);
         d_sig3_ = dev_alloc<double>(kSigma * n);
         d_fxf_ = dev_alloc<unsigned long long>(8 * n);
-        d_fxe_ = dev_alloc<unsigned long long>(20 * n8);
+        d_fxe_ = dev_alloc<unsigned long long>(kAtmTileSums * n8);
         d_atm_queue_ = dev_alloc<unsigned long long>(2);
         d_guard_ = dev_alloc<int>(1);
         check(cudaMallocHost(&h_atm_total_, sizeof(int)), "cudaMallocHost");

@@ -18,6 +18,7 @@
 // -> 25 us and with the three-body term 68 -> 48 us, 251 atoms (zero damping) 38 -> 34
 // us (16 SMs share the FP64 work of 63 000 pair ends then: 25 us in the kernel).
 #include <cooperative_groups.h>
+#include <math_constants.h>
 
 #include <cfloat>
 #include <cstdint>
@@ -313,7 +314,7 @@ __global__ void __launch_bounds__(kMolThreads, 1) k_mol_pairs(MolArgs a)
                 a.v.sub[slot] = active ? a0 + i : -1;
                 a.v.pos[slot] = active ? make_double4(xi, yi, zi, (double)(a0 + i)) : make_double4(0.0, 0.0, 0.0, 0.0);
             }
-            if (i % kMolSlots == 0 && lane < 20) a.fxe[(size_t)20 * (slot / kMolSlots) + lane] = 0;
+            if (i % kMolSlots == 0 && lane < kTileSums) a.fxe[(size_t)kTileSums * (slot / kMolSlots) + lane] = 0;
         }
         if (sys == 0 && rank == 0 && tid < 2) a.queue[tid] = 0;
         if (active) {
@@ -351,17 +352,21 @@ __global__ void __launch_bounds__(kMolThreads, 1) k_mol_finish(MolArgs a)
     const Batch& b = a.b;
     const int a0 = b.atom_off[sys], n = b.atom_off[sys + 1] - a0;
     const double s9 = a.d.s9;
+    // NaN for a marked tile
+    const unsigned long long* fe = a.fxe + (size_t)kTileSums * a.v.t8_off[sys];
+    auto mark = [&](int k) { return fe[(size_t)kTileSums * (k / kMolSlots) + kTileMark] ? CUDART_NAN : 0.0; };
     if (GRAD)
         for (int k = tid; k < n; k += kMolThreads) {
             sh.pos[3 * k] = a.x[a0 + k]; sh.pos[3 * k + 1] = a.y[a0 + k]; sh.pos[3 * k + 2] = a.z[a0 + k];
-            sh.de[k] = a.w.dEdcn[a0 + k] + s9 * fixed_value(a.fxf + (size_t)8 * (a0 + k) + 6);
+            sh.de[k] = a.w.dEdcn[a0 + k] + s9 * fixed_value(a.fxf + (size_t)8 * (a0 + k) + 6) + mark(k);
         }
     cluster.sync();
     const int i = kMolWarps * rank + wid;
     double v[7] = {0, 0, 0, 0, 0, 0, 0};
     if (i < n) {
-        v[0] = a.w.e_atom[a0 + i];
-        if (i % kMolSlots == 0) v[0] += s9 * fixed_value(a.fxe + (size_t)20 * (a.v.t8_off[sys] + i / kMolSlots));
+        const double nan = mark(i);
+        v[0] = a.w.e_atom[a0 + i] + nan;
+        if (i % kMolSlots == 0) v[0] += s9 * fixed_value(fe + (size_t)kTileSums * (i / kMolSlots));
         if (GRAD) {
             R fk[kMolSteps];
             const R* fs = (const R*)a.fstore + (size_t)(a0 + i) * kMolAtoms;
@@ -372,7 +377,8 @@ __global__ void __launch_bounds__(kMolThreads, 1) k_mol_finish(MolArgs a)
             gx = mol_wsum(gx); gy = mol_wsum(gy); gz = mol_wsum(gz);
             for (int k = 0; k < kSigma; k++) sg[k] = mol_wsum(sg[k]);
             const unsigned long long* f = a.fxf + (size_t)8 * (a0 + i);
-            const double tx = 2.0 * s9 * fixed_value(f), ty = 2.0 * s9 * fixed_value(f + 2), tz = 2.0 * s9 * fixed_value(f + 4);
+            const double tx = 2.0 * s9 * fixed_value(f) + nan, ty = 2.0 * s9 * fixed_value(f + 2) + nan,
+                         tz = 2.0 * s9 * fixed_value(f + 4) + nan;
             // the three-body virial is sum F_a (x) x_a, the origin being free
             const double x = sh.pos[3 * i] - sh.pos[0], y = sh.pos[3 * i + 1] - sh.pos[1], z = sh.pos[3 * i + 2] - sh.pos[2];
             const double t3[kSigma] = {tx * x, ty * y, tz * z, 0.5 * (tx * y + ty * x), 0.5 * (tx * z + tz * x),

@@ -44,3 +44,27 @@ def test_other_systems_keep_their_bits(sizes, periodic, precision, where):
     assert e1[1] == e0[1] and np.array_equal(g1[sizes[0]:], g0[sizes[0]:])
     e2, g2 = evaluate(x)
     assert np.array_equal(e2, e0) and np.array_equal(g2, g0)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("sizes, periodic", [((12, 40), False), ((300, 31), False), ((17, 270), False), ((12, 37), True)])
+@pytest.mark.parametrize("where, value", [(0, float("nan")), (11, float("nan")), (3, float("inf"))])
+def test_three_body_term_is_nan(sizes, periodic, precision, where, value):
+    """The three-body term alone: NaN for the system and for the atom, as any sum with a NaN, not the numbers its
+    fixed-point form would have."""
+    import torch
+    from dftd3.torch_api import D3Batch
+    nums, pos, lats = _systems(sizes, periodic)
+    model = D3Batch(nums, lattices=lats, periodic=np.ones((2, 3), dtype=bool) if periodic else None,
+                    precision=precision, cutoffs=(20.0, 15.0, 15.0, 0.0, 0.0))
+    params = torch.tensor([0.0, 0.0, 0.4289, 4.4407, 1.0], dtype=torch.float64)
+    x = torch.tensor(np.concatenate(pos), device="cuda")
+    e0 = model(x.clone().requires_grad_(), params)      # the energies of the pass with gradients
+    x[where, 2] = value
+    x.requires_grad_()
+    e1 = model(x, params)
+    e1.sum().backward()
+    assert torch.isnan(e1[0]) and e1[1] == e0[1]
+    assert torch.isnan(x.grad[where]).all()
+    assert torch.isfinite(x.grad[sizes[0]:]).all()
+    assert torch.isnan(model(x.detach(), params)[0])
