@@ -731,8 +731,7 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
             Pair Djk[4], Wjk[4];
             Pair fjk[4];                       // force and dE/dCN of j and of k
             double vr[3] = {0, 0, 0};          // component (lane >> 1) & 3 of sum F_i (x) T_I
-            R esum = R(0);
-            double etot = 0.0;
+            double esum = 0.0;
             int ntrip = 0;
             if (GRAD)
 #pragma unroll
@@ -844,9 +843,7 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
                     }
                 }
                 const R sumE = lo(rE) + hi(rE);
-                // FP32: sums of 32 triples (four steps of eight) at most
-                esum += sumE;
-                if (sizeof(R) == 4 && (r0 & 12) == 12) { etot += double(esum); esum = R(0); }
+                esum += double(sumE);
                 if constexpr (GRAD) {
                     // after four moves the lane holds column j (upper value) and column j ^ 4 (lower)
                     const R Wik = hi(kE) + __shfl_xor_sync(kAll, lo(kE), 4);
@@ -899,7 +896,7 @@ k_atm_triples(Batch b, Config c, Partition part, AtmView v, double alp3d, int sp
             // ---- flush: energy, then the (j, k) sums and the forces of j and k
             unsigned long long* fe = fxe + (size_t)kTileSums * (id.t8 + J);
             {
-                double es = etot + double(esum);
+                double es = esum;
                 for (int o = 16; o > 0; o >>= 1) es += __shfl_xor_sync(kAll, es, o);
                 if (lane == 0) fixed_add(fe, es, fe);
                 if (GEN && counting) {
