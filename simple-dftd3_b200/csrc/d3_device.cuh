@@ -182,11 +182,14 @@ struct Tuning {
 
 // Pairwise decomposition (d3_pairwise.cu), FP64: energy2 and energy3 of every
 // system as [n_s][n_s] blocks at off[sys] (input atom order); c6 is scratch of
-// the same size, factors of twice that (16-byte aligned; used for molecules: every
-// system has one lattice point).  Needs the sorted atoms and the reference weights.
+// the same size.  factors: pairwise_factor_doubles, 16-byte aligned (the pair factors
+// of every pair and three-body translation, n_s^2 nT_s from foff[sys], ftotal in all),
+// null with s9 = 0, or for periodic systems without the memory: the triples compute
+// them.  Needs the sorted atoms and the reference weights.
+size_t pairwise_factor_doubles(long long total, long long ftotal, int natoms);
 void launch_pairwise(const Batch& b, const Species& s, const Damp& d, const Config& c, const Work& w,
-                     const long long* off, long long total, bool molecules, double* c6, double* factors, double* e2,
-                     double* e3, cudaStream_t stream);
+                     const long long* off, long long total, const long long* foff, long long ftotal, double* c6,
+                     double* factors, double* e2, double* e3, cudaStream_t stream);
 // dst[k] = src[k], k < n (dst pinned host memory).
 void launch_copy_out(const double* src, double* dst, long long n, cudaStream_t stream);
 

@@ -660,11 +660,37 @@ void Engine::pairwise_host(const Damp& d, const double* positions, double* energ
     ensure_workspace(false, false, false);
     upload_pair_table(d, stream);
     const long long total = std::max<long long>(c6mat_total_, 1);
-    if (!d_pw_off_) {
-        d_pw_ = dev_alloc<double>(5 * (size_t)total);
-        d_pw_off_ = dev_alloc<long long>(nsys_);
-        check(cudaMemcpy(d_pw_off_, c6mat_off_.data(), sizeof(long long) * nsys_, cudaMemcpyHostToDevice),
-              "pairwise offsets");
+    if (!d_pw_) d_pw_ = dev_alloc<double>(3 * (size_t)total);
+    if (!d_pw_off_) d_pw_off_ = dev_alloc<long long>(2 * (size_t)nsys_);
+    std::vector<long long> off(c6mat_off_);
+    long long ftotal = 0;
+    for (int sy = 0; sy < nsys_; sy++) {
+        off.push_back(ftotal);
+        ftotal += (long long)sys_natoms_[sy] * sys_natoms_[sy] * img_rep_[4 * (size_t)sy + 3];
+    }
+    if (off != pw_off_) {
+        pw_off_.clear();
+        check(cudaMemcpy(d_pw_off_, off.data(), sizeof(long long) * off.size(), cudaMemcpyHostToDevice), "pairwise offsets");
+        pw_off_ = std::move(off);
+    }
+    // without memory for them the triples of periodic systems compute the factors (cell of
+    // 400 atoms 647 ms, from the table 88 ms)
+    struct Held {
+        double* p = nullptr;
+        ~Held() { if (p) cudaFree(p); }
+    } held;
+    double* factors = nullptr;
+    if (std::fabs(d.s9) >= DBL_EPSILON) {
+        const size_t len = pairwise_factor_doubles(c6mat_total_, ftotal, natoms_);
+        if (sizeof(double) * len <= kPwKeep || ftotal == c6mat_total_) {
+            if (len > pw_mp_len_) regrow(d_pw_mp_, pw_mp_len_, len);
+            factors = d_pw_mp_;
+        } else if (cudaMalloc(&held.p, sizeof(double) * len) == cudaSuccess) {
+            factors = held.p;
+        } else {
+            held.p = nullptr;
+            (void)cudaGetLastError();
+        }
     }
     check(cudaMemcpyAsync(d_pos_in_, positions, sizeof(double) * 3 * natoms_, cudaMemcpyHostToDevice, stream),
           "positions");
@@ -695,23 +721,23 @@ void Engine::pairwise_host(const Damp& d, const double* positions, double* energ
         launch_cn_units(b, s, c, Partition{}, w, pu_, false, stream);
         launch_weights(b, s, c, w, stream);
     }
-    launch_pairwise(b, s, d, c, w, d_pw_off_, c6mat_total_, !any_periodic_, d_pw_ + 2 * total, d_pw_, d_pw_ + 3 * total,
-                    d_pw_ + 4 * total, stream);
+    launch_pairwise(b, s, d, c, w, d_pw_off_, c6mat_total_, d_pw_off_ + nsys_, ftotal, d_pw_, factors, d_pw_ + total,
+                    d_pw_ + 2 * total, stream);
     check(cudaGetLastError(), "pairwise kernels");
     const size_t nn = (size_t)c6mat_total_;
     if (double* out = pinned_results(2 * nn)) {
         // Both matrices side by side, by a kernel's stores.  Two copies to the caller's
         // pageable memory took 68 us of a call for 150 atoms (167 us, 99 now).
-        launch_copy_out(d_pw_ + 3 * total, out, 2 * c6mat_total_, stream);
+        launch_copy_out(d_pw_ + total, out, 2 * c6mat_total_, stream);
         check(cudaGetLastError(), "pairwise kernels");
         check(cudaStreamSynchronize(stream), "pairwise");
         std::memcpy(energy2, out, sizeof(double) * nn);
         std::memcpy(energy3, out + nn, sizeof(double) * nn);
         return;
     }
-    check(cudaMemcpyAsync(energy2, d_pw_ + 3 * total, sizeof(double) * c6mat_total_, cudaMemcpyDeviceToHost, stream),
+    check(cudaMemcpyAsync(energy2, d_pw_ + total, sizeof(double) * c6mat_total_, cudaMemcpyDeviceToHost, stream),
           "pairwise energy2");
-    check(cudaMemcpyAsync(energy3, d_pw_ + 4 * total, sizeof(double) * c6mat_total_, cudaMemcpyDeviceToHost, stream),
+    check(cudaMemcpyAsync(energy3, d_pw_ + 2 * total, sizeof(double) * c6mat_total_, cudaMemcpyDeviceToHost, stream),
           "pairwise energy3");
     check(cudaStreamSynchronize(stream), "pairwise");
 }

@@ -159,8 +159,13 @@ private:
     double* d_hs_ = nullptr;             // Hessian scratch and result
     double* d_rvdw_ = nullptr;           // [nid][nid] van der Waals radii (Hessian damping kernels)
     std::vector<int> img_off_host_;      // host copy of the image offsets
-    double* d_pw_ = nullptr;             // pairwise decomposition: pair factors, C6, energy2, energy3 (5 x sum n_s^2)
-    long long* d_pw_off_ = nullptr;
+    double* d_pw_ = nullptr;             // pairwise decomposition: C6, energy2, energy3 (3 x sum n_s^2)
+    long long* d_pw_off_ = nullptr;      // [2][nsys] first pair of each system, first pair and translation
+    std::vector<long long> pw_off_;      // its host copy
+    // pair factors of the triples: kept with the engine up to 256 MB, above that for the call
+    static constexpr size_t kPwKeep = size_t(256) << 20;
+    double* d_pw_mp_ = nullptr;
+    size_t pw_mp_len_ = 0;
     void run(const Damp& d, const double* d_positions, double* d_energies, double* d_gradient,
              double* d_sigma9, double* d_param_grad, bool grad, cudaStream_t stream);
     template <class T> T* dev_alloc(size_t n);
