@@ -290,9 +290,12 @@ Engine::Engine(int nsys, const int* natoms, const int* numbers, const double* la
     pu_.units = d_units_;
     pu_.unit_base = d_unit_base_;
     pu_.U = dev_alloc<double>(species_vector_doubles(natoms_, nid));
-    // slots for the largest split: four, or more for few tile pairs
+    any_periodic_ = false;
+    for (int sy = 0; sy < nsys; sy++) any_periodic_ = any_periodic_ || periodic_any(sy);
+    // slots for the largest split: four, or as many as auto_split takes for few tile pairs
     max_split_ = 4;
-    while (max_split_ < 32 && (long long)pu_.nunits * max_split_ < 6LL * sms_) max_split_ *= 2;
+    const long long want = any_periodic_ ? 6LL * sms_ : max_sys_atoms_ > kDiagonalMaxAtoms ? 2LL * sms_ : 0;
+    while (max_split_ < 32 && pu_.nunits * (long long)max_split_ < want) max_split_ *= 2;
     const size_t items = (size_t)std::max(pu_.nunits, 1) * max_split_;
     pu_.unit_i = dev_alloc<double>(items * pair_unit_slot_doubles());
     pu_.unit_j = pu_.unit_i + items * pair_unit_i_doubles();
@@ -309,8 +312,6 @@ Engine::Engine(int nsys, const int* natoms, const int* numbers, const double* la
     }
     c6mat_total_ = off;
     sys_natoms_.assign(natoms, natoms + nsys);
-    any_periodic_ = false;
-    for (int sy = 0; sy < nsys; sy++) any_periodic_ = any_periodic_ || periodic_any(sy);
     t8_off_.assign(nsys + 1, 0);
     for (int sy = 0; sy < nsys; sy++) t8_off_[sy + 1] = t8_off_[sy] + (natoms[sy] + 7) / 8;
     ntiles8_ = t8_off_[nsys];
@@ -638,7 +639,11 @@ void Engine::order_atoms(const Damp& d, const double* d_positions, const Batch& 
 
 double* Engine::pinned_results(size_t n)
 {
-    if (n > kPinnedResults) return nullptr;
+    // a model's first matrix is often its only one: the buffer comes with the second
+    if (!results_asked_ || n > kPinnedResults) {
+        results_asked_ = true;
+        return nullptr;
+    }
     if (n > h_results_len_) {
         if (h_results_) {
             check(cudaStreamSynchronize(stream_), "results");
@@ -646,7 +651,11 @@ double* Engine::pinned_results(size_t n)
             h_results_ = nullptr;
             h_results_len_ = 0;
         }
-        check(cudaMallocHost(&h_results_, sizeof(double) * n), "cudaMallocHost");
+        if (cudaMallocHost(&h_results_, sizeof(double) * n) != cudaSuccess) {
+            (void)cudaGetLastError();
+            h_results_ = nullptr;
+            return nullptr;
+        }
         h_results_len_ = n;
     }
     return h_results_;
@@ -760,8 +769,8 @@ int Engine::auto_split(int least) const
 }
 
 // Molecules: the two-body and CN diagonal walks (FP64 only for systems of at most
-// 256 atoms, where few tile pairs lie beyond the cutoff), which take whole units.
-bool Engine::diagonal_walks() const { return !any_periodic_ && (mixed_ || max_sys_atoms_ <= 256); }
+// kDiagonalMaxAtoms, where few tile pairs lie beyond the cutoff), which take whole units.
+bool Engine::diagonal_walks() const { return !any_periodic_ && (mixed_ || max_sys_atoms_ <= kDiagonalMaxAtoms); }
 
 int Engine::pair_split() const
 {

@@ -195,6 +195,7 @@ private:
     std::vector<int> sys_natoms_;
     int max_split_ = 4;                  // items per tile pair the slots are sized for
     int auto_split(int least) const;
+    static constexpr int kDiagonalMaxAtoms = 256;
     bool diagonal_walks() const;
     int pair_split() const;              // items per tile pair of the two-body sweep
     int cn_split() const;                // items per tile pair of the CN sweeps
@@ -272,12 +273,14 @@ private:
     double *d_energies_ = nullptr, *d_grad_out_ = nullptr, *d_sigma_ = nullptr;
     double *h_stage_ = nullptr;   // pinned staging: positions in, results out
     size_t h_stage_len_ = 0;
-    // Pinned buffer for n result doubles (grown, kept with the engine), or null above
-    // kPinnedResults = 8 MB.  Below it stores to the buffer were the faster way at every
+    // Pinned buffer for n result doubles (grown, kept with the engine) from the second
+    // request on, or null: its allocation (6 ms for 0.4 and for 6 MB) takes longer than the
+    // copies it saves in one call.  Null as well above kPinnedResults = 8 MB.  Below it stores to the buffer were the faster way at every
     // size (pairwise 700 atoms 5.3 -> 4.1 ms, Hessian of 330 2.69 -> 2.62 ms); above it
     // the kernels' work grows with the cube and pinned memory is not worth holding.
     static constexpr size_t kPinnedResults = size_t(1) << 20;
     double* pinned_results(size_t n);
+    bool results_asked_ = false;
     double* h_results_ = nullptr;
     size_t h_results_len_ = 0;
     unsigned long long* d_counts_ = nullptr;
