@@ -61,7 +61,7 @@ constexpr int kRootChunk = 128;         // roots between two flushes: FP32 sums 
 
 // Resident blocks per SM the triple kernel is compiled for.  FP32 with gradient:
 // 168 registers and 12 warps beat 128 registers (spills) and 16 warps, 54.8
-// against 59.1 ms on eight frames; FP64 with gradient: 254 registers and 8 warps
+// against 59.1 ms on eight frames; FP64 with gradient: 252 registers and 8 warps
 // beat 168 and 12 (cluster of 5000 atoms 15.5 against 17.7 ms); energies: 16 and
 // 12 warps beat 20 and 16 (slab 0.63 against 0.74 ms, before its pair sweeps were
 // cut into more items).
@@ -548,7 +548,7 @@ __device__ __forceinline__ void async_copy_value(V* dst, const V* src)
 // Columns of the pair p of a step: with gradients the lanes of a quarter take
 // different k, (j + p) mod 8 and k ^ 4, and the column sums travel with k; energies
 // have no column sums, so that all lanes take the same k, p and p + 4, and its records
-// are broadcast reads (141-atom slab 339 -> 299 us; with gradients the exchanges of
+// are broadcast reads (141-atom slab 339 -> 305 us; with gradients the exchanges of
 // the column sums cost what the reads save: eight frames 51.2 against 52.5 ms).
 template <bool GRAD>
 __device__ __forceinline__ int column(int j, int p) { return GRAD ? (j + p) & 7 : p; }
@@ -556,7 +556,7 @@ __device__ __forceinline__ int column(int j, int p) { return GRAD ? (j + p) & 7 
 // What bounds it: the data pipe of L1 and shared memory (74% busy in FP32, 86% in
 // FP64: the (i, k) records of a step, staged roots, shuffles of the column sums),
 // with 12 or 8 warps per SM to hide its latency and that of the FMA chains (2.2 and
-// 1.7 instructions per cycle and SM; FMA pipe 44%, FP64 pipe 51%).  A step of two
+// 1.7 instructions per cycle and SM; FMA pipe 44%, FP64 pipe 49%).  A step of two
 // partners (k and k ^ 4) is 39 packed FP32 instructions, two reciprocals, four
 // shuffles and two 16-byte shared loads; the (j, k) records and sums stay in
 // registers.  One partner at a time and
@@ -564,10 +564,10 @@ __device__ __forceinline__ int column(int j, int p) { return GRAD ? (j + p) & 7 
 // frames and, in FP64, 16.7 instead of 15.3 ms on the cluster (both before the unit
 // order).  Whole evaluations with the neighbour-list and block-per-molecule kernels
 // that this one replaced (185 instructions per slot, exp, log and divisions per
-// triple in FP64) against now: cluster of 5000 atoms (FP64) 54.4 -> 15.1 ms, 512
-// molecules (FP64) 21.2 -> 2.1 ms, 4096 molecules (mixed) 13.6 -> 5.8 ms, eight
-// periodic frames (mixed) 163 -> 51 ms, one molecule of 100 atoms 220 -> 67 us, slab
-// energy 2.8 -> 0.31 ms.
+// triple in FP64) against now: cluster of 5000 atoms (FP64) 54.0 -> 15.2 ms, 512
+// molecules (FP64) 21.1 -> 2.15 ms, 4096 molecules (mixed) 13.5 -> 5.9 ms, eight
+// periodic frames (mixed) 166 -> 53 ms, one molecule of 100 atoms 222 -> 70 us, slab
+// energy 2.73 -> 0.31 ms.
 // GEN: work partition and term counting (the owner test of every triple).
 template <class R, bool GRAD, bool PER, bool GEN>
 __global__ void __launch_bounds__(32 * kAtmWarps, kTripleBlocks<R, GRAD>)

@@ -14,9 +14,10 @@
 // its pairs in registers from the first phase to the last, and the kernel reads the
 // positions from and writes the results to pinned host memory where the call has host
 // buffers.  Four staged kernels and two copies before, one or (with the three-body
-// term) four launches now, a call of the C entry: 12 atoms 33 -> 20 us, 100 atoms 34
-// -> 25 us and with the three-body term 68 -> 48 us, 251 atoms (zero damping) 38 -> 34
-// us (16 SMs share the FP64 work of 63 000 pair ends then: 25 us in the kernel).
+// term) four launches now, a call of the C entry: 12 atoms 33 -> 21 us, 100 atoms 34
+// -> 27 us and with the three-body term 68 -> 50 us, 251 atoms (zero damping) 38 -> 35
+// us (16 SMs share the FP64 work of 63 000 pair ends then: 25 us in the kernel).  Up to
+// a microsecond of it is the barrier before the first remote store.
 #include <cooperative_groups.h>
 #include <math_constants.h>
 
