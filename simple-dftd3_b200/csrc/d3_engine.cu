@@ -292,10 +292,11 @@ Engine::Engine(int nsys, const int* natoms, const int* numbers, const double* la
     pu_.U = dev_alloc<double>(species_vector_doubles(natoms_, nid));
     any_periodic_ = false;
     for (int sy = 0; sy < nsys; sy++) any_periodic_ = any_periodic_ || periodic_any(sy);
-    // slots for the largest split: four, or as many as auto_split takes for few tile pairs
+    // slots for the largest split: four, or more for few tile pairs (molecules up to
+    // kDiagonalMaxAtoms take whole units, or what the tuning asks for)
     max_split_ = 4;
-    const long long want = any_periodic_ ? 6LL * sms_ : max_sys_atoms_ > kDiagonalMaxAtoms ? 2LL * sms_ : 0;
-    while (max_split_ < 32 && pu_.nunits * (long long)max_split_ < want) max_split_ *= 2;
+    const bool split_more = any_periodic_ || max_sys_atoms_ > kDiagonalMaxAtoms;
+    while (split_more && max_split_ < 32 && (long long)pu_.nunits * max_split_ < 6LL * sms_) max_split_ *= 2;
     const size_t items = (size_t)std::max(pu_.nunits, 1) * max_split_;
     pu_.unit_i = dev_alloc<double>(items * pair_unit_slot_doubles());
     pu_.unit_j = pu_.unit_i + items * pair_unit_i_doubles();
